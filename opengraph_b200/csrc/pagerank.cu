@@ -33,9 +33,7 @@
 // memory latency more than by HBM bandwidth.  Pull therefore runs on a
 // re-laid copy of the inverse neighbour array (built once per graph): source
 // ids renumbered by descending out-degree, so the contribs of the sources of
-// most edges share few cache lines (contrib is kept in that numbering; a
-// pull CTA can also stage the leading renumbered sources in shared memory,
-// off by default), and the rows of in-degree <= warp_thr stored first and
+// most edges share few cache lines (contrib is kept in that numbering), and the rows of in-degree <= warp_thr stored first and
 // contiguous, so a warp loads the edges of 128 light rows with coalesced
 // loads and gathers them 256 at a time (light rows were the latency tail of
 // the iteration: a lane walked its row one dependent gather per step).  The
@@ -57,12 +55,11 @@ constexpr int kPullThreads = 1024;   // pull: one CTA per SM
 constexpr int kPullGroup = 256;      // threads per chunk group (the oracle's cta_threads)
 constexpr int kPullGroups = kPullThreads / kPullGroup;
 constexpr uint32_t kStage = 256;     // staged edges per warp and window
-constexpr int kLightR = 4;           // light rows per lane (128 per warp unit)
-constexpr uint32_t kUnit = 4096;     // medium-row edges per warp unit
+constexpr uint32_t kUnitMax = 4096;  // medium-row edges per warp unit: between these, by
+constexpr uint32_t kUnitMin = 256;   // the graph's size (pr_unit_edges)
 constexpr uint32_t kTab = 64;        // medium rows per table batch
 constexpr uint32_t kWarpSmemWords = kStage + 3 * kTab + 1;  // stage + table of one warp
 constexpr size_t kPullDynSmem = (size_t)(kPullThreads / 32) * kWarpSmemWords * 4;
-constexpr uint32_t kHotLimit = 0;    // renumbered sources whose contrib a pull CTA stages in shared memory
 constexpr uint32_t kPrChunk = 8192;  // edges per chunk of a very heavy row
 constexpr uint32_t kPushHubDeg = 256;  // push: destinations with more in-edges are hubs
 constexpr uint32_t kHubChunk = 1024;   // push: in-edges of a hub summed by one warp
@@ -106,7 +103,6 @@ struct PrWork {
   bool rl_ready = false;
   DevBuf perm, nbr_rl, rows_rl, off_light, med_v, med_off, unit_first, rl_tmp;
   uint32_t n_med = 0, n_units = 0, med_base = 0;
-  uint32_t hot = 0;  // staged renumbered sources
   DevBuf contrib0, contrib1, next, ctl;
   DevBuf heavy;                        // vertex ids of the warp rows (n_warp), then the chunked rows
   DevBuf chunks;                       // PrChunkItem per chunk
@@ -308,16 +304,11 @@ struct StagePipe {
   // Gather window [w0, min(w0 + kStage, e1)) into stage; the next window's
   // ids are loaded into u meanwhile.  The caller syncs the warp afterwards.
   __device__ __forceinline__ void gather(float* stage, const uint32_t* __restrict__ nbr, const float* __restrict__ c,
-                                         const float* s_hot, uint32_t hot, uint32_t w0, uint32_t e1, uint32_t lane) {
+                                         uint32_t w0, uint32_t e1, uint32_t lane) {
 #pragma unroll
     for (uint32_t m = 0; m < kStage / 32; m++) {
       const uint32_t j = w0 + m * 32 + lane;
-      if (j < e1) {
-        if (u[m] < hot)
-          stage[m * 32 + lane] = s_hot[u[m]];
-        else
-          cp_async4(&stage[m * 32 + lane], c + u[m]);
-      }
+      if (j < e1) cp_async4(&stage[m * 32 + lane], c + u[m]);
     }
     load(nbr, w0 + kStage, e1, lane);
     cp_async_wait_all();
@@ -333,31 +324,34 @@ struct StagePipe {
 //      flight per CTA): lanes strided, warps folded, the group's warps summed
 //      in order, the chunk sums in chunk order by the group that finishes a
 //      row's last chunk;
-//  (2) medium rows, a warp per unit of kUnit edges (the rows starting in
+//  (2) medium rows, a warp per unit of `unit` edges (the rows starting in
 //      it): the unit's edges are gathered kStage at a time into the warp's
 //      stage with coalesced loads; lane l adds the elements l, l+32, ... of
 //      each row in order, and the row is butterfly-folded when it ends;
-//  (3) light rows, a warp per 128 consecutive vertices: their edges are
+//  (3) light rows, a warp per 32 R consecutive vertices: their edges are
 //      contiguous, gathered into the stage the same way, and each lane adds
-//      its four rows' values in CSR order.
+//      its R rows' values in CSR order.
+// A warp's first unit of either kind is its own index (the light ones counted
+// from the other end, so that a graph with few medium units spreads over all
+// warps); only when there are more units than warps are the rest handed out by
+// an atomic counter.  Claiming every unit from the counter cost 19 K atomics on
+// one address per iteration, more than a small graph's whole work (RMAT-22: 266
+// -> 257 us per iteration without them).
 // rows_rl, pr and out_degree are in original vertex order; contrib and
 // contrib_next are indexed by renumbered id (perm).
+template <int R>
 __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
-    uint32_t hot, const PrChunkItem* __restrict__ chunks, uint32_t n_chunks, const uint32_t* __restrict__ vfirst,
+    const PrChunkItem* __restrict__ chunks, uint32_t n_chunks, const uint32_t* __restrict__ vfirst,
     const uint32_t* __restrict__ vcount, uint32_t* __restrict__ done, float* __restrict__ partials,
     const uint2* __restrict__ rows, const uint32_t* __restrict__ off_light, const uint32_t* __restrict__ unit_first,
     uint32_t n_units, const uint32_t* __restrict__ med_off, const uint32_t* __restrict__ med_v, uint32_t med_base,
     const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ out_degree, const uint32_t* __restrict__ perm,
     const float* __restrict__ contrib, float* __restrict__ contrib_next, float* __restrict__ pr, PrParams p,
     PrCtl* __restrict__ ctl, uint32_t it) {
-  extern __shared__ uint32_t s_dyn[];  // per warp: stage and medium-row table; then the hot contribs
+  extern __shared__ uint32_t s_dyn[];  // per warp: stage and medium-row table
   __shared__ float s_part[kPullGroups][kPullGroup / 32];
   __shared__ uint32_t s_last[kPullGroups];
   if (ctl->stop) return;
-  float* s_hot = reinterpret_cast<float*>(s_dyn + (kPullThreads / 32) * kWarpSmemWords);
-  for (uint32_t i = threadIdx.x; i < hot / 4; i += kPullThreads)
-    reinterpret_cast<float4*>(s_hot)[i] = __ldg(reinterpret_cast<const float4*>(contrib) + i);
-  __syncthreads();
   double err = 0.0;
   uint32_t active = 0;
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
@@ -398,10 +392,12 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
   uint32_t* toff = mine + kStage;
   uint32_t* tv = toff + kTab + 1;
   float* tsum = reinterpret_cast<float*>(tv + kTab);
-  uint32_t* claim = &ctl->claim_med[it];
-  uint32_t t = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(claim, 1u) : 0u, 0);
+  const uint32_t nwarps = gridDim.x * (kPullThreads / 32);
+  const uint32_t gw = warp * gridDim.x + blockIdx.x;
+  uint32_t t = gw;
   while (t < n_units) {
-    const uint32_t t_next = lane == 0 ? atomicAdd(claim, 1u) : 0u;  // next claim, in flight meanwhile
+    // next claim, in flight meanwhile
+    const uint32_t t_next = (lane == 0 && n_units > nwarps) ? nwarps + atomicAdd(&ctl->claim_med[it], 1u) : n_units;
     const uint32_t i0 = unit_first[t], i1 = unit_first[t + 1];
     for (uint32_t ib = i0; ib < i1; ib += kTab) {
       const uint32_t nr = min(ib + kTab, i1) - ib;
@@ -415,7 +411,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
       pipe.load(nbr, e0, e1, lane);
       for (uint32_t w0 = e0; w0 < e1; w0 += kStage) {
         const uint32_t w1 = min(w0 + kStage, e1);
-        pipe.gather(stage, nbr, contrib, s_hot, hot, w0, e1, lane);
+        pipe.gather(stage, nbr, contrib, w0, e1, lane);
         __syncwarp();
         while (r < nr) {
           const uint32_t rs = toff[r], re = toff[r + 1];
@@ -440,20 +436,19 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
     t = __shfl_sync(0xffffffffu, t_next, 0);
   }
 
-  // (3) light rows, a warp per 128 consecutive vertices
-  const uint32_t n_light = ceil_div_dev(p.V, 32 * kLightR);
-  claim = &ctl->claim_light[it];
-  t = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(claim, 1u) : 0u, 0);
+  // (3) light rows, a warp per 32 R consecutive vertices
+  const uint32_t n_light = ceil_div_dev(p.V, 32 * R);
+  t = nwarps - 1 - gw;
   while (t < n_light) {
-    const uint32_t t_next = lane == 0 ? atomicAdd(claim, 1u) : 0u;
-    const uint32_t base = t * (32 * kLightR);
-    const uint32_t vend = min(base + 32 * kLightR, p.V);
-    uint32_t st[kLightR], en[kLightR];
-    bool light[kLightR];
-    PrVtx x[kLightR];
-    float s[kLightR];
+    const uint32_t t_next = (lane == 0 && n_light > nwarps) ? nwarps + atomicAdd(&ctl->claim_light[it], 1u) : n_light;
+    const uint32_t base = t * (32 * R);
+    const uint32_t vend = min(base + 32 * R, p.V);
+    uint32_t st[R], en[R];
+    bool light[R];
+    PrVtx x[R];
+    float s[R];
 #pragma unroll
-    for (int k = 0; k < kLightR; k++) {
+    for (int k = 0; k < R; k++) {
       const uint32_t v = base + k * 32 + lane;
       st[k] = en[k] = 0;
       light[k] = false;
@@ -470,11 +465,11 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
     pipe.load(nbr, seg0, seg1, lane);
     for (uint32_t w0 = seg0; w0 < seg1; w0 += kStage) {
       const uint32_t w1 = min(w0 + kStage, seg1);
-      pipe.gather(stage, nbr, contrib, s_hot, hot, w0, seg1, lane);
+      pipe.gather(stage, nbr, contrib, w0, seg1, lane);
       __syncwarp();
-      uint32_t lo[kLightR], n[kLightR], nmax = 0;
+      uint32_t lo[R], n[R], nmax = 0;
 #pragma unroll
-      for (int k = 0; k < kLightR; k++) {
+      for (int k = 0; k < R; k++) {
         lo[k] = max(st[k], w0);
         const uint32_t hi = min(en[k], w1);
         n[k] = hi > lo[k] ? hi - lo[k] : 0u;
@@ -482,13 +477,13 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
       }
       for (uint32_t i = 0; i < nmax; i++) {
 #pragma unroll
-        for (int k = 0; k < kLightR; k++)
+        for (int k = 0; k < R; k++)
           if (i < n[k]) s[k] = __fadd_rn(s[k], stage[lo[k] - w0 + i]);
       }
       __syncwarp();
     }
 #pragma unroll
-    for (int k = 0; k < kLightR; k++)
+    for (int k = 0; k < R; k++)
       if (light[k]) pr_update_pre(base + k * 32 + lane, s[k], x[k], pr, contrib_next, p, err, active);
     t = __shfl_sync(0xffffffffu, t_next, 0);
   }
@@ -551,11 +546,11 @@ __global__ void pr_rl_rows_kernel(uint32_t V, const uint2* __restrict__ rows, ui
   if (blockIdx.x == 0 && threadIdx.x == 0) med_off[idx_m[V]] = M;
 }
 
-// unit_first[t] = first medium row starting at or after t * kUnit.
-__global__ void pr_rl_units_kernel(uint32_t n_units, const uint32_t* __restrict__ med_off, uint32_t n_med,
+// unit_first[t] = first medium row starting at or after t * unit.
+__global__ void pr_rl_units_kernel(uint32_t n_units, uint32_t unit, const uint32_t* __restrict__ med_off, uint32_t n_med,
                                    uint32_t* __restrict__ unit_first) {
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t <= n_units; t += gridDim.x * blockDim.x) {
-    const uint64_t key = (uint64_t)t * kUnit;
+    const uint64_t key = (uint64_t)t * unit;
     uint32_t lo = 0, hi = n_med;  // answer in [0, n_med]
     while (lo < hi) {
       const uint32_t mid = (lo + hi) >> 1;
@@ -834,6 +829,41 @@ static int pr_build_lists(DevGraph& g, PrWork* w, bool pull, cudaStream_t s) {
   return OK;
 }
 
+// Edges of a medium unit: the graph's edges over two units per warp of the
+// pull kernel, as a power of two between 256 (one window: a smaller unit would
+// be a partial one) and 4096.  A warp walks its unit alone, so with 4096 edges
+// throughout, RMAT-16 (1 M edges) had work for 150 of 4736 warps: 45 us an
+// iteration, 16 us at 256; RMAT-22 (67 M) has two units per warp at 4096.
+static uint32_t pr_unit_edges(uint32_t E) {
+  const uint32_t want = E / (2 * (uint32_t)sm_count() * (kPullThreads / 32));
+  uint32_t u = kUnitMin;
+  while (u < kUnitMax && u < want) u *= 2;
+  return u;
+}
+
+// Light rows per lane: four (128 vertices per warp unit) when that still gives
+// every warp a unit, else one.
+static bool pr_wide_light(uint32_t V) { return V >= 128u * (uint32_t)sm_count() * (kPullThreads / 32); }
+
+// Shared memory of the pull kernels; the rest of the SM's unified L1 / shared
+// memory stays L1: the gathers of the highest-degree sources hit there.
+template <int R>
+static int pr_pull_attrs_of(int optin_sm) {
+  cudaFuncAttributes fa;
+  OGB_CUDA(cudaFuncGetAttributes(&fa, pr_pull_kernel<R>));
+  OGB_CUDA(cudaFuncSetAttribute(pr_pull_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPullDynSmem));
+  const int pct = (int)std::min<size_t>(100, ((kPullDynSmem + fa.sharedSizeBytes + 2048) * 100 + optin_sm - 1) / optin_sm);
+  OGB_CUDA(cudaFuncSetAttribute(pr_pull_kernel<R>, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+  return OK;
+}
+static int pr_pull_attrs() {
+  int dev = 0, per_sm = 0;
+  OGB_CUDA(cudaGetDevice(&dev));
+  OGB_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+  OGB_TRY(pr_pull_attrs_of<1>(per_sm));
+  return pr_pull_attrs_of<4>(per_sm);
+}
+
 // Re-laid pull graph (once per graph, warp_thr and cta_thr): ids sorted by
 // descending out-degree (stable: ties by id), perm = old -> new; the inverse
 // neighbour array copied with renumbered ids into light | medium | chunked
@@ -875,34 +905,20 @@ static int pr_build_relabel(DevGraph& g, PrWork* w, cudaStream_t s) {
   OGB_CUDA(cudaStreamSynchronize(s));
   w->med_base = tot[0];
   w->n_med = tot[2];
-  w->n_units = ceil_div(tot[1], kUnit);
+  const uint32_t unit = pr_unit_edges(E);
+  w->n_units = ceil_div(tot[1], unit);
   OGB_TRY(w->med_v.alloc((size_t)w->n_med * 4 + 16));
   OGB_TRY(w->med_off.alloc((size_t)w->n_med * 4 + 16));
   OGB_TRY(w->unit_first.alloc((size_t)w->n_units * 4 + 16));
   pr_rl_rows_kernel<<<grid, 256, 0, s>>>(V, g.inv.d_rows(), g_warp_thr, g_cta_thr, w->off_light.as<uint32_t>(), a[4],
                                          a[5], a[6], w->rows_rl.as<uint2>(), w->med_v.as<uint32_t>(),
                                          w->med_off.as<uint32_t>());
-  pr_rl_units_kernel<<<grid, 256, 0, s>>>(w->n_units, w->med_off.as<uint32_t>(), w->n_med,
+  pr_rl_units_kernel<<<grid, 256, 0, s>>>(w->n_units, unit, w->med_off.as<uint32_t>(), w->n_med,
                                           w->unit_first.as<uint32_t>());
   pr_rl_copy_kernel<<<grid, 256, 0, s>>>(V, g.inv.d_rows(), g.inv.d_dst(), w->rows_rl.as<uint2>(),
                                          w->perm.as<uint32_t>(), w->nbr_rl.as<uint32_t>());
   OGB_CUDA(cudaGetLastError());
-  int dev = 0, optin = 0;
-  OGB_CUDA(cudaGetDevice(&dev));
-  OGB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  cudaFuncAttributes fa;
-  OGB_CUDA(cudaFuncGetAttributes(&fa, pr_pull_kernel));
-  const size_t room = (size_t)optin - fa.sharedSizeBytes - kPullDynSmem - 1024;  // and a margin
-  const uint32_t vcap = (V + 3) & ~3u;  // contrib buffers hold V + 4 floats
-  w->hot = std::min<uint32_t>(kHotLimit & ~3u, (uint32_t)std::min<size_t>(vcap, (room / 16) * 4));
-  const size_t smem = kPullDynSmem + (size_t)w->hot * 4;
-  OGB_CUDA(cudaFuncSetAttribute(pr_pull_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // the rest of the SM's unified L1 / shared memory stays L1: the gathers of
-  // the highest-degree sources hit there
-  int smem_per_sm = 0;
-  OGB_CUDA(cudaDeviceGetAttribute(&smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-  const int pct = (int)std::min<size_t>(100, ((smem + fa.sharedSizeBytes + 2048) * 100 + smem_per_sm - 1) / smem_per_sm);
-  OGB_CUDA(cudaFuncSetAttribute(pr_pull_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+  OGB_TRY(pr_pull_attrs());
   OGB_CUDA(cudaStreamSynchronize(s));
   return OK;
 }
@@ -989,6 +1005,18 @@ static int pr_work_get(DevGraph& g, bool pull, PrWork** out, cudaStream_t s) {
   return OK;
 }
 
+// One pull iteration on stream s.
+static void pr_launch_pull(DevGraph& g, PrWork* w, const float* c_cur, float* c_nxt, float* ranks, const PrParams& p,
+                           uint32_t it, cudaStream_t s) {
+  const auto kernel = pr_wide_light(p.V) ? pr_pull_kernel<4> : pr_pull_kernel<1>;
+  kernel<<<sm_count(), kPullThreads, kPullDynSmem, s>>>(
+      w->chunks.as<PrChunkItem>(), w->n_chunks, w->vfirst.as<uint32_t>(), w->vcount.as<uint32_t>(),
+      w->done.as<uint32_t>(), w->partials.as<float>(), w->rows_rl.as<uint2>(), w->off_light.as<uint32_t>(),
+      w->unit_first.as<uint32_t>(), w->n_units, w->med_off.as<uint32_t>(), w->med_v.as<uint32_t>(), w->med_base,
+      w->nbr_rl.as<uint32_t>(), g.fwd.d_out_degree(), w->perm.as<uint32_t>(), c_cur, c_nxt, ranks, p,
+      w->ctl.as<PrCtl>(), it);
+}
+
 int pagerank_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsilon, float* ranks, const float* init,
                  PrResult* res, cudaStream_t s) {
   if (max_iters > kPrMaxIters) return fail(ERR_ARG, "pagerank: at most %u iterations", kPrMaxIters);
@@ -1024,19 +1052,15 @@ int pagerank_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsilon,
   const uint32_t nb_hub = (!pull && w->n_hub_items)
                               ? std::min<uint32_t>(sms * 4, ceil_div(w->n_hub_items, T / 32)) : 0;
   const uint32_t grid = nb_hub + nb_chunk + nb_warp + nb_light;
-  const uint2* rows = pull ? g.inv.d_rows() : w->rows_fp.as<uint2>();
-  const uint32_t* nbr = pull ? g.inv.d_dst() : w->nbr_fp.as<uint32_t>();
+  const uint2* rows = w->rows_fp.as<uint2>();
+  const uint32_t* nbr = w->nbr_fp.as<uint32_t>();
   const uint32_t* heavy = w->heavy.as<uint32_t>();
   const PrChunkItem* chunks = w->chunks.as<PrChunkItem>();
 
   OGB_CUDA(cudaEventRecord(w->ev0, s));
   for (uint32_t it = 0; it < max_iters; it++) {
     if (pull) {
-      pr_pull_kernel<<<sms, kPullThreads, kPullDynSmem + (size_t)w->hot * 4, s>>>(
-          w->hot, chunks, w->n_chunks, w->vfirst.as<uint32_t>(), w->vcount.as<uint32_t>(), w->done.as<uint32_t>(),
-          w->partials.as<float>(), w->rows_rl.as<uint2>(), w->off_light.as<uint32_t>(), w->unit_first.as<uint32_t>(),
-          w->n_units, w->med_off.as<uint32_t>(), w->med_v.as<uint32_t>(), w->med_base, w->nbr_rl.as<uint32_t>(),
-          g.fwd.d_out_degree(), perm, c_cur, c_nxt, ranks, p, d_ctl, it);
+      pr_launch_pull(g, w, c_cur, c_nxt, ranks, p, it, s);
     } else {
       pr_push_scatter_kernel<<<grid, T, 0, s>>>(nb_hub, w->hub_items.as<uint4>(), w->n_hub_items, g.inv.d_dst(),
                                                  nb_chunk, nb_warp, heavy, w->n_warp, chunks, w->n_chunks, V,
@@ -1169,11 +1193,7 @@ int pagerank_batch_run(DevGraph& g, const PrBatchDev& b, uint32_t ngraphs, uint3
       cudaMemsetAsync(b.executed, 0, (size_t)ngraphs * 4, cs);
       pr_init_kernel<<<sms * 8, 256, 0, cs>>>(V, g.fwd.d_out_degree(), nullptr, p.base_pr, ranks, c_cur, nullptr, perm);
       for (uint32_t it = 0; it < max_iters; it++) {
-        pr_pull_kernel<<<sms, kPullThreads, kPullDynSmem + (size_t)w->hot * 4, cs>>>(
-            w->hot, w->chunks.as<PrChunkItem>(), w->n_chunks, w->vfirst.as<uint32_t>(), w->vcount.as<uint32_t>(),
-            w->done.as<uint32_t>(), w->partials.as<float>(), w->rows_rl.as<uint2>(), w->off_light.as<uint32_t>(),
-            w->unit_first.as<uint32_t>(), w->n_units, w->med_off.as<uint32_t>(), w->med_v.as<uint32_t>(),
-            w->med_base, w->nbr_rl.as<uint32_t>(), g.fwd.d_out_degree(), perm, c_cur, c_nxt, ranks, p, d_ctl, it);
+        pr_launch_pull(g, w, c_cur, c_nxt, ranks, p, it, cs);
         prk_batch_reduce<<<ngraphs, 256, 0, cs>>>(b, epsilon, it);
         std::swap(c_cur, c_nxt);
       }
