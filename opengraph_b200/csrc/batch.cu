@@ -805,6 +805,8 @@ struct GraphBatch {
   uint32_t ngraphs = 0;
   std::vector<uint32_t> voff;  // host copy of the vertex offsets
   DevBuf d_voff, d_eoff, gid, frozen, stop_iter, executed, active_last, err_last, delta;
+  DevBuf pieces, piece_err, piece_act, piece_done;
+  uint32_t npieces = 0;
   cudaGraphExec_t pr_exec = nullptr;
   uint32_t pr_iters = 0, pr_warp = 0, pr_cta = 0, pr_build = 0;
   double pr_eps = -1.0;
@@ -912,6 +914,21 @@ int batch_create(GraphBatch& b, uint32_t ngraphs, const uint32_t* nv, const uint
   OGB_TRY(b.active_last.alloc((size_t)ngraphs * 4 + 16));
   OGB_TRY(b.err_last.alloc((size_t)ngraphs * 8 + 16));
   OGB_TRY(b.delta.alloc(V * 4 + 16));
+  std::vector<uint4> pieces;
+  for (uint32_t i = 0; i < ngraphs; i++) {
+    const uint32_t first = (uint32_t)pieces.size();
+    uint32_t v = b.voff[i];
+    do {  // a graph without vertices keeps one empty piece: it stops at its first iteration
+      pieces.push_back(make_uint4(i, v, std::min(b.voff[i + 1], v + kBatchPiece), first));
+      v += kBatchPiece;
+    } while (v < b.voff[i + 1]);
+  }
+  b.npieces = (uint32_t)pieces.size();
+  OGB_TRY(b.pieces.alloc(pieces.size() * sizeof(uint4) + 16));
+  OGB_TRY(b.piece_err.alloc(pieces.size() * 8 + 16));
+  OGB_TRY(b.piece_act.alloc(pieces.size() * 4 + 16));
+  OGB_TRY(b.piece_done.alloc((size_t)ngraphs * 4 + 16));
+  OGB_CUDA(cudaMemcpyAsync(b.pieces.p, pieces.data(), pieces.size() * sizeof(uint4), cudaMemcpyHostToDevice, s));
   if (!b.ev0) {
     OGB_CUDA(cudaEventCreate(&b.ev0));
     OGB_CUDA(cudaEventCreate(&b.ev1));
@@ -952,6 +969,11 @@ int batch_pagerank(GraphBatch& b, uint32_t max_iters, double epsilon, float* ran
   d.active_last = b.active_last.as<uint32_t>();
   d.err_last = b.err_last.as<double>();
   d.delta = b.delta.as<float>();
+  d.pieces = b.pieces.as<uint4>();
+  d.npieces = b.npieces;
+  d.piece_err = b.piece_err.as<double>();
+  d.piece_act = b.piece_act.as<uint32_t>();
+  d.piece_done = b.piece_done.as<uint32_t>();
   bool rebuilt = false;
   // capture happens outside the timed region
   if (!b.pr_exec) {

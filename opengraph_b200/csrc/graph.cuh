@@ -159,7 +159,14 @@ struct PrBatchDev {
   uint32_t* active_last;  // per graph: active vertices of its last iteration
   double* err_last;       // per graph: error_total of its last iteration
   float* delta;           // per vertex: change in the last iteration
+  const uint4* pieces;    // npieces runs of at most kBatchPiece vertices of one graph:
+                          // graph, first vertex, end, the graph's first piece
+  uint32_t npieces;
+  double* piece_err;      // per piece: its totals of an iteration
+  uint32_t* piece_act;
+  uint32_t* piece_done;   // per graph: its finished pieces
 };
+constexpr uint32_t kBatchPiece = 2048;
 int pagerank_batch_run(DevGraph& g, const PrBatchDev& b, uint32_t ngraphs, uint32_t max_iters, double epsilon,
                        float* ranks, cudaGraphExec_t* exec, bool* rebuilt, cudaStream_t s);
 
