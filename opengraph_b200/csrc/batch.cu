@@ -808,7 +808,7 @@ struct GraphBatch {
   DevBuf pieces, piece_err, piece_act, piece_done;
   uint32_t npieces = 0;
   cudaGraphExec_t pr_exec = nullptr;
-  uint32_t pr_iters = 0, pr_warp = 0, pr_cta = 0, pr_build = 0;
+  uint32_t pr_gen = 0, pr_iters = 0, pr_warp = 0, pr_cta = 0, pr_build = 0;
   double pr_eps = -1.0;
   float* pr_ranks = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -977,7 +977,7 @@ int batch_pagerank(GraphBatch& b, uint32_t max_iters, double epsilon, float* ran
   bool rebuilt = false;
   // capture happens outside the timed region
   if (!b.pr_exec) {
-    OGB_TRY(pagerank_batch_run(b.g, d, b.ngraphs, max_iters, epsilon, ranks, &b.pr_exec, &rebuilt, s));
+    OGB_TRY(pagerank_batch_run(b.g, d, b.ngraphs, max_iters, epsilon, ranks, &b.pr_exec, &b.pr_gen, &rebuilt, s));
     OGB_CUDA(cudaStreamSynchronize(s));
     b.pr_iters = max_iters;
     b.pr_eps = epsilon;
@@ -987,7 +987,7 @@ int batch_pagerank(GraphBatch& b, uint32_t max_iters, double epsilon, float* ran
     b.pr_build = b.g.build_id;
   }
   OGB_CUDA(cudaEventRecord(b.ev0, s));
-  OGB_TRY(pagerank_batch_run(b.g, d, b.ngraphs, max_iters, epsilon, ranks, &b.pr_exec, nullptr, s));
+  OGB_TRY(pagerank_batch_run(b.g, d, b.ngraphs, max_iters, epsilon, ranks, &b.pr_exec, &b.pr_gen, nullptr, s));
   OGB_CUDA(cudaEventRecord(b.ev1, s));
   std::vector<uint32_t> stop(b.ngraphs), exe(b.ngraphs), act(b.ngraphs);
   std::vector<double> err(b.ngraphs);

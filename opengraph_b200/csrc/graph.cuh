@@ -168,7 +168,7 @@ struct PrBatchDev {
 };
 constexpr uint32_t kBatchPiece = 2048;
 int pagerank_batch_run(DevGraph& g, const PrBatchDev& b, uint32_t ngraphs, uint32_t max_iters, double epsilon,
-                       float* ranks, cudaGraphExec_t* exec, bool* rebuilt, cudaStream_t s);
+                       float* ranks, cudaGraphExec_t* exec, uint32_t* gen, bool* rebuilt, cudaStream_t s);
 
 // ---- many graphs in one disjoint union (batch.cu) ---------------------------
 struct GraphBatch;

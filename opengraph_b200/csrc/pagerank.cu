@@ -94,20 +94,29 @@ struct PrChunkItem {
   uint32_t v, j0, j1, k;  // vertex, edge range, index of the vertex in the chunked list
 };
 
+// Totals of the re-laid pull graph, on the device.
+struct PrLay {
+  uint32_t light_edges, med_edges, cut_edges;  // edges of each row class
+  uint32_t n_med, n_cut, n_chunks;             // medium rows, chunked rows, their chunks
+  uint32_t n_units;                            // medium units
+  uint32_t n_items;                            // pieces of the long rows still to be copied
+};
+
 struct PrWork {
   uint32_t V = 0;
-  int listed_pull = -1;                // direction the lists describe
-  uint32_t listed_warp = 0, listed_cta = 0, listed_build = 0;
-  // pull: source ids renumbered by descending out-degree
+  // pull: source ids renumbered by descending out-degree, rows by class
   uint32_t rl_build = 0, rl_warp = 0, rl_cta = 0;
   bool rl_ready = false;
-  DevBuf perm, nbr_rl, rows_rl, off_light, med_v, med_off, unit_first, rl_tmp;
-  uint32_t n_med = 0, n_units = 0, med_base = 0;
+  DevBuf perm, nbr_rl, rows_rl, off_light, med_v, med_off, unit_first, rl_tmp, lay, rl_items;
+  DevBuf rl_chunks, rl_first, rl_count, rl_done, rl_partials;  // chunked rows, as the push lists below
+  uint32_t unit = 0;    // edges per medium unit
+  uint32_t rl_gen = 0;  // layouts built so far (their buffers may have moved)
   DevBuf contrib0, contrib1, next, ctl;
+  // push: lists of the filtered forward rows
+  bool listed = false;
+  uint32_t listed_warp = 0, listed_cta = 0, listed_build = 0;
   DevBuf heavy;                        // vertex ids of the warp rows (n_warp), then the chunked rows
   DevBuf chunks;                       // PrChunkItem per chunk
-  DevBuf vfirst, vcount, done;         // per chunked vertex: first chunk, chunk count, finished chunks
-  DevBuf partials;                     // float per chunk
   uint32_t n_warp = 0, n_cta = 0, n_chunks = 0;
   // push: the pushes into each hub (in-degree > kPushHubDeg) are summed over
   // the hub's in-row and applied once per chunk; the other out-edges scatter
@@ -341,16 +350,16 @@ struct StagePipe {
 // contrib_next are indexed by renumbered id (perm).
 template <int R>
 __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
-    const PrChunkItem* __restrict__ chunks, uint32_t n_chunks, const uint32_t* __restrict__ vfirst,
+    const PrLay* __restrict__ lay, const PrChunkItem* __restrict__ chunks, const uint32_t* __restrict__ vfirst,
     const uint32_t* __restrict__ vcount, uint32_t* __restrict__ done, float* __restrict__ partials,
     const uint2* __restrict__ rows, const uint32_t* __restrict__ off_light, const uint32_t* __restrict__ unit_first,
-    uint32_t n_units, const uint32_t* __restrict__ med_off, const uint32_t* __restrict__ med_v, uint32_t med_base,
-    const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ out_degree, const uint32_t* __restrict__ perm,
+    const uint32_t* __restrict__ med_off, const uint32_t* __restrict__ med_v, const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ out_degree, const uint32_t* __restrict__ perm,
     const float* __restrict__ contrib, float* __restrict__ contrib_next, float* __restrict__ pr, PrParams p,
     PrCtl* __restrict__ ctl, uint32_t it) {
   extern __shared__ uint32_t s_dyn[];  // per warp: stage and medium-row table
   __shared__ float s_part[kPullGroups][kPullGroup / 32];
   __shared__ uint32_t s_last[kPullGroups];
+  const uint32_t n_chunks = lay->n_chunks, n_units = lay->n_units, med_base = lay->light_edges;
   if (ctl->stop) return;
   double err = 0.0;
   uint32_t active = 0;
@@ -492,11 +501,15 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
 
 // ---------------------------------------------------------------- renumbering
 
-// key = ~out_degree (ascending sort = descending degree), payload = id.
+// key = 2^16 - 1 - out-degree (ascending sort = descending degree; degrees
+// above 2^16 - 1 tie), payload = id.  The order decides only which contribs
+// share cache lines, so two radix passes over 16 bits do.
+constexpr uint32_t kRlKeyBits = 16;
 __global__ void pr_rl_keys_kernel(uint32_t V, const uint32_t* __restrict__ out_degree, uint32_t* __restrict__ keys,
                                   uint32_t* __restrict__ ids) {
+  constexpr uint32_t top = (1u << kRlKeyBits) - 1;
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    keys[v] = ~out_degree[v];
+    keys[v] = top - min(out_degree[v], top);
     ids[v] = v;
   }
 }
@@ -506,49 +519,165 @@ __global__ void pr_rl_perm_kernel(uint32_t V, const uint32_t* __restrict__ order
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x) perm[order[i]] = i;
 }
 
-// Row lengths by class (light <= warp_thr < medium <= cta_thr < chunked),
-// and the medium flag.
-__global__ void pr_rl_split_kernel(uint32_t V, const uint2* __restrict__ rows, uint32_t warp_thr, uint32_t cta_thr,
-                                   uint32_t* __restrict__ dl, uint32_t* __restrict__ dm, uint32_t* __restrict__ dc,
-                                   uint32_t* __restrict__ fm) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    const uint32_t d = rows[v].y;
-    const uint32_t cls = d <= warp_thr ? 0u : (d <= cta_thr ? 1u : 2u);
-    dl[v] = cls == 0 ? d : 0u;
-    dm[v] = cls == 1 ? d : 0u;
-    dc[v] = cls == 2 ? d : 0u;
-    fm[v] = cls == 1 ? 1u : 0u;
+// The classes of all rows (light <= warp_thr < medium <= cta_thr < chunked) and
+// where each row goes, in three passes: per tile of kLayTile vertices the class
+// totals, a scan of those by one CTA, then every row's place from its tile's
+// offsets and a scan inside the tile.  (Separate flag arrays, four device scans
+// and lists filled through one atomic counter took 16 launches and three host
+// round trips: 340 us of kernels at RMAT-22, 110 us at RMAT-16.)
+constexpr uint32_t kLayTile = 2048;  // 256 threads x 8 consecutive vertices
+constexpr int kLayQ = 6;             // light, medium, chunked edges; medium, chunked rows; chunks
+struct LaySum {
+  uint32_t q[kLayQ];
+};
+__device__ __forceinline__ void lay_add(LaySum& t, uint32_t d, uint32_t warp_thr, uint32_t cta_thr) {
+  if (d <= warp_thr) {
+    t.q[0] += d;
+  } else if (d <= cta_thr) {
+    t.q[1] += d;
+    t.q[3]++;
+  } else {
+    t.q[2] += d;
+    t.q[4]++;
+    t.q[5] += (d + kPrChunk - 1) / kPrChunk;
   }
 }
 
-// New row offsets (light | medium | chunked), and the medium row list:
-// med_v[i] = vertex, med_off[i] = its offset inside the medium class.
-__global__ void pr_rl_rows_kernel(uint32_t V, const uint2* __restrict__ rows, uint32_t warp_thr, uint32_t cta_thr,
-                                  const uint32_t* __restrict__ off_l, const uint32_t* __restrict__ off_m,
-                                  const uint32_t* __restrict__ off_c, const uint32_t* __restrict__ idx_m,
-                                  uint2* __restrict__ rows_rl, uint32_t* __restrict__ med_v,
-                                  uint32_t* __restrict__ med_off) {
-  const uint32_t L = off_l[V], M = off_m[V];
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    const uint32_t d = rows[v].y;
-    uint32_t o;
-    if (d <= warp_thr) {
-      o = off_l[v];
-    } else if (d <= cta_thr) {
-      o = L + off_m[v];
-      med_v[idx_m[v]] = v;
-      med_off[idx_m[v]] = off_m[v];
-    } else {
-      o = L + M + off_c[v];
+// Exclusive block scan (256 threads) of every total; sums left in tot.
+__device__ __forceinline__ LaySum lay_block_scan(const LaySum& in, LaySum* s_w, LaySum& tot) {
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  LaySum x = in;
+#pragma unroll
+  for (int i = 0; i < kLayQ; i++)
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x.q[i], o);
+      if (lane >= (uint32_t)o) x.q[i] += y;
     }
-    rows_rl[v] = make_uint2(o, d);
+  if (lane == 31) s_w[warp] = x;
+  __syncthreads();
+  LaySum r;
+#pragma unroll
+  for (int i = 0; i < kLayQ; i++) {
+    uint32_t before = 0, all = 0;
+    for (uint32_t w = 0; w < 8; w++) {
+      if (w < warp) before += s_w[w].q[i];
+      all += s_w[w].q[i];
+    }
+    r.q[i] = before + x.q[i] - in.q[i];
+    tot.q[i] = all;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) med_off[idx_m[V]] = M;
+  __syncthreads();
+  return r;
+}
+
+__global__ void __launch_bounds__(256) pr_lay_sums_kernel(uint32_t V, const uint2* __restrict__ rows,
+                                                          uint32_t warp_thr, uint32_t cta_thr,
+                                                          uint32_t* __restrict__ sums, uint32_t ntiles) {
+  __shared__ LaySum s_w[8];
+  LaySum t = {}, tot;
+  const uint64_t base = (uint64_t)blockIdx.x * kLayTile;
+#pragma unroll
+  for (uint32_t k = 0; k < kLayTile / 256; k++) {
+    const uint64_t v = base + k * 256 + threadIdx.x;
+    if (v < V) lay_add(t, rows[v].y, warp_thr, cta_thr);
+  }
+  lay_block_scan(t, s_w, tot);
+  if (threadIdx.x < kLayQ) sums[threadIdx.x * ntiles + blockIdx.x] = tot.q[threadIdx.x];
+}
+
+// One CTA: exclusive scan of the tile totals in place, the grand totals into lay.
+__global__ void __launch_bounds__(256) pr_lay_scan_kernel(uint32_t* __restrict__ sums, uint32_t ntiles, uint32_t unit,
+                                                          PrLay* __restrict__ lay) {
+  __shared__ LaySum s_w[8];
+  LaySum carry = {};
+  for (uint32_t b = 0; b < ntiles; b += 256) {
+    const uint32_t i = b + threadIdx.x;
+    LaySum t, tot;
+#pragma unroll
+    for (int q = 0; q < kLayQ; q++) t.q[q] = i < ntiles ? sums[q * ntiles + i] : 0u;
+    const LaySum e = lay_block_scan(t, s_w, tot);
+#pragma unroll
+    for (int q = 0; q < kLayQ; q++) {
+      if (i < ntiles) sums[q * ntiles + i] = carry.q[q] + e.q[q];
+      carry.q[q] += tot.q[q];
+    }
+  }
+  if (threadIdx.x == 0) {
+    lay->light_edges = carry.q[0];
+    lay->med_edges = carry.q[1];
+    lay->cut_edges = carry.q[2];
+    lay->n_med = carry.q[3];
+    lay->n_cut = carry.q[4];
+    lay->n_chunks = carry.q[5];
+    lay->n_units = (carry.q[1] + unit - 1) / unit;
+    lay->n_items = 0;
+  }
+}
+
+// New row offsets (light | medium | chunked), off_light (V + 1 entries, rows of
+// the other classes empty), the medium row list (med_v[i] = vertex, med_off[i] =
+// its offset inside the class) and the chunk table of the chunked rows.
+__global__ void __launch_bounds__(256) pr_lay_rows_kernel(uint32_t V, const uint2* __restrict__ rows,
+                                                          uint32_t warp_thr, uint32_t cta_thr,
+                                                          const uint32_t* __restrict__ sums, uint32_t ntiles,
+                                                          const PrLay* __restrict__ lay,
+                                                          uint32_t* __restrict__ off_light,
+                                                          uint2* __restrict__ rows_rl, uint32_t* __restrict__ med_v,
+                                                          uint32_t* __restrict__ med_off,
+                                                          PrChunkItem* __restrict__ chunks,
+                                                          uint32_t* __restrict__ vfirst, uint32_t* __restrict__ vcount,
+                                                          uint32_t* __restrict__ done) {
+  constexpr uint32_t K = kLayTile / 256;
+  __shared__ LaySum s_w[8];
+  const uint64_t base = (uint64_t)blockIdx.x * kLayTile + threadIdx.x * K;
+  uint32_t d[K];
+  LaySum t = {}, tot;
+#pragma unroll
+  for (uint32_t k = 0; k < K; k++) {
+    d[k] = base + k < V ? rows[base + k].y : 0u;
+    if (base + k < V) lay_add(t, d[k], warp_thr, cta_thr);
+  }
+  LaySum o = lay_block_scan(t, s_w, tot);
+#pragma unroll
+  for (int q = 0; q < kLayQ; q++) o.q[q] += sums[q * ntiles + blockIdx.x];
+  const uint32_t L = lay->light_edges, M = lay->med_edges;
+#pragma unroll
+  for (uint32_t k = 0; k < K; k++) {
+    if (base + k >= V) break;
+    const uint32_t v = (uint32_t)base + k;
+    off_light[v] = o.q[0];
+    uint32_t at;
+    if (d[k] <= warp_thr) {
+      at = o.q[0];
+    } else if (d[k] <= cta_thr) {
+      at = L + o.q[1];
+      med_v[o.q[3]] = v;
+      med_off[o.q[3]] = o.q[1];
+    } else {
+      at = L + M + o.q[2];
+      const uint32_t n = (d[k] + kPrChunk - 1) / kPrChunk;
+      vfirst[o.q[4]] = o.q[5];
+      vcount[o.q[4]] = n;
+      done[o.q[4]] = 0;
+      for (uint32_t c = 0; c < n; c++) {
+        const uint32_t j0 = at + c * kPrChunk;
+        chunks[o.q[5] + c] = {v, j0, min(at + d[k], j0 + kPrChunk), o.q[4]};
+      }
+    }
+    rows_rl[v] = make_uint2(at, d[k]);
+    lay_add(o, d[k], warp_thr, cta_thr);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    off_light[V] = L;
+    med_off[lay->n_med] = M;
+  }
 }
 
 // unit_first[t] = first medium row starting at or after t * unit.
-__global__ void pr_rl_units_kernel(uint32_t n_units, uint32_t unit, const uint32_t* __restrict__ med_off, uint32_t n_med,
+__global__ void pr_rl_units_kernel(const PrLay* __restrict__ lay, uint32_t unit, const uint32_t* __restrict__ med_off,
                                    uint32_t* __restrict__ unit_first) {
+  const uint32_t n_units = lay->n_units, n_med = lay->n_med;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t <= n_units; t += gridDim.x * blockDim.x) {
     const uint64_t key = (uint64_t)t * unit;
     uint32_t lo = 0, hi = n_med;  // answer in [0, n_med]
@@ -563,20 +692,84 @@ __global__ void pr_rl_units_kernel(uint32_t n_units, uint32_t unit, const uint32
   }
 }
 
-// Copy every row into the new layout with renumbered source ids (a warp
-// per row).
-__global__ void pr_rl_copy_kernel(uint32_t V, const uint2* __restrict__ rows, const uint32_t* __restrict__ nbr,
-                                  const uint2* __restrict__ rows_rl, const uint32_t* __restrict__ perm,
-                                  uint32_t* __restrict__ out) {
+// Copy every row into the new layout with renumbered source ids.  A warp takes
+// 32 consecutive rows and copies their edges as one sequence, 128 at a time
+// (each lane finds its edge's row among the 32 by a search through shuffles), so
+// short rows fill the lanes; a row longer than kCopyLong goes into `items` in
+// pieces of kCopyPiece edges, a CTA of the second kernel each.  (A warp per row
+// left lanes idle on short rows and walked a hub's 161 K edges alone: 3.69 ms at
+// RMAT-22, 254 us at RMAT-16.)
+constexpr uint32_t kCopyLong = 1024, kCopyPiece = 4096;
+__global__ void __launch_bounds__(256) pr_rl_copy_kernel(uint32_t V, const uint2* __restrict__ rows,
+                                                         const uint32_t* __restrict__ nbr,
+                                                         const uint2* __restrict__ rows_rl,
+                                                         const uint32_t* __restrict__ perm, uint32_t* __restrict__ out,
+                                                         uint4* __restrict__ items, PrLay* __restrict__ lay) {
   const uint32_t lane = lane_id();
-  const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
-  for (uint32_t v = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); v < V; v += nwarps) {
-    const uint2 r = rows[v];
-    const uint32_t o = rows_rl[v].x;
-    for (uint32_t i = lane; i < r.y; i += 32) out[o + i] = perm[nbr[r.x + i] & 0x3FFFFFFFu];
+  const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x / 32);
+  for (uint64_t g = (uint64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); g * 32 < V; g += nwarps) {
+    const uint64_t v = g * 32 + lane;
+    uint2 r = make_uint2(0u, 0u);
+    uint32_t o = 0;
+    if (v < V) {
+      r = rows[v];
+      o = rows_rl[v].x;
+    }
+    if (r.y > kCopyLong) {
+      const uint32_t n = (r.y + kCopyPiece - 1) / kCopyPiece;
+      const uint32_t at = atomicAdd(&lay->n_items, n);
+      for (uint32_t c = 0; c < n; c++)
+        items[at + c] = make_uint4(r.x + c * kCopyPiece, o + c * kCopyPiece, min(kCopyPiece, r.y - c * kCopyPiece), 0u);
+      r.y = 0;
+    }
+    uint32_t ex = r.y;  // inclusive, then exclusive scan of the 32 lengths
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, ex, k);
+      if (lane >= (uint32_t)k) ex += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, ex, 31);
+    ex -= r.y;
+    for (uint32_t e0 = 0; e0 < total; e0 += 128) {
+      uint32_t id[4], to[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t e = e0 + k * 32 + lane;
+        uint32_t p = 0;  // last row whose first edge is at or before e
+#pragma unroll
+        for (int step = 16; step; step >>= 1) {
+          const uint32_t first = __shfl_sync(0xffffffffu, ex, p + step);
+          if (first <= e) p += step;
+        }
+        const uint32_t from = __shfl_sync(0xffffffffu, r.x - ex, p) + e;
+        to[k] = __shfl_sync(0xffffffffu, o - ex, p) + e;
+        id[k] = e < total ? (__ldg(&nbr[from]) & 0x3FFFFFFFu) : 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (e0 + k * 32 + lane < total) out[to[k]] = __ldg(&perm[id[k]]);
+    }
   }
 }
 
+__global__ void __launch_bounds__(256) pr_rl_copy_long_kernel(const PrLay* __restrict__ lay,
+                                                              const uint4* __restrict__ items,
+                                                              const uint32_t* __restrict__ nbr,
+                                                              const uint32_t* __restrict__ perm,
+                                                              uint32_t* __restrict__ out) {
+  const uint32_t n = lay->n_items;
+  for (uint32_t t = blockIdx.x; t < n; t += gridDim.x) {
+    const uint4 it = items[t];
+    for (uint32_t j = threadIdx.x; j < it.z; j += 4 * 256) {
+      uint32_t id[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) id[k] = j + k * 256 < it.z ? (__ldg(&nbr[it.x + j + k * 256]) & 0x3FFFFFFFu) : 0u;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (j + k * 256 < it.z) out[it.y + j + k * 256] = __ldg(&perm[id[k]]);
+    }
+  }
+}
 
 // ---------------------------------------------------------------- push ------
 //
@@ -779,13 +972,11 @@ __global__ void pr_normalize_kernel(uint32_t V, float* __restrict__ pr) {
     pr[v] = __fdiv_rn(pr[v], fv);
 }
 
-// Heavy lists and the chunk table of one direction (built once per graph,
-// direction and thresholds; the only host round trips of PageRank).
-// Pull lists refer to the renumbered layout (rows_rl), push lists to the
-// filtered forward CSR (rows_fp).
-static int pr_build_lists(DevGraph& g, PrWork* w, bool pull, cudaStream_t s) {
+// Heavy lists and the chunk table of the filtered forward rows (once per graph
+// and thresholds).
+static int pr_build_lists(DevGraph& g, PrWork* w, cudaStream_t s) {
   const uint32_t V = g.V;
-  const uint2* rows = pull ? w->rows_rl.as<uint2>() : w->rows_fp.as<uint2>();
+  const uint2* rows = w->rows_fp.as<uint2>();
   uint32_t* cnt = w->ctl.as<uint32_t>() + sizeof(PrCtl) / 4;  // scratch words after the control block
   OGB_CUDA(cudaMemsetAsync(cnt, 0, 16, s));
   const int grid = sm_count() * 8;
@@ -806,25 +997,14 @@ static int pr_build_lists(DevGraph& g, PrWork* w, bool pull, cudaStream_t s) {
   if (w->n_cta) OGB_CUDA(cudaMemcpyAsync(cr.data(), cta_rows.p, (size_t)w->n_cta * 16, cudaMemcpyDeviceToHost, s));
   OGB_CUDA(cudaStreamSynchronize(s));
   std::vector<PrChunkItem> items;
-  std::vector<uint32_t> first(w->n_cta), count(w->n_cta);
   for (uint32_t k = 0; k < w->n_cta; k++) {
     const uint32_t v = cr[k].x, a = cr[k].y, d = cr[k].z;
-    first[k] = (uint32_t)items.size();
     for (uint32_t c = 0; c < d; c += kPrChunk) items.push_back({v, a + c, a + std::min(d, c + kPrChunk), k});
-    count[k] = (uint32_t)items.size() - first[k];
   }
   w->n_chunks = (uint32_t)items.size();
   OGB_TRY(w->chunks.alloc(items.size() * sizeof(PrChunkItem) + 16));
-  OGB_TRY(w->partials.alloc(items.size() * 4 + 16));
-  OGB_TRY(w->vfirst.alloc((size_t)w->n_cta * 4 + 16));
-  OGB_TRY(w->vcount.alloc((size_t)w->n_cta * 4 + 16));
-  OGB_TRY(w->done.alloc((size_t)w->n_cta * 4 + 16));
-  if (!items.empty()) {
+  if (!items.empty())
     OGB_CUDA(cudaMemcpyAsync(w->chunks.p, items.data(), items.size() * sizeof(PrChunkItem), cudaMemcpyHostToDevice, s));
-    OGB_CUDA(cudaMemcpyAsync(w->vfirst.p, first.data(), first.size() * 4, cudaMemcpyHostToDevice, s));
-    OGB_CUDA(cudaMemcpyAsync(w->vcount.p, count.data(), count.size() * 4, cudaMemcpyHostToDevice, s));
-  }
-  OGB_CUDA(cudaMemsetAsync(w->done.p, 0, (size_t)w->n_cta * 4 + 16, s));
   OGB_CUDA(cudaStreamSynchronize(s));
   return OK;
 }
@@ -867,60 +1047,59 @@ static int pr_pull_attrs() {
 // Re-laid pull graph (once per graph, warp_thr and cta_thr): ids sorted by
 // descending out-degree (stable: ties by id), perm = old -> new; the inverse
 // neighbour array copied with renumbered ids into light | medium | chunked
-// classes, each contiguous in vertex order; rows_rl = {new offset,
-// in-degree}; off_light = offsets of the light rows (V + 1 entries, other
-// rows empty); the medium row list (med_v, med_off) and its units.
+// classes, each contiguous in vertex order; rows_rl = {new offset, in-degree};
+// off_light, the medium row list with its units, and the chunk table.  The
+// lists' sizes stay on the device (PrLay); the buffers hold the most that E
+// edges can need.
 static int pr_build_relabel(DevGraph& g, PrWork* w, cudaStream_t s) {
   const uint32_t V = g.V, E = g.E;
-  const size_t Vp = ((size_t)V + 8) & ~(size_t)3;  // words per V + 1 array, padded
+  const size_t Vp = ((size_t)V + 8) & ~(size_t)3;
+  const uint32_t ntiles = ceil_div(V, kLayTile);
+  const size_t max_med = std::min<size_t>(V, E / ((size_t)g_warp_thr + 1));
+  const size_t max_cut = std::min<size_t>(V, E / ((size_t)g_cta_thr + 1));
+  const size_t max_chunks = max_cut + E / kPrChunk;
+  const size_t max_items = E / kCopyLong + E / kCopyPiece;
+  w->unit = pr_unit_edges(E);
   OGB_TRY(w->perm.alloc((size_t)V * 4 + 16));
   OGB_TRY(w->nbr_rl.alloc((size_t)E * 4 + 16));
   OGB_TRY(w->rows_rl.alloc((size_t)V * 8 + 16));
   OGB_TRY(w->off_light.alloc(Vp * 4));
-  OGB_TRY(w->rl_tmp.alloc((Vp * 8 + scan_tmp_words(V)) * 4));
+  OGB_TRY(w->rl_tmp.alloc((Vp * 4 + (size_t)ntiles * kLayQ) * 4));
+  OGB_TRY(w->lay.alloc(sizeof(PrLay)));
+  OGB_TRY(w->med_v.alloc(max_med * 4 + 16));
+  OGB_TRY(w->med_off.alloc(max_med * 4 + 16));
+  OGB_TRY(w->unit_first.alloc(((size_t)E / w->unit + 2) * 4 + 16));
+  OGB_TRY(w->rl_chunks.alloc(max_chunks * sizeof(PrChunkItem) + 16));
+  OGB_TRY(w->rl_partials.alloc(max_chunks * 4 + 16));
+  OGB_TRY(w->rl_first.alloc(max_cut * 4 + 16));
+  OGB_TRY(w->rl_count.alloc(max_cut * 4 + 16));
+  OGB_TRY(w->rl_done.alloc(max_cut * 4 + 16));
+  OGB_TRY(w->rl_items.alloc(max_items * 16 + 16));
   const int grid = sm_count() * 8;
   uint32_t* t0 = w->rl_tmp.as<uint32_t>();
-  uint32_t* a[8];
-  for (int i = 0; i < 8; i++) a[i] = t0 + i * Vp;
-  uint32_t* scan_tmp = t0 + 8 * Vp;
-  // sort ids by ~out_degree: a0 keys, a1 ids -> a2 sorted keys, a3 order
-  pr_rl_keys_kernel<<<grid, 256, 0, s>>>(V, g.fwd.d_out_degree(), a[0], a[1]);
+  uint32_t* sums = t0 + 4 * Vp;
+  PrLay* lay = w->lay.as<PrLay>();
+  const uint2* rows = g.inv.d_rows();
+  pr_rl_keys_kernel<<<grid, 256, 0, s>>>(V, g.fwd.d_out_degree(), t0, t0 + Vp);
   OGB_CUDA(cudaGetLastError());
-  KV in{a[0], a[1], nullptr};
-  KV out{a[2], a[3], nullptr};
-  OGB_TRY(sort_pairs(in, out, V, g.sort_ws, s));
-  pr_rl_perm_kernel<<<grid, 256, 0, s>>>(V, a[3], w->perm.as<uint32_t>());
-  // classes: a0 light, a1 medium, a2 chunked lengths, a3 medium flags; scans
-  // into off_light, a4, a5, a6
-  pr_rl_split_kernel<<<grid, 256, 0, s>>>(V, g.inv.d_rows(), g_warp_thr, g_cta_thr, a[0], a[1], a[2], a[3]);
+  KV in{t0, t0 + Vp, nullptr};
+  KV out{t0 + 2 * Vp, t0 + 3 * Vp, nullptr};
+  OGB_TRY(sort_pairs(in, out, V, g.sort_ws, s, kRlKeyBits));
+  pr_rl_perm_kernel<<<grid, 256, 0, s>>>(V, out.v0, w->perm.as<uint32_t>());
+  pr_lay_sums_kernel<<<ntiles, 256, 0, s>>>(V, rows, g_warp_thr, g_cta_thr, sums, ntiles);
+  pr_lay_scan_kernel<<<1, 256, 0, s>>>(sums, ntiles, w->unit, lay);
+  pr_lay_rows_kernel<<<ntiles, 256, 0, s>>>(V, rows, g_warp_thr, g_cta_thr, sums, ntiles, lay,
+                                            w->off_light.as<uint32_t>(), w->rows_rl.as<uint2>(),
+                                            w->med_v.as<uint32_t>(), w->med_off.as<uint32_t>(),
+                                            w->rl_chunks.as<PrChunkItem>(), w->rl_first.as<uint32_t>(),
+                                            w->rl_count.as<uint32_t>(), w->rl_done.as<uint32_t>());
+  pr_rl_units_kernel<<<grid, 256, 0, s>>>(lay, w->unit, w->med_off.as<uint32_t>(), w->unit_first.as<uint32_t>());
+  pr_rl_copy_kernel<<<grid, 256, 0, s>>>(V, rows, g.inv.d_dst(), w->rows_rl.as<uint2>(), w->perm.as<uint32_t>(),
+                                         w->nbr_rl.as<uint32_t>(), w->rl_items.as<uint4>(), lay);
+  pr_rl_copy_long_kernel<<<grid, 256, 0, s>>>(lay, w->rl_items.as<uint4>(), g.inv.d_dst(), w->perm.as<uint32_t>(),
+                                              w->nbr_rl.as<uint32_t>());
   OGB_CUDA(cudaGetLastError());
-  OGB_TRY(scan_exclusive_u32(a[0], w->off_light.as<uint32_t>(), V, scan_tmp, s));
-  OGB_TRY(scan_exclusive_u32(a[1], a[4], V, scan_tmp, s));
-  OGB_TRY(scan_exclusive_u32(a[2], a[5], V, scan_tmp, s));
-  OGB_TRY(scan_exclusive_u32(a[3], a[6], V, scan_tmp, s));
-  uint32_t tot[3];
-  OGB_CUDA(cudaMemcpyAsync(&tot[0], w->off_light.as<uint32_t>() + V, 4, cudaMemcpyDeviceToHost, s));
-  OGB_CUDA(cudaMemcpyAsync(&tot[1], a[4] + V, 4, cudaMemcpyDeviceToHost, s));
-  OGB_CUDA(cudaMemcpyAsync(&tot[2], a[6] + V, 4, cudaMemcpyDeviceToHost, s));
-  OGB_CUDA(cudaStreamSynchronize(s));
-  w->med_base = tot[0];
-  w->n_med = tot[2];
-  const uint32_t unit = pr_unit_edges(E);
-  w->n_units = ceil_div(tot[1], unit);
-  OGB_TRY(w->med_v.alloc((size_t)w->n_med * 4 + 16));
-  OGB_TRY(w->med_off.alloc((size_t)w->n_med * 4 + 16));
-  OGB_TRY(w->unit_first.alloc((size_t)w->n_units * 4 + 16));
-  pr_rl_rows_kernel<<<grid, 256, 0, s>>>(V, g.inv.d_rows(), g_warp_thr, g_cta_thr, w->off_light.as<uint32_t>(), a[4],
-                                         a[5], a[6], w->rows_rl.as<uint2>(), w->med_v.as<uint32_t>(),
-                                         w->med_off.as<uint32_t>());
-  pr_rl_units_kernel<<<grid, 256, 0, s>>>(w->n_units, unit, w->med_off.as<uint32_t>(), w->n_med,
-                                          w->unit_first.as<uint32_t>());
-  pr_rl_copy_kernel<<<grid, 256, 0, s>>>(V, g.inv.d_rows(), g.inv.d_dst(), w->rows_rl.as<uint2>(),
-                                         w->perm.as<uint32_t>(), w->nbr_rl.as<uint32_t>());
-  OGB_CUDA(cudaGetLastError());
-  OGB_TRY(pr_pull_attrs());
-  OGB_CUDA(cudaStreamSynchronize(s));
-  return OK;
+  return pr_pull_attrs();
 }
 
 // Push preparation (once per graph): the filtered forward CSR without the
@@ -971,32 +1150,32 @@ static int pr_work_get(DevGraph& g, bool pull, PrWork** out, cudaStream_t s) {
     OGB_TRY(w->heavy.alloc((size_t)V * 4 + 16));
     OGB_TRY(w->ctl.alloc(sizeof(PrCtl) + 64));
     w->V = V;
-    w->listed_pull = -1;
+    w->listed = false;
   }
   if (!w->h_ctl) OGB_CUDA(cudaMallocHost(&w->h_ctl, sizeof(PrCtl)));
   if (!w->ev0) {
     OGB_CUDA(cudaEventCreate(&w->ev0));
     OGB_CUDA(cudaEventCreate(&w->ev1));
   }
-  const int want = pull ? 1 : 0;
   if (pull && (!w->rl_ready || w->rl_build != g.build_id || w->rl_warp != g_warp_thr || w->rl_cta != g_cta_thr)) {
+    w->rl_ready = false;
+    w->rl_gen++;
     OGB_TRY(pr_build_relabel(g, w, s));
     w->rl_ready = true;
     w->rl_build = g.build_id;
     w->rl_warp = g_warp_thr;
     w->rl_cta = g_cta_thr;
-    w->listed_pull = -1;
   }
   if (!pull && (!w->push_ready || w->push_build != g.build_id)) {
     OGB_TRY(pr_build_push(g, w, s));
     w->push_ready = true;
     w->push_build = g.build_id;
-    w->listed_pull = -1;
+    w->listed = false;
   }
-  if (w->listed_pull != want || w->listed_warp != g_warp_thr || w->listed_cta != g_cta_thr ||
-      w->listed_build != g.build_id) {
-    OGB_TRY(pr_build_lists(g, w, pull, s));
-    w->listed_pull = want;
+  if (!pull && (!w->listed || w->listed_warp != g_warp_thr || w->listed_cta != g_cta_thr ||
+                w->listed_build != g.build_id)) {
+    OGB_TRY(pr_build_lists(g, w, s));
+    w->listed = true;
     w->listed_warp = g_warp_thr;
     w->listed_cta = g_cta_thr;
     w->listed_build = g.build_id;
@@ -1010,11 +1189,10 @@ static void pr_launch_pull(DevGraph& g, PrWork* w, const float* c_cur, float* c_
                            uint32_t it, cudaStream_t s) {
   const auto kernel = pr_wide_light(p.V) ? pr_pull_kernel<4> : pr_pull_kernel<1>;
   kernel<<<sm_count(), kPullThreads, kPullDynSmem, s>>>(
-      w->chunks.as<PrChunkItem>(), w->n_chunks, w->vfirst.as<uint32_t>(), w->vcount.as<uint32_t>(),
-      w->done.as<uint32_t>(), w->partials.as<float>(), w->rows_rl.as<uint2>(), w->off_light.as<uint32_t>(),
-      w->unit_first.as<uint32_t>(), w->n_units, w->med_off.as<uint32_t>(), w->med_v.as<uint32_t>(), w->med_base,
-      w->nbr_rl.as<uint32_t>(), g.fwd.d_out_degree(), w->perm.as<uint32_t>(), c_cur, c_nxt, ranks, p,
-      w->ctl.as<PrCtl>(), it);
+      w->lay.as<PrLay>(), w->rl_chunks.as<PrChunkItem>(), w->rl_first.as<uint32_t>(), w->rl_count.as<uint32_t>(),
+      w->rl_done.as<uint32_t>(), w->rl_partials.as<float>(), w->rows_rl.as<uint2>(), w->off_light.as<uint32_t>(),
+      w->unit_first.as<uint32_t>(), w->med_off.as<uint32_t>(), w->med_v.as<uint32_t>(), w->nbr_rl.as<uint32_t>(),
+      g.fwd.d_out_degree(), w->perm.as<uint32_t>(), c_cur, c_nxt, ranks, p, w->ctl.as<PrCtl>(), it);
 }
 
 int pagerank_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsilon, float* ranks, const float* init,
@@ -1188,14 +1366,19 @@ __global__ void prk_batch_normalize(uint32_t V, PrBatchDev b, float* __restrict_
 // the per-graph reductions and the normalization -- is captured once into a
 // CUDA graph (cached in *exec for the same arguments) and launched as one.
 int pagerank_batch_run(DevGraph& g, const PrBatchDev& b, uint32_t ngraphs, uint32_t max_iters, double epsilon,
-                       float* ranks, cudaGraphExec_t* exec, bool* rebuilt, cudaStream_t s) {
+                       float* ranks, cudaGraphExec_t* exec, uint32_t* gen, bool* rebuilt, cudaStream_t s) {
   if (max_iters > kPrMaxIters) return fail(ERR_ARG, "pagerank: at most %u iterations", kPrMaxIters);
   const uint32_t V = g.V;
   if (V == 0) return fail(ERR_ARG, "pagerank: empty graph");
   PrWork* w = nullptr;
   OGB_TRY(pr_work_get(g, true, &w, s));
   if (rebuilt) *rebuilt = false;
+  if (*exec && *gen != w->rl_gen) {  // the layout it was captured on is gone
+    cudaGraphExecDestroy(*exec);
+    *exec = nullptr;
+  }
   if (!*exec) {
+    *gen = w->rl_gen;
     const int sms = sm_count();
     PrParams p;
     p.damp = 0.85f;
