@@ -10,7 +10,7 @@
 //    digits that are constant over all keys are skipped (for V = 2^22 only
 //    three passes run, the last with 6 live bits);
 //  * each CTA claims a tile of kTile keys in launch order, ranks the keys of
-//    the tile stably with warp match masks (order = warp, item, lane, which is
+//    the tile stably with warp ballots (order = warp, item, lane, which is
 //    input order), publishes its per-digit counts and resolves the per-digit
 //    prefix of all earlier tiles by decoupled look-back;
 //  * keys and payloads are staged in shared memory in digit order and written
@@ -28,8 +28,27 @@ constexpr int kSortItems = 16;
 constexpr int kTile = kSortThreads * kSortItems;
 constexpr int kWarps = kSortThreads / 32;
 constexpr int kMaxPasses = 8;  // 4 digits x (primary, secondary)
-constexpr unsigned long long kFlagAgg = 1ull << 32;
-constexpr unsigned long long kFlagInc = 2ull << 32;
+constexpr int kLookBack = 4;   // predecessors read at once by the look-back
+
+// A look-back word: a count and a two-bit flag.  32-bit words hold counts
+// below 2^30; longer inputs take 64-bit ones.
+template <class S>
+struct LbWord;
+template <>
+struct LbWord<uint32_t> {
+  static constexpr uint32_t kAgg = 1u << 30, kInc = 2u << 30, kFlag = 3u << 30;
+};
+template <>
+struct LbWord<unsigned long long> {
+  static constexpr unsigned long long kAgg = 1ull << 32, kInc = 2ull << 32, kFlag = 3ull << 32;
+};
+constexpr uint64_t kNarrowLimit = 1ull << 30;
+__device__ __forceinline__ uint32_t lb_load(const uint32_t* p) { return ld_volatile_u32(p); }
+__device__ __forceinline__ unsigned long long lb_load(const unsigned long long* p) { return ld_volatile_u64(p); }
+__device__ __forceinline__ void lb_store(uint32_t* p, uint32_t v) {
+  asm volatile("st.volatile.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void lb_store(unsigned long long* p, unsigned long long v) { st_volatile_u64(p, v); }
 
 // counters layout (u32): [0, kMaxPasses) tile counters, [kMaxPasses] error
 // word, [kMaxPasses+1] OR of all primary keys, [kMaxPasses+2] OR of all
@@ -159,131 +178,230 @@ __device__ __forceinline__ void cp_async_commit_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
+// Lanes of `valid` whose digit equals this lane's (digits of at most NB bits):
+// one ballot per bit.  (__match_any_sync took as long as the rest of the pass:
+// 627 -> 499 us unweighted with nothing else changed.)
+template <int NB>
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d, uint32_t valid) {
+  uint32_t p = valid;
+#pragma unroll
+  for (int b = 0; b < NB; b++)
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b32 t, m;\n\t"
+        "and.b32 t, %1, %2;\n\t"
+        "setp.ne.u32 q, t, 0;\n\t"
+        "vote.sync.ballot.b32 m, q, 0xffffffff;\n\t"
+        "@!q not.b32 m, m;\n\t"
+        "and.b32 %0, %0, m;\n\t}"
+        : "+r"(p)
+        : "r"(d), "r"(1u << b));
+  return p;
+}
+
+template <class S>
+struct PassArgs {
+  const uint32_t* kin;
+  const uint32_t* p0in;
+  const uint32_t* p1in;
+  uint32_t* kout;
+  uint32_t* p0out;
+  uint32_t* p1out;
+  uint32_t n, shift, mask;
+  const uint32_t* digit_base;
+  S* status;
+  uint32_t* tile_ctr;
+  uint32_t* err;
+};
+
 // One pass over one tile.  Only the keys pass through registers: once the
 // tile-local digit prefix is known, each payload element is copied from
 // global memory straight into its slot of the digit-ordered stage by an
 // asynchronous copy, and those copies land while the look-back runs; the
 // kernel holds no payload registers.  Keys and payloads are then written out
-// run by run (consecutive threads, consecutive addresses).  Shared memory: a
-// stage per array (32 KB unweighted: four CTAs per SM; 48 KB weighted: three).
-template <bool HAS_P1>
-__global__ void __launch_bounds__(kSortThreads, HAS_P1 ? 3 : 4)
-onesweep_kernel(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ p0in,
-                const uint32_t* __restrict__ p1in, uint32_t* __restrict__ kout,
-                uint32_t* __restrict__ p0out, uint32_t* __restrict__ p1out, uint32_t n,
-                uint32_t shift, uint32_t mask, const uint32_t* __restrict__ digit_base,
-                unsigned long long* __restrict__ status, uint32_t* __restrict__ tile_ctr,
-                uint32_t* __restrict__ err) {
-  __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_whist[kWarps][256];
-  __shared__ uint32_t s_local_start[256];
-  __shared__ uint32_t s_global_start[256];
-  __shared__ uint32_t s_warp[kWarps];
-  extern __shared__ uint32_t s_dyn[];  // kTile keys, kTile payload0 [, kTile payload1]
+// run by run (consecutive threads, consecutive addresses).
+// A pass is bound by instructions and latency, not by DRAM (31 % of its peak):
+// so a full tile has no bounds checks, a rank is kept with its digit in one
+// word, the leader of a digit is the lane with none before it, and the warp
+// histograms hold 16-bit counts, which with 64 (weighted) and 48 registers
+// gives four and five CTAs per SM.  One pass of 67 M keys by a 7-bit digit:
+// 655 -> 435 us weighted (24 bytes per key: 3.7 TB/s), 627 -> 317 us unweighted
+// (3.4 TB/s), against the version with match masks, 64-bit status words, one
+// look-back word at a time and 32-bit histograms.  512 threads (476 us), 20 keys
+// per thread (457 us) and payloads through registers were slower.
+template <bool HAS_P1, int NB, class S, bool FULL>
+__device__ __forceinline__ void onesweep_tile(const PassArgs<S>& a, uint32_t tile, uint32_t* s_dyn,
+                                              uint16_t (*s_whist)[256], uint32_t* s_global_start, uint32_t* s_warp) {
   uint32_t* s_k = s_dyn;
   uint32_t* s_p0 = s_dyn + kTile;
   uint32_t* s_p1 = s_dyn + 2 * kTile;
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_tile = atomicAdd(tile_ctr, 1u);
-  for (int i = tid; i < kWarps * 256; i += kSortThreads) (&s_whist[0][0])[i] = 0;
-  __syncthreads();
-  const uint32_t tile = s_tile;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint64_t tile_base = (uint64_t)tile * kTile;
   const uint64_t warp_base = tile_base + (uint64_t)warp * 32 * kSortItems;
   // this warp's items: [0, wn) of kSortItems * 32, addressed from per-warp bases
-  const uint32_t wn = n > warp_base ? (uint32_t)min((uint64_t)kSortItems * 32, (uint64_t)n - warp_base) : 0u;
-  const uint32_t* kw = kin + warp_base;
+  const uint32_t wn = FULL ? 32 * kSortItems
+                           : (a.n > warp_base ? (uint32_t)min((uint64_t)kSortItems * 32, (uint64_t)a.n - warp_base) : 0u);
+  const uint32_t* kw = a.kin + warp_base + lane;
 
-  uint32_t key[kSortItems], pos[kSortItems];
+  uint32_t key[kSortItems], rank[kSortItems];  // rank: digit << 16 | position among the warp's equal digits
 #pragma unroll
-  for (int i = 0; i < kSortItems; i++) {
-    const uint32_t o = (uint32_t)i * 32 + lane;
-    key[i] = o < wn ? kw[o] : 0xFFFFFFFFu;
-  }
+  for (int i = 0; i < kSortItems; i++) key[i] = (FULL || (uint32_t)i * 32 + lane < wn) ? kw[i * 32] : 0xFFFFFFFFu;
 
   // Stable warp-level ranking: order within the warp is (item, lane).
-  uint32_t* wh = s_whist[warp];
+  uint16_t* wh = s_whist[warp];
+  const uint32_t before_me = lanemask_lt();
 #pragma unroll
   for (int i = 0; i < kSortItems; i++) {
-    const uint32_t d = ((uint32_t)i * 32 + lane < wn) ? ((key[i] >> shift) & mask) : 256u;
-    const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    uint32_t before = (d < 256) ? wh[d] : 0u;
+    const uint32_t d = (key[i] >> a.shift) & a.mask;
+    const bool in = FULL || (uint32_t)i * 32 + lane < wn;
+    const uint32_t peers = digit_peers<NB>(d, FULL ? 0xffffffffu : __ballot_sync(0xffffffffu, in));
+    const uint32_t seen = wh[d];
+    const uint32_t r = __popc(peers & before_me);
     __syncwarp();
-    if (d < 256 && lane == __ffs(peers) - 1) wh[d] = before + __popc(peers);
+    if (r == 0 && in) wh[d] = (uint16_t)(seen + __popc(peers));
     __syncwarp();
-    pos[i] = before + __popc(peers & lanemask_lt());
+    rank[i] = seen + r + (d << 16);
   }
   __syncthreads();
 
-  // Per digit (thread = digit): exclusive prefix over warps, tile count.
-  uint32_t cnt = 0;
+  // Per digit (thread = digit): tile count, published, and its start in the
+  // tile; each warp's histogram entry becomes the warp's start in the digit.
+  static_assert(kSortThreads == 256, "a thread per digit");
+  uint32_t cnt = 0, c[kWarps];
 #pragma unroll
   for (int w = 0; w < kWarps; w++) {
-    uint32_t c = s_whist[w][tid];
-    s_whist[w][tid] = cnt;
-    cnt += c;
+    c[w] = s_whist[w][tid];
+    cnt += c[w];
   }
   // digits above the mask never occur in this pass: no status, no look-back
-  const bool live = (uint32_t)tid <= mask;
-  unsigned long long* my_status = status + (uint64_t)tile * 256 + tid;
-  if (live) st_volatile_u64(my_status, (tile == 0 ? kFlagInc : kFlagAgg) | cnt);
+  const bool live = tid <= a.mask;
+  S* my_status = a.status + (uint64_t)tile * 256 + tid;
+  if (live) lb_store(my_status, (tile == 0 ? LbWord<S>::kInc : LbWord<S>::kAgg) | (S)cnt);
   const uint32_t local_start = block_exclusive_scan_256(cnt, s_warp);
-  s_local_start[tid] = local_start;
+  uint32_t at = local_start;
+#pragma unroll
+  for (int w = 0; w < kWarps; w++) {
+    s_whist[w][tid] = (uint16_t)at;
+    at += c[w];
+  }
   __syncthreads();
 
   // Stage slots (digit order within the tile): keys staged, payloads copied
   // into their slots asynchronously.
   {
-    const uint32_t* p0w = p0in + warp_base;
-    const uint32_t* p1w = HAS_P1 ? p1in + warp_base : nullptr;
+    const uint32_t* p0w = a.p0in + warp_base + lane;
+    const uint32_t* p1w = HAS_P1 ? a.p1in + warp_base + lane : nullptr;
 #pragma unroll
     for (int i = 0; i < kSortItems; i++) {
-      const uint32_t o = (uint32_t)i * 32 + lane;
-      if (o < wn) {
-        const uint32_t d = (key[i] >> shift) & mask;
-        const uint32_t p = s_local_start[d] + s_whist[warp][d] + pos[i];
+      if (FULL || (uint32_t)i * 32 + lane < wn) {
+        const uint32_t p = wh[rank[i] >> 16] + (rank[i] & 0xFFFFu);
         s_k[p] = key[i];
-        cp_async_u32(&s_p0[p], p0w + o);
-        if (HAS_P1) cp_async_u32(&s_p1[p], p1w + o);
+        cp_async_u32(&s_p0[p], p0w + i * 32);
+        if (HAS_P1) cp_async_u32(&s_p1[p], p1w + i * 32);
       }
     }
   }
 
-  // Decoupled look-back over earlier tiles for this digit.
+  // Decoupled look-back over earlier tiles for this digit, kLookBack of them
+  // read at once (one at a time: 613 -> 562 us for a weighted pass).
   uint32_t excl = 0;
   if (tile > 0 && live) {
     int64_t pred = (int64_t)tile - 1;
+    const S* col = a.status + tid;
     uint32_t spins = 0;
-    while (pred >= 0) {
-      unsigned long long s = ld_volatile_u64(status + (uint64_t)pred * 256 + tid);
-      unsigned long long flag = s & ~0xFFFFFFFFull;
-      if (flag == 0) {
-        if (++spins > kSpinLimit) {
-          atomicExch(err, (uint32_t)ERR_SPIN);
+    bool done = false;
+    while (!done && pred >= 0) {
+      S s[kLookBack];
+#pragma unroll
+      for (int q = 0; q < kLookBack; q++)
+        s[q] = pred - q >= 0 ? lb_load(col + (uint64_t)(pred - q) * 256) : LbWord<S>::kInc;
+#pragma unroll
+      for (int q = 0; q < kLookBack; q++) {
+        if (done) continue;
+        const S flag = s[q] & LbWord<S>::kFlag;
+        if (flag == 0) {
+          if (++spins > kSpinLimit) {
+            atomicExch(a.err, (uint32_t)ERR_SPIN);
+            done = true;
+          }
           break;
         }
-        continue;
+        excl += (uint32_t)(s[q] & ~LbWord<S>::kFlag);
+        --pred;
+        if (flag == LbWord<S>::kInc) done = true;
       }
-      excl += (uint32_t)s;
-      if (flag == kFlagInc) break;
-      --pred;
     }
-    st_volatile_u64(my_status, kFlagInc | (unsigned long long)(excl + cnt));
+    lb_store(my_status, LbWord<S>::kInc | (S)(excl + cnt));
   }
-  s_global_start[tid] = digit_base[tid] + excl - local_start;
+  s_global_start[tid] = a.digit_base[tid] + excl - local_start;
   cp_async_commit_wait_all();
   __syncthreads();
 
-  const uint32_t valid = (uint32_t)min((uint64_t)kTile, (uint64_t)n - tile_base);
-#pragma unroll 4
-  for (uint32_t j = tid; j < valid; j += kSortThreads) {
-    const uint32_t k = s_k[j];
-    const uint32_t o = s_global_start[(k >> shift) & mask] + j;
-    kout[o] = k;
-    p0out[o] = s_p0[j];
-    if (HAS_P1) p1out[o] = s_p1[j];
+  if (FULL) {
+    constexpr int U = 4;
+    static_assert(kSortItems % U == 0, "whole groups");
+#pragma unroll 1
+    for (uint32_t j0 = tid; j0 < kTile; j0 += U * kSortThreads) {
+      uint32_t k[U], o[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) k[u] = s_k[j0 + u * kSortThreads];
+#pragma unroll
+      for (int u = 0; u < U; u++) o[u] = s_global_start[(k[u] >> a.shift) & a.mask] + j0 + u * kSortThreads;
+#pragma unroll
+      for (int u = 0; u < U; u++) a.kout[o[u]] = k[u];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        a.p0out[o[u]] = s_p0[j0 + u * kSortThreads];
+        if (HAS_P1) a.p1out[o[u]] = s_p1[j0 + u * kSortThreads];
+      }
+    }
+  } else {
+    const uint32_t valid = (uint32_t)min((uint64_t)kTile, (uint64_t)a.n - tile_base);
+    for (uint32_t j = tid; j < valid; j += kSortThreads) {
+      const uint32_t k = s_k[j];
+      const uint32_t o = s_global_start[(k >> a.shift) & a.mask] + j;
+      a.kout[o] = k;
+      a.p0out[o] = s_p0[j];
+      if (HAS_P1) a.p1out[o] = s_p1[j];
+    }
   }
+}
+
+template <bool HAS_P1, int NB, class S>
+__global__ void __launch_bounds__(kSortThreads, HAS_P1 ? 4 : 5) onesweep_kernel(PassArgs<S> a) {
+  __shared__ uint32_t s_tile;
+  __shared__ uint16_t s_whist[kWarps][256];
+  __shared__ uint32_t s_global_start[256];
+  __shared__ uint32_t s_warp[kWarps];
+  extern __shared__ uint32_t s_dyn[];  // kTile keys, kTile payload0 [, kTile payload1]
+  if (threadIdx.x == 0) s_tile = atomicAdd(a.tile_ctr, 1u);
+  for (int i = threadIdx.x; i < kWarps * 128; i += kSortThreads) reinterpret_cast<uint32_t*>(s_whist)[i] = 0;
+  __syncthreads();
+  const uint32_t tile = s_tile;
+  if (((uint64_t)tile + 1) * kTile <= a.n)
+    onesweep_tile<HAS_P1, NB, S, true>(a, tile, s_dyn, s_whist, s_global_start, s_warp);
+  else
+    onesweep_tile<HAS_P1, NB, S, false>(a, tile, s_dyn, s_whist, s_global_start, s_warp);
+}
+
+template <bool HAS_P1, int NB, class S>
+static int launch_pass_of(const PassArgs<S>& a, cudaStream_t stream) {
+  constexpr size_t smem = (size_t)(HAS_P1 ? 3 : 2) * kTile * sizeof(uint32_t);  // a stage per array
+  const auto kernel = onesweep_kernel<HAS_P1, NB, S>;
+  OGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  OGB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                cudaSharedmemCarveoutMaxShared));
+  kernel<<<ceil_div(a.n, kTile), kSortThreads, smem, stream>>>(a);
+  OGB_CUDA(cudaGetLastError());
+  return OK;
+}
+
+// One pass: the variant without the second payload when there is none, and
+// seven ballots instead of eight when the digit has at most seven bits.
+template <class S>
+static int launch_pass(const PassArgs<S>& a, cudaStream_t stream) {
+  const bool p1 = a.p1in != nullptr, narrow = a.mask < 128;
+  if (p1) return narrow ? launch_pass_of<true, 7>(a, stream) : launch_pass_of<true, 8>(a, stream);
+  return narrow ? launch_pass_of<false, 7>(a, stream) : launch_pass_of<false, 8>(a, stream);
 }
 
 struct PinnedCounts {
@@ -306,10 +424,14 @@ struct PassPlan {
 
 }  // namespace
 
+static size_t status_word_bytes(uint64_t n) {
+  return n < kNarrowLimit ? sizeof(uint32_t) : sizeof(unsigned long long);
+}
+
 int SortWorkspace::reserve(uint64_t n, bool weighted, int max_passes) {
   const uint64_t tiles = (n + kTile - 1) / kTile;
   OGB_TRY(hist.alloc(2 * 8 * 256 * sizeof(uint32_t)));
-  OGB_TRY(status.alloc((size_t)max_passes * tiles * 256 * sizeof(unsigned long long) + 256));
+  OGB_TRY(status.alloc((size_t)max_passes * tiles * 256 * status_word_bytes(n) + 256));
   OGB_TRY(counters.alloc(kCtrWords * sizeof(uint32_t)));
   OGB_TRY(tmp_k.alloc(n * 4));
   OGB_TRY(tmp_v0.alloc(n * 4));
@@ -369,34 +491,39 @@ static int sort_impl(const KV& in, const KV& out, uint64_t n, bool lex, uint32_t
     return OK;
   }
   const uint64_t tiles = (n + kTile - 1) / kTile;
-  const size_t dyn_smem = (size_t)(has_p1 ? 3 : 2) * kTile * sizeof(uint32_t);  // a stage per array
-  static bool attr_set = false;
-  if (!attr_set) {
-    OGB_CUDA(cudaFuncSetAttribute(onesweep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * kTile * 4));
-    OGB_CUDA(cudaFuncSetAttribute(onesweep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kTile * 4));
-    attr_set = true;
-  }
-  OGB_CUDA(cudaMemsetAsync(ws.status.p, 0, (size_t)P * tiles * 256 * sizeof(unsigned long long), stream));
+  const size_t word = status_word_bytes(n);
+  OGB_CUDA(cudaMemsetAsync(ws.status.p, 0, (size_t)P * tiles * 256 * word, stream));
 
   KV tmp{ws.tmp_k.as<uint32_t>(), ws.tmp_v0.as<uint32_t>(), has_p1 ? ws.tmp_v1.as<uint32_t>() : nullptr};
   KV cur = in;
   for (int i = 0; i < P; i++) {
     const KV dst = ((P - 1 - i) % 2 == 0) ? out : tmp;
     const PassPlan& pp = plan[i];
-    const uint32_t* kin = pp.role == 0 ? cur.k : cur.v0;
-    const uint32_t* p0in = pp.role == 0 ? cur.v0 : cur.k;
-    uint32_t* kout = pp.role == 0 ? dst.k : dst.v0;
-    uint32_t* p0out = pp.role == 0 ? dst.v0 : dst.k;
-    unsigned long long* st = ws.status.as<unsigned long long>() + (uint64_t)i * tiles * 256;
-    if (has_p1)
-      onesweep_kernel<true><<<(unsigned)tiles, kSortThreads, dyn_smem, stream>>>(
-          kin, p0in, cur.v1, kout, p0out, dst.v1, (uint32_t)n, pp.shift, pp.mask, d_base + pp.hist_index * 256, st,
-          d_ctr + i, d_ctr + kCtrErr);
-    else
-      onesweep_kernel<false><<<(unsigned)tiles, kSortThreads, dyn_smem, stream>>>(
-          kin, p0in, nullptr, kout, p0out, nullptr, (uint32_t)n, pp.shift, pp.mask, d_base + pp.hist_index * 256, st,
-          d_ctr + i, d_ctr + kCtrErr);
-    OGB_CUDA(cudaGetLastError());
+    char* st = ws.status.as<char>() + (uint64_t)i * tiles * 256 * word;
+    const auto fill = [&](auto& a) {
+      a.kin = pp.role == 0 ? cur.k : cur.v0;
+      a.p0in = pp.role == 0 ? cur.v0 : cur.k;
+      a.p1in = has_p1 ? cur.v1 : nullptr;
+      a.kout = pp.role == 0 ? dst.k : dst.v0;
+      a.p0out = pp.role == 0 ? dst.v0 : dst.k;
+      a.p1out = has_p1 ? dst.v1 : nullptr;
+      a.n = (uint32_t)n;
+      a.shift = pp.shift;
+      a.mask = pp.mask;
+      a.digit_base = d_base + pp.hist_index * 256;
+      a.status = reinterpret_cast<decltype(a.status)>(st);
+      a.tile_ctr = d_ctr + i;
+      a.err = d_ctr + kCtrErr;
+    };
+    if (word == sizeof(uint32_t)) {
+      PassArgs<uint32_t> a;
+      fill(a);
+      OGB_TRY(launch_pass(a, stream));
+    } else {
+      PassArgs<unsigned long long> a;
+      fill(a);
+      OGB_TRY(launch_pass(a, stream));
+    }
     cur = dst;
   }
   return OK;

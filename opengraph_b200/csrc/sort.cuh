@@ -14,7 +14,7 @@ struct KV {
 
 struct SortWorkspace {
   DevBuf hist;       // passes*256 u32 counts, then passes*256 exclusive bases
-  DevBuf status;     // look-back words: passes * tiles * 256 u64
+  DevBuf status;     // look-back words: passes * tiles * 256 of 4 bytes (8 from 2^30 keys on)
   DevBuf counters;   // per-pass tile counters + error word
   DevBuf tmp_k, tmp_v0, tmp_v1;  // one ping-pong array set
   int reserve(uint64_t n, bool weighted, int max_passes);
