@@ -99,9 +99,7 @@ struct BfsCtl {
   uint32_t scan_tiles;       // tile counter of the degree scan
   uint32_t all_count;        // host-state step: entries written to all_out
   unsigned long long edges;  // bottom-up: edges examined
-  unsigned long long reached_edges;
-  uint32_t reached;
-  uint32_t maxdeg;            // largest out-degree on the next expansion list
+  uint32_t maxdeg, pad;            // largest out-degree on the next expansion list
   unsigned long long fedges;  // out-edges of the vertices the step discovered
 };
 
@@ -126,6 +124,12 @@ struct BfsCtrl {
 // Inputs of the learned direction switch, from the state before a step.
 constexpr int kFeat = 8;
 
+// One step of the trace and the switch inputs before it.
+struct BfsStep {
+  BfsLevel level;
+  float feat[kFeat];
+};
+
 struct BfsDevState {
   BfsCtrl c;
   int32_t* parents;
@@ -134,10 +138,12 @@ struct BfsDevState {
   uint32_t bar;       // grid barrier word
   uint32_t pad[2];
   BfsCtl ctl[3];      // per-phase counters, rotating
-  BfsCtl aux;         // reached counts and the host-state steps
-  BfsLevel trace[kMaxTrace];
-  float feat[kMaxTrace][kFeat];  // switch inputs before every step
+  BfsCtl aux;         // the host-state steps
+  BfsStep steps[kMaxTrace];
 };
+
+constexpr uint32_t kFirstSteps = 32;
+constexpr size_t kStateCopy = offsetof(BfsDevState, steps) + kFirstSteps * sizeof(BfsStep);
 
 // Device buffers of one graph (fixed; passed by value to every kernel).
 struct BfsBufs {
@@ -173,12 +179,12 @@ const float* bfs_policy_tail();
 struct BfsWork {
   uint32_t V = 0, E = 0;
   DevBuf q0, q1, bm0, bm1, bm2, ul0, ul1, state;
-  DevBuf offs, fstart, fdist, tile_i0, scan_status;
+  DevBuf offs, fstart, fdist, tile_i0, scan_status, roots;
   DevBuf cand_a, cand_b;            // records of the vertices with in-edges (built once per graph)
   DevBuf ul_a0, ul_a1, ul_b0, ul_b1;  // records of the unvisited lists (at most n_cand0 each)
   uint32_t n_cand0 = 0, cand0_build = 0;
   bool cand0_ready = false;
-  BfsDevState* h_state = nullptr;   // pinned copy of the header only (up to the trace)
+  BfsDevState* h_state = nullptr;   // pinned copy of the first kStateCopy bytes
   uint32_t epoch = 0;               // last scan epoch used
   int search_grid = 0;          // CTAs of the search launch (co-resident)
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
@@ -215,9 +221,9 @@ static int bfs_work_get(DevGraph& g, BfsWork** out) {
     w->V = V;
     w->E = E;
   }
-  // the header (control state, error word, counters) is all the host reads
-  // back through it; the trace arrays after it are copied on request
-  if (!w->h_state) OGB_CUDA(cudaMallocHost(&w->h_state, offsetof(BfsDevState, trace)));
+  // the host reads back the header (control state, error word, counters) and,
+  // in the same copy, the first kFirstSteps steps of the trace; more on request
+  if (!w->h_state) OGB_CUDA(cudaMallocHost(&w->h_state, kStateCopy));
   if (!w->ev_start) {
     OGB_CUDA(cudaEventCreate(&w->ev_start));
     OGB_CUDA(cudaEventCreate(&w->ev_stop));
@@ -1332,7 +1338,7 @@ __device__ void ctrl_level(BfsCtrl& c, BfsDevState* st, bool leader, uint32_t di
     L.mu = c.mu;
     L.edges = edges;
     L.ms = (float)((double)(global_ns() - t0) * 1e-6);
-    st->trace[c.nlevels] = L;
+    st->steps[c.nlevels].level = L;
   }
   c.nlevels++;
   c.iteration++;
@@ -1507,26 +1513,45 @@ __global__ void __launch_bounds__(256) bfsk_init(BfsBufs b, BfsDevState* st, uin
 // More roots after bfsk_init's first one (a search over a disjoint union of
 // graphs, one root each): each gets itself as parent and its frontier bit,
 // joins the queue (and the expansion list when it has out-edges); mf sums
-// their out-degrees.  Duplicates are skipped.  One thread, after bfsk_init.
-__global__ void bfsk_set_roots(BfsBufs b, BfsDevState* st, const uint32_t* __restrict__ roots, uint32_t n) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  int32_t* parents = st->parents;
-  BfsCtrl c = st->c;
-  for (uint32_t i = 1; i < n; i++) {
-    const uint32_t r = roots[i];
-    if (parents[r] == (int32_t)r) continue;
-    parents[r] = (int32_t)r;
-    b.bm[0][r >> 5] |= 1u << (r & 31);
-    const uint32_t d = b.out_degree[r];
-    c.lmax = max(c.lmax, d);
-    c.qcount++;
-    c.processed++;
-    c.mf += d;
-    c.fedges += d;
-    c.edges_visited += d;
-    if (d) b.list[0][c.lsize++] = r;
+// their out-degrees.  Duplicates are skipped (the first claim of a parent entry
+// counts).  One CTA, after bfsk_init, a thread per root: one thread walking
+// 96 roots alone took 132 us.
+__global__ void __launch_bounds__(1024) bfsk_set_roots(BfsBufs b, BfsDevState* st, const uint32_t* __restrict__ roots,
+                                                       uint32_t n) {
+  __shared__ uint32_t s_q, s_l, s_mf, s_max;
+  __shared__ unsigned long long s_edges;
+  if (threadIdx.x == 0) {
+    s_q = s_mf = s_max = 0;
+    s_l = st->c.lsize;
+    s_edges = 0;
   }
-  st->c = c;
+  __syncthreads();
+  int32_t* parents = st->parents;
+  for (uint32_t i = 1 + threadIdx.x; i < n; i += blockDim.x) {
+    const uint32_t r = roots[i];
+    const int32_t p = parents[r];
+    if (p == (int32_t)r || atomicCAS(&parents[r], p, (int32_t)r) != p) continue;
+    atomicOr(&b.bm[0][r >> 5], 1u << (r & 31));
+    const uint32_t d = b.out_degree[r];
+    atomicAdd(&s_q, 1u);
+    if (d) {
+      atomicAdd(&s_mf, d);
+      atomicAdd(&s_edges, (unsigned long long)d);
+      atomicMax(&s_max, d);
+      b.list[0][atomicAdd(&s_l, 1u)] = r;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    BfsCtrl& c = st->c;
+    c.lsize = s_l;
+    c.lmax = max(c.lmax, s_max);
+    c.qcount += s_q;
+    c.processed += s_q;
+    c.mf += s_mf;
+    c.fedges += s_edges;
+    c.edges_visited += s_edges;
+  }
 }
 
 // The whole search: all CTAs co-resident (cooperative launch), one grid
@@ -1557,7 +1582,7 @@ __global__ void __launch_bounds__(kSearchT, 4) bfsk_search(BfsBufs b, BfsDevStat
       float f[kFeat];
       bfs_features(S, b.E, f);
       if (leader && S.nlevels < (uint32_t)kMaxTrace && !S.overflow)
-        for (int i = 0; i < kFeat; i++) st->feat[S.nlevels][i] = f[i];
+        for (int i = 0; i < kFeat; i++) st->steps[S.nlevels].feat[i] = f[i];
       bool bu = false, need = false;
       if (learned) {
         // z = prior . f + bias; the network adds at most +-bound, so it is
@@ -1696,23 +1721,6 @@ __global__ void bfsk_filter_list(const uint32_t* __restrict__ in, uint32_t n, co
   }
 }
 
-// Number of reached vertices and the sum of their out-degrees (Graph500
-// traversed edges), into st->aux.
-__global__ void __launch_bounds__(256) bfsk_reached(BfsBufs b, BfsDevState* st) {
-  __shared__ unsigned long long s_red[8];
-  const int32_t* parents = st->parents;
-  unsigned long long e = 0;
-  uint32_t r = 0;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < b.V; v += gridDim.x * blockDim.x) {
-    if (parents[v] >= 0) {
-      r++;
-      e += b.out_degree[v];
-    }
-  }
-  block_add_total<unsigned long long>(&st->aux.reached_edges, e, s_red);
-  block_add_total<uint32_t>(&st->aux.reached, r, reinterpret_cast<uint32_t*>(s_red));
-}
-
 // ------------------------------------------------------------ host copy ----
 
 // One byte of depth per vertex (a search of fewer than 255 levels): the host
@@ -1800,14 +1808,12 @@ static int bfs_cand0(DevGraph& g, BfsWork* w, cudaStream_t s) {
 }
 
 int bfs_run(DevGraph& g, uint32_t root, uint32_t mode, int32_t* parents, uint32_t* distances, BfsResult* res,
-            bool want_trace, bool bu_entry_nf_frontier, cudaStream_t s, bool want_reached) {
-  return bfs_run_roots(g, &root, 1, mode, parents, distances, res, want_trace, bu_entry_nf_frontier, s,
-                       want_reached);
+            bool want_trace, bool bu_entry_nf_frontier, cudaStream_t s) {
+  return bfs_run_roots(g, &root, 1, mode, parents, distances, res, want_trace, bu_entry_nf_frontier, s);
 }
 
 int bfs_run_roots(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint32_t mode, int32_t* parents,
-                  uint32_t* distances, BfsResult* res, bool want_trace, bool bu_entry_nf_frontier, cudaStream_t s,
-                  bool want_reached) {
+                  uint32_t* distances, BfsResult* res, bool want_trace, bool bu_entry_nf_frontier, cudaStream_t s) {
   const uint32_t V = g.V;
   if (nroots == 0) return fail(ERR_ARG, "bfs: no root");
   for (uint32_t i = 0; i < nroots; i++)
@@ -1832,23 +1838,17 @@ int bfs_run_roots(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint32_t 
   }
   bfsk_init<<<sm_count() * 8, 256, 0, s>>>(b, st, root, parents, distances, mode, bu_entry_nf_frontier ? 1u : 0u,
                                             g.E, w->epoch, w->n_cand0);
-  DevBuf d_roots;
   if (nroots > 1) {
-    OGB_TRY(d_roots.alloc((size_t)nroots * 4));
-    OGB_CUDA(cudaMemcpyAsync(d_roots.p, roots, (size_t)nroots * 4, cudaMemcpyHostToDevice, s));
-    bfsk_set_roots<<<1, 32, 0, s>>>(b, st, d_roots.as<uint32_t>(), nroots);
+    OGB_TRY(w->roots.alloc((size_t)nroots * 4));
+    OGB_CUDA(cudaMemcpyAsync(w->roots.p, roots, (size_t)nroots * 4, cudaMemcpyHostToDevice, s));
+    bfsk_set_roots<<<1, 1024, 0, s>>>(b, st, w->roots.as<uint32_t>(), nroots);
   }
   OGB_CUDA(cudaGetLastError());
   OGB_CUDA(cudaEventRecord(w->ev_start, s));
   void* args[] = {(void*)&b, (void*)&st};
   OGB_CUDA(cudaLaunchCooperativeKernel((void*)bfsk_search, dim3(w->search_grid), dim3(kSearchT), args, 0, s));
   OGB_CUDA(cudaEventRecord(w->ev_stop, s));
-  OGB_CUDA(cudaMemsetAsync(&st->aux, 0, sizeof(BfsCtl), s));
-  if (want_reached) {
-    bfsk_reached<<<sm_count() * 8, 256, 0, s>>>(b, st);
-    OGB_CUDA(cudaGetLastError());
-  }
-  OGB_CUDA(cudaMemcpyAsync(w->h_state, w->state.p, offsetof(BfsDevState, trace), cudaMemcpyDeviceToHost, s));
+  OGB_CUDA(cudaMemcpyAsync(w->h_state, w->state.p, kStateCopy, cudaMemcpyDeviceToHost, s));
   OGB_CUDA(cudaStreamSynchronize(s));
   float total_ms = 0.f;
   OGB_CUDA(cudaEventElapsedTime(&total_ms, w->ev_start, w->ev_stop));
@@ -1864,18 +1864,30 @@ int bfs_run_roots(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint32_t 
   r.td_steps = h->c.td_steps;
   r.bu_steps = h->c.bu_steps;
   r.edges_examined = h->c.edges_examined;
-  r.reached = h->aux.reached;
-  r.reached_out_edges = h->aux.reached_edges;
+  // every reached vertex is counted once, by the step that discovers it, with
+  // its out-edges (a separate pass over all vertices for these two counts took
+  // 18 us at RMAT-22)
+  r.reached = h->c.processed;
+  r.reached_out_edges = h->c.edges_visited;
   r.ms = total_ms;
   r.launches = 1;  // kernels in the timed region: the search (init runs before it)
   r.nlevels = (int)h->c.nlevels;
   const uint32_t ntrace = std::min<uint32_t>(h->c.nlevels, kMaxTrace);
   if (want_trace && ntrace) {
+    std::vector<BfsStep> more;
+    if (ntrace > kFirstSteps) {
+      more.resize(ntrace - kFirstSteps);
+      OGB_CUDA(cudaMemcpyAsync(more.data(), st->steps + kFirstSteps, sizeof(BfsStep) * more.size(),
+                               cudaMemcpyDeviceToHost, s));
+      OGB_CUDA(cudaStreamSynchronize(s));
+    }
     r.levels.resize(ntrace);
     r.feat.resize((size_t)ntrace * kFeat);
-    OGB_CUDA(cudaMemcpyAsync(r.levels.data(), st->trace, sizeof(BfsLevel) * ntrace, cudaMemcpyDeviceToHost, s));
-    OGB_CUDA(cudaMemcpyAsync(r.feat.data(), st->feat, sizeof(float) * kFeat * ntrace, cudaMemcpyDeviceToHost, s));
-    OGB_CUDA(cudaStreamSynchronize(s));
+    for (uint32_t i = 0; i < ntrace; i++) {
+      const BfsStep& x = i < kFirstSteps ? h->steps[i] : more[i - kFirstSteps];
+      r.levels[i] = x.level;
+      std::copy(x.feat, x.feat + kFeat, r.feat.begin() + (size_t)i * kFeat);
+    }
   }
   if (res) *res = std::move(r);
   return OK;
@@ -1921,7 +1933,7 @@ int bfs_td_step_host(DevGraph& g, const uint32_t* q, uint32_t qsize, int32_t* pa
                                                          d_all.as<uint32_t>());
     OGB_CUDA(cudaGetLastError());
   }
-  OGB_CUDA(cudaMemcpyAsync(w->h_state, w->state.p, offsetof(BfsDevState, trace), cudaMemcpyDeviceToHost, s));
+  OGB_CUDA(cudaMemcpyAsync(w->h_state, w->state.p, offsetof(BfsDevState, steps), cudaMemcpyDeviceToHost, s));
   OGB_CUDA(cudaStreamSynchronize(s));
   if (w->h_state->err) return fail((int)w->h_state->err, "bfs step: a bounded device wait gave up");
   *next_size = w->h_state->aux.qnext;
@@ -1953,7 +1965,7 @@ int bfs_bu_step_host(DevGraph& g, const uint32_t* bm_cur, uint32_t* bm_next, int
   OGB_CUDA(cudaMemsetAsync(&st->aux, 0, sizeof(BfsCtl), s));
   bfsk_bu_host<<<sm_count() * 8, kSearchT, 0, s>>>(b, st, d_par.as<int32_t>(), d_dist.as<uint32_t>());
   OGB_CUDA(cudaGetLastError());
-  OGB_CUDA(cudaMemcpyAsync(w->h_state, w->state.p, offsetof(BfsDevState, trace), cudaMemcpyDeviceToHost, s));
+  OGB_CUDA(cudaMemcpyAsync(w->h_state, w->state.p, offsetof(BfsDevState, steps), cudaMemcpyDeviceToHost, s));
   OGB_CUDA(cudaStreamSynchronize(s));
   *nf = w->h_state->aux.nf;
   OGB_CUDA(cudaMemcpyAsync(bm_next, w->bm1.p, words * 4, cudaMemcpyDeviceToHost, s));
