@@ -476,11 +476,19 @@ int msbfs_run(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint16_t* dep
 // below epsilon, or after max_iterations.  A warp takes a vertex (or a chunk
 // of a long row): its four 8-lane groups walk the row's edges in turn, each
 // lane owning 4 seeds (one float4 of the row), four edges per group in
-// flight; the groups' sums are folded at the end.  Rows longer than
-// kPprChunk edges are cut into chunks (handed out one per claim, before the
-// other vertices, 64 per claim) whose sums the warp finishing the last one
-// adds in chunk order.  Dangling vertices' rank is not redistributed,
-// as in the reference.
+// flight; the groups' sums are folded at the end, and the update is one seed
+// per lane (by the eight lanes of one group, with four divisions and fp64 errors
+// each, it was most of the 17 warp instructions per edge).  The next vertex's
+// ids and old ranks load under the current one's gathers: an old rank loaded
+// when its sum is ready waited 5600 cycles on average (1370 us per iteration at
+// RMAT-20 against 376 with the early load; 588 us before both changes).  Rows
+// longer than kPprChunk
+// edges are cut into chunks (handed out one per claim, before the other
+// vertices, 32 per claim) whose sums the warp finishing the last one adds in
+// chunk order.  A vertex without in-edges keeps its teleport value, so after
+// the first two iterations, which write it into both contrib buffers, only the
+// vertices with in-edges are visited.  Dangling vertices' rank is not
+// redistributed, as in the reference.
 // ===========================================================================
 
 constexpr uint32_t kPprSeeds = 32;
@@ -491,7 +499,7 @@ struct PprCtl {
   double err[kPprMaxIters][kPprSeeds];
   uint32_t stop, stop_iter;
   uint32_t claim_chunk[kPprMaxIters];  // chunks handed out, one per claim
-  uint32_t claim_row[kPprMaxIters];    // other vertices handed out, 64 per claim
+  uint32_t claim_row[kPprMaxIters];    // other vertices handed out, 32 per claim
 };
 
 struct PprChunk {
@@ -501,8 +509,9 @@ struct PprChunk {
 struct PprWork {
   uint32_t V = 0, build = 0;
   bool ready = false;
-  DevBuf R, C0, C1, ctl, chunks, vfirst, vcount, done, partials, light;
-  uint32_t n_chunks = 0, n_cut = 0, n_light = 0;
+  DevBuf R, C0, C1, ctl, chunks, vfirst, vcount, done, partials, light, seeds;
+  uint32_t n_chunks = 0, n_cut = 0;
+  uint32_t n_light = 0, n_fed = 0;  // vertices in `light`; the first n_fed have in-edges
   PprCtl* h_ctl = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   ~PprWork() {
@@ -525,22 +534,32 @@ __global__ void pprk_seed(const uint32_t* __restrict__ seeds, uint32_t nseeds, c
   }
 }
 
-// Sum of the 32-float contrib rows of in-edges [j0, j1) (each lane: 4 seeds):
-// group g of 8 lanes takes edges g, g+4, g+8, g+12, then the next 16, four
-// rows in flight per group; the four groups are folded at the end.
-__device__ __forceinline__ float4 ppr_row_sum(const uint32_t* __restrict__ nbr, const float4* __restrict__ C4,
-                                              uint32_t j0, uint32_t j1, uint32_t grp, uint32_t sub) {
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (uint32_t j = j0 + grp; j < j1; j += 16) {
-    uint32_t u[4];
+// The seed of a lane in the update (every seed once over the warp).
+__device__ __forceinline__ uint32_t ppr_lane_seed(uint32_t lane) { return 4 * (lane & 7) + (lane >> 3); }
+
+// Ids of the 16 in-edges from j on: group g of 8 lanes has edges g, g + 4,
+// g + 8, g + 12 of them.
+struct PprIds {
+  uint32_t u[4];
+  __device__ __forceinline__ void load(const uint32_t* __restrict__ nbr, uint32_t j, uint32_t j1, uint32_t grp) {
 #pragma unroll
-    for (int q = 0; q < 4; q++) u[q] = (j + 4 * q < j1) ? (__ldg(&nbr[j + 4 * q]) & 0x3FFFFFFFu) : 0xFFFFFFFFu;
+    for (int q = 0; q < 4; q++) u[q] = (j + grp + 4 * q < j1) ? (__ldg(&nbr[j + grp + 4 * q]) & 0x3FFFFFFFu) : 0xFFFFFFFFu;
+  }
+};
+
+// Sum over the in-edges [j0, j1) of their source's 32 contribs, 16 edges at a
+// time (the first 16 ids come loaded); returns this lane's seed's sum.
+__device__ __forceinline__ float ppr_row_sum(const uint32_t* __restrict__ nbr, const float4* __restrict__ C4,
+                                             uint32_t j0, uint32_t j1, uint32_t grp, uint32_t sub, PprIds ids) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t j = j0; j < j1; j += 16) {
     float4 c[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       c[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (u[q] != 0xFFFFFFFFu) c[q] = __ldg(&C4[(size_t)u[q] * 8 + sub]);
+      if (ids.u[q] != 0xFFFFFFFFu) c[q] = __ldg(&C4[(size_t)ids.u[q] * 8 + sub]);
     }
+    if (j + 16 < j1) ids.load(nbr, j + 16, j1, grp);
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       acc.x += c[q].x;
@@ -557,7 +576,7 @@ __device__ __forceinline__ float4 ppr_row_sum(const uint32_t* __restrict__ nbr, 
     acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
     acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
   }
-  return acc;
+  return grp == 0 ? acc.x : (grp == 1 ? acc.y : (grp == 2 ? acc.z : acc.w));
 }
 
 struct PprParams {
@@ -567,42 +586,34 @@ struct PprParams {
   const uint32_t* seeds;
 };
 
-// Update of vertex v from its sums (lanes 0..7 hold seeds 4l..4l+3).
-__device__ __forceinline__ void ppr_update(uint32_t v, float4 s, uint32_t sub, const PprParams& p,
+// Update of vertex v from its sums: seed number k, vertex `seed`, on this lane.
+__device__ __forceinline__ void ppr_update(uint32_t v, float s, uint32_t k, uint32_t seed, const PprParams& p,
                                            const uint32_t* __restrict__ out_degree, float* __restrict__ R,
-                                           float* __restrict__ Cn, double* err4) {
-  const uint32_t d = out_degree[v];
-  float4* R4 = reinterpret_cast<float4*>(R) + (size_t)v * 8 + sub;
-  float4* C4 = reinterpret_cast<float4*>(Cn) + (size_t)v * 8 + sub;
-  const float4 old = *R4;
-  float sv[4] = {s.x, s.y, s.z, s.w}, ov[4] = {old.x, old.y, old.z, old.w}, nv[4], cv[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t k = sub * 4 + i;
-    const float tele = (k < p.nseeds && p.seeds[k] == v) ? p.base : 0.0f;
-    nv[i] = __fadd_rn(tele, __fmul_rn(p.damp, sv[i]));
-    cv[i] = d ? __fdiv_rn(nv[i], (float)d) : 0.0f;
-    err4[i] += fabs((double)nv[i] - (double)ov[i]);
-  }
-  *R4 = make_float4(nv[0], nv[1], nv[2], nv[3]);
-  *C4 = make_float4(cv[0], cv[1], cv[2], cv[3]);
+                                           float* __restrict__ Cn, double& err, float old, uint32_t d) {
+  const size_t at = (size_t)v * kPprSeeds + k;
+  const float nv = __fadd_rn(seed == v ? p.base : 0.0f, __fmul_rn(p.damp, s));
+  R[at] = nv;
+  Cn[at] = d ? __fdiv_rn(nv, (float)d) : 0.0f;
+  err += fabs((double)nv - (double)old);
 }
 
-__global__ void __launch_bounds__(256) pprk_iter(const PprChunk* __restrict__ chunks, uint32_t n_chunks,
-                                                 const uint32_t* __restrict__ vfirst,
-                                                 const uint32_t* __restrict__ vcount, uint32_t* __restrict__ done,
-                                                 float4* __restrict__ partials, const uint32_t* __restrict__ light,
-                                                 uint32_t n_light, const uint2* __restrict__ rows,
-                                                 const uint32_t* __restrict__ nbr,
-                                                 const uint32_t* __restrict__ out_degree, const float* __restrict__ C,
-                                                 float* __restrict__ Cn, float* __restrict__ R, PprParams p,
-                                                 PprCtl* __restrict__ ctl, uint32_t it) {
+__global__ void __launch_bounds__(256, 6) pprk_iter(const PprChunk* __restrict__ chunks, uint32_t n_chunks,
+                                                    const uint32_t* __restrict__ vfirst,
+                                                    const uint32_t* __restrict__ vcount, uint32_t* __restrict__ done,
+                                                    float* __restrict__ partials, const uint32_t* __restrict__ light,
+                                                    uint32_t n_light, const uint2* __restrict__ rows,
+                                                    const uint32_t* __restrict__ nbr,
+                                                    const uint32_t* __restrict__ out_degree,
+                                                    const float* __restrict__ C, float* __restrict__ Cn,
+                                                    float* __restrict__ R, PprParams p, PprCtl* __restrict__ ctl,
+                                                    uint32_t it) {
   __shared__ double s_err[8][kPprSeeds];
   if (ctl->stop) return;
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  const uint32_t grp = lane >> 3, sub = lane & 7;
+  const uint32_t grp = lane >> 3, sub = lane & 7, k = ppr_lane_seed(lane);
+  const uint32_t seed = k < p.nseeds ? p.seeds[k] : 0xFFFFFFFFu;
   const float4* C4 = reinterpret_cast<const float4*>(C);
-  double err4[4] = {0, 0, 0, 0};
+  double err = 0.0;
   // chunks of long rows, one per claim
   for (;;) {
     uint32_t t = 0;
@@ -610,45 +621,59 @@ __global__ void __launch_bounds__(256) pprk_iter(const PprChunk* __restrict__ ch
     t = __shfl_sync(0xffffffffu, t, 0);
     if (t >= n_chunks) break;
     const PprChunk ci = chunks[t];
-    const float4 s = ppr_row_sum(nbr, C4, ci.j0, ci.j1, grp, sub);
-    uint32_t last = 0;
-    if (lane < 8) partials[(size_t)t * 8 + sub] = s;
+    PprIds ids;
+    ids.load(nbr, ci.j0, ci.j1, grp);
+    partials[(size_t)t * kPprSeeds + k] = ppr_row_sum(nbr, C4, ci.j0, ci.j1, grp, sub, ids);
     __threadfence();
     __syncwarp();
+    uint32_t last = 0;
     if (lane == 0) last = (atomicAdd(&done[ci.k], 1u) == vcount[ci.k] - 1) ? 1u : 0u;
     last = __shfl_sync(0xffffffffu, last, 0);
     if (last) {
       __threadfence();
       const uint32_t f = vfirst[ci.k], cnt = vcount[ci.k];
-      float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (uint32_t c = 0; c < cnt; c++) {
-        const float4 q = __ldcg(&partials[(size_t)(f + c) * 8 + sub]);
-        tot.x += q.x;
-        tot.y += q.y;
-        tot.z += q.z;
-        tot.w += q.w;
-      }
-      if (lane < 8) ppr_update(ci.v, tot, sub, p, out_degree, R, Cn, err4);
+      float tot = 0.f;
+      for (uint32_t c = 0; c < cnt; c++) tot += __ldcg(&partials[(size_t)(f + c) * kPprSeeds + k]);
+      ppr_update(ci.v, tot, k, seed, p, out_degree, R, Cn, err, __ldcg(&R[(size_t)ci.v * kPprSeeds + k]), __ldg(&out_degree[ci.v]));
       if (lane == 0) done[ci.k] = 0;
     }
   }
-  // the other vertices, 64 per claim
+  // the other vertices, 32 per claim, their rows loaded a lane each
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(&ctl->claim_row[it], 64u);
+    if (lane == 0) base = atomicAdd(&ctl->claim_row[it], 32u);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= n_light) break;
-    const uint32_t end = min(base + 64, n_light);
-    for (uint32_t t = base; t < end; t++) {
-      const uint32_t v = light[t];
-      const uint2 r = rows[v];
-      const float4 s = ppr_row_sum(nbr, C4, r.x, r.x + r.y, grp, sub);
-      if (lane < 8) ppr_update(v, s, sub, p, out_degree, R, Cn, err4);
+    const uint32_t n = min(32u, n_light - base);
+    uint32_t mv = 0, md = 0;
+    uint2 mr = make_uint2(0u, 0u);
+    if (lane < n) {
+      mv = light[base + lane];
+      mr = rows[mv];
+      md = out_degree[mv];
+    }
+    uint32_t j0 = __shfl_sync(0xffffffffu, mr.x, 0), j1 = j0 + __shfl_sync(0xffffffffu, mr.y, 0);
+    PprIds ids;
+    ids.load(nbr, j0, j1, grp);
+    uint32_t v_next = __shfl_sync(0xffffffffu, mv, 0);
+    float old_next = R[(size_t)v_next * kPprSeeds + k];
+    for (uint32_t t = 0; t < n; t++) {
+      const uint32_t v = v_next;
+      const float old = old_next;
+      const uint32_t a0 = j0, a1 = j1;
+      const PprIds cur = ids;
+      // the next vertex's ids load under this one's gathers (n - 1: itself again)
+      const uint32_t tn = min(t + 1, n - 1);
+      j0 = __shfl_sync(0xffffffffu, mr.x, tn);
+      j1 = j0 + __shfl_sync(0xffffffffu, mr.y, tn);
+      ids.load(nbr, j0, j1, grp);
+      v_next = __shfl_sync(0xffffffffu, mv, tn);
+      old_next = R[(size_t)v_next * kPprSeeds + k];
+      const uint32_t d = __shfl_sync(0xffffffffu, md, t);
+      ppr_update(v, ppr_row_sum(nbr, C4, a0, a1, grp, sub, cur), k, seed, p, out_degree, R, Cn, err, old, d);
     }
   }
-  // per-seed error: lanes 0..7 hold seeds 4l..4l+3
-  if (lane < 8)
-    for (int i = 0; i < 4; i++) s_err[warp][lane * 4 + i] = err4[i];
+  s_err[warp][k] = err;
   __syncthreads();
   if (threadIdx.x < kPprSeeds) {
     double e = 0.0;
@@ -677,6 +702,7 @@ static int ppr_work_get(DevGraph& g, PprWork** out, cudaStream_t s) {
     OGB_TRY(w->C0.alloc((size_t)V * kPprSeeds * 4 + 64));
     OGB_TRY(w->C1.alloc((size_t)V * kPprSeeds * 4 + 64));
     OGB_TRY(w->ctl.alloc(sizeof(PprCtl) + 64));
+    OGB_TRY(w->seeds.alloc(kPprSeeds * 4));
     w->V = V;
     w->ready = false;
   }
@@ -702,10 +728,13 @@ static int ppr_work_get(DevGraph& g, PprWork** out, cudaStream_t s) {
         first.push_back((uint32_t)chunks.size());
         for (uint32_t c = 0; c < r.y; c += kPprChunk) chunks.push_back({v, r.x + c, r.x + std::min(r.y, c + kPprChunk), k});
         count.push_back((uint32_t)chunks.size() - first.back());
-      } else {
+      } else if (r.y) {
         light.push_back(v);
       }
     }
+    w->n_fed = (uint32_t)light.size();
+    for (uint32_t v = 0; v < V; v++)
+      if (!h_rows[v].y) light.push_back(v);
     w->n_light = (uint32_t)light.size();
     w->n_chunks = (uint32_t)chunks.size();
     w->n_cut = (uint32_t)first.size();
@@ -740,9 +769,7 @@ int ppr_run(DevGraph& g, const uint32_t* seeds, uint32_t nseeds, uint32_t max_it
     if (seeds[i] >= V) return fail(ERR_ARG, "ppr: seed %u out of range (V=%u)", seeds[i], V);
   PprWork* w = nullptr;
   OGB_TRY(ppr_work_get(g, &w, s));
-  DevBuf d_seeds;
-  OGB_TRY(d_seeds.alloc(kPprSeeds * 4));
-  OGB_CUDA(cudaMemcpyAsync(d_seeds.p, seeds, nseeds * 4, cudaMemcpyHostToDevice, s));
+  OGB_CUDA(cudaMemcpyAsync(w->seeds.p, seeds, nseeds * 4, cudaMemcpyHostToDevice, s));
   PprCtl* ctl = w->ctl.as<PprCtl>();
   float* C = w->C0.as<float>();
   float* Cn = w->C1.as<float>();
@@ -752,7 +779,7 @@ int ppr_run(DevGraph& g, const uint32_t* seeds, uint32_t nseeds, uint32_t max_it
   p.base = 1.0f - p.damp;
   p.eps = epsilon;
   p.nseeds = nseeds;
-  p.seeds = d_seeds.as<uint32_t>();
+  p.seeds = w->seeds.as<uint32_t>();
   const int sms = sm_count();
   OGB_CUDA(cudaEventRecord(w->ev0, s));
   OGB_CUDA(cudaMemsetAsync(ctl, 0, sizeof(PprCtl), s));
@@ -761,9 +788,9 @@ int ppr_run(DevGraph& g, const uint32_t* seeds, uint32_t nseeds, uint32_t max_it
   pprk_seed<<<1, 32, 0, s>>>(p.seeds, nseeds, g.fwd.d_out_degree(), R, C);
   OGB_CUDA(cudaGetLastError());
   for (uint32_t it = 0; it < max_iters; it++) {
-    pprk_iter<<<sms * 8, 256, 0, s>>>(w->chunks.as<PprChunk>(), w->n_chunks, w->vfirst.as<uint32_t>(),
-                                      w->vcount.as<uint32_t>(), w->done.as<uint32_t>(), w->partials.as<float4>(),
-                                      w->light.as<uint32_t>(), w->n_light, g.inv.d_rows(), g.inv.d_dst(),
+    pprk_iter<<<sms * 6, 256, 0, s>>>(w->chunks.as<PprChunk>(), w->n_chunks, w->vfirst.as<uint32_t>(),
+                                      w->vcount.as<uint32_t>(), w->done.as<uint32_t>(), w->partials.as<float>(),
+                                      w->light.as<uint32_t>(), it < 2 ? w->n_light : w->n_fed, g.inv.d_rows(), g.inv.d_dst(),
                                       g.fwd.d_out_degree(), C, Cn, R, p, ctl, it);
     pprk_check<<<1, 32, 0, s>>>(ctl, it, nseeds, epsilon);
     OGB_CUDA(cudaGetLastError());
