@@ -71,8 +71,33 @@ struct DdCtl {
   uint32_t done_a[kDdMaxIters];   // blocks of the iteration's first kernel that finished
   uint32_t done_b[kDdMaxIters];   // blocks of its second kernel that finished
   uint32_t stop, stop_iter;
-  uint32_t n_med, n_heavy, cur_med, cur_heavy;  // kept across runs of one graph build
+  uint32_t n_med, cur_heavy, n_hch;  // medium rows, heavy rows, their chunks: kept across runs of one graph build
   uint32_t n_och;                               // chunks of the long out-rows
+};
+
+// The heavy in-rows (more than kCtaThr edges) cut into chunks of kChunk edges:
+// chunks {v, first edge, end, heavy row}, and per heavy row its first chunk, its
+// chunk count and the chunks finished in the pass (0 between passes); a sum per
+// chunk.
+struct HeavyRows {
+  uint4* chunks;
+  uint32_t *first, *count, *done;
+  float* partials;
+};
+struct HeavyBuf {
+  DevBuf chunks, rows, partials;
+  size_t max_rows = 0;
+  int alloc(uint32_t E) {
+    max_rows = E / ((size_t)kCtaThr + 1) + 1;
+    const size_t max_chunks = max_rows + E / kChunk;
+    OGB_TRY(chunks.alloc(max_chunks * 16));
+    OGB_TRY(rows.alloc(max_rows * 12));
+    return partials.alloc(max_chunks * 4);
+  }
+  HeavyRows view() const {
+    uint32_t* r = rows.as<uint32_t>();
+    return {chunks.as<uint4>(), r, r + max_rows, r + 2 * max_rows, partials.as<float>()};
+  }
 };
 
 struct DdWork {
@@ -82,7 +107,8 @@ struct DdWork {
   // defer: out-row of v pushed / marked by the deferred-row kernel this
   // iteration; dvec: its push delta; selfcnt: self loops per vertex; och:
   // {v, j0, j1} chunks of the out-rows longer than kOutBig
-  DevBuf ctl, contrib, flags0, flags1, resid, med, heavy, defer, dvec, selfcnt, och, xin;
+  DevBuf ctl, contrib, flags0, flags1, resid, med, defer, dvec, selfcnt, och, xin;
+  HeavyBuf heavy;
   uint32_t n_och = 0;
   DdCtl* h_ctl = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -101,17 +127,6 @@ struct DdSlot {
 };
 std::mutex g_dd_mu;
 std::vector<DdSlot> g_dd;
-
-__global__ void dd_count_kernel(uint32_t V, const uint2* __restrict__ rows, DdCtl* __restrict__ ctl) {
-  uint32_t cm = 0, ch = 0;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    const uint32_t d = rows[v].y;
-    cm += (d > kWarpThr && d <= kCtaThr);
-    ch += (d > kCtaThr);
-  }
-  warp_atomic_add_total(&ctl->n_med, cm);
-  warp_atomic_add_total(&ctl->n_heavy, ch);
-}
 
 // Self loops per vertex (counted once per graph build).
 __global__ void dd_self_kernel(uint32_t E, const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst,
@@ -140,15 +155,38 @@ __global__ void dd_och_fill_kernel(uint32_t V, const uint2* __restrict__ rows_f,
   }
 }
 
-__global__ void dd_fill_kernel(uint32_t V, const uint2* __restrict__ rows, uint32_t* __restrict__ med,
-                               uint32_t* __restrict__ heavy, DdCtl* __restrict__ ctl) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    const uint32_t d = rows[v].y;
-    if (d > kCtaThr)
-      heavy[atomicAdd(&ctl->cur_heavy, 1u)] = v;
-    else if (d > kWarpThr)
-      med[atomicAdd(&ctl->cur_med, 1u)] = v;
+// The medium list and the heavy rows' chunks of the vertices [lo, hi).
+__global__ void dd_fill_kernel(uint32_t lo, uint32_t hi, const uint2* __restrict__ rows, uint32_t* __restrict__ med,
+                               HeavyRows h, DdCtl* __restrict__ ctl) {
+  for (uint32_t v = lo + blockIdx.x * blockDim.x + threadIdx.x; v < hi; v += gridDim.x * blockDim.x) {
+    const uint2 r = rows[v];
+    if (r.y > kCtaThr) {
+      const uint32_t k = atomicAdd(&ctl->cur_heavy, 1u), n = (r.y + kChunk - 1) / kChunk;
+      const uint32_t at = atomicAdd(&ctl->n_hch, n);
+      h.first[k] = at;
+      h.count[k] = n;
+      h.done[k] = 0;
+      for (uint32_t c = 0; c < n; c++)
+        h.chunks[at + c] = make_uint4(v, r.x + c * kChunk, r.x + min(r.y, (c + 1) * kChunk), k);
+    } else if (r.y > kWarpThr) {
+      med[warp_atomic_inc(&ctl->n_med)] = v;
+    }
   }
+}
+
+// Blocks of a pass by row class.
+struct Grid3 {
+  uint32_t light, med, heavy;
+  uint32_t total() const { return light + med + heavy; }
+};
+
+Grid3 rows_grid(uint32_t V) {
+  const uint32_t sms = sm_count();
+  Grid3 g;
+  g.light = std::max<uint32_t>(1, std::min<uint32_t>(sms * 8, ceil_div(V, kT)));
+  g.med = sms * 8;
+  g.heavy = sms * 2;
+  return g;
 }
 
 // ---- row sums in the GPU summation order -------------------------------------
@@ -180,52 +218,63 @@ __device__ __forceinline__ float warp_row_sum(uint32_t a, uint32_t d, const Term
   return s;
 }
 
-// Sum over a long row by the whole CTA (kCtaThreads threads): chunks of
-// kChunk edges, each chunk strided over the threads, warps folded, warp sums
-// added in warp order; chunk sums added in chunk order.  The total is valid
-// in thread 0.  Called by every thread of the CTA.
+// Sum over one chunk [j0, j1) of a long row by the whole CTA (kCtaThreads
+// threads strided, warps folded, warp sums added in warp order), valid in thread
+// 0.  Called by every thread of the CTA.
 template <class Term>
-__device__ float cta_row_sum(uint32_t a, uint32_t d, const Term& term, float* s_part) {
-  float tot = 0.0f;
-  for (uint32_t c = 0; c < d; c += kChunk) {
-    const uint32_t len = min(kChunk, d - c);
-    float s = strided_sum4(0.0f, a + c + threadIdx.x, a + c + len, kCtaThreads, term);
+__device__ float cta_chunk_sum(uint32_t j0, uint32_t j1, const Term& term, float* s_part) {
+  float s = strided_sum4(0.0f, j0 + threadIdx.x, j1, kCtaThreads, term);
 #pragma unroll
-    for (int o = 16; o; o >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
-    if (lane_id() == 0) s_part[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float ch = 0.0f;
-      for (uint32_t w = 0; w < kCtaThreads / 32; w++) ch = __fadd_rn(ch, s_part[w]);
-      tot = __fadd_rn(tot, ch);
-    }
-    __syncthreads();
-  }
-  return tot;
+  for (int o = 16; o; o >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+  if (lane_id() == 0) s_part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  float ch = 0.0f;
+  if (threadIdx.x == 0)
+    for (uint32_t w = 0; w < kCtaThreads / 32; w++) ch = __fadd_rn(ch, s_part[w]);
+  __syncthreads();
+  return ch;
 }
 
-// One pass over the rows of the inverse CSR in three classes: blocks
-// [0, nb_light) take the rows of at most kWarpThr edges (a thread each, in
-// CSR order), the next nb_med blocks the medium list (a warp each), the rest
-// the heavy list (a CTA each).  For each row with P.want(v): s = the row sum
-// of P.term(j) in the order above, light rows starting from P.start(v),
-// others P.start(v) + sum; then P.finish(v, s) (by lane 0 / thread 0 for the
-// warp and CTA rows).
+// One pass over the rows of the inverse CSR in three classes, by blocks
+// numbered b: [0, nb_heavy) take the chunks of the heavy rows (a CTA each; the
+// CTA that finishes a row's last chunk adds the chunk sums in chunk order), the
+// next nb_med the medium list (a warp each), the rest the rows of at most
+// kWarpThr edges (a thread each, in CSR order).  For each row with P.want(v): s
+// = the row sum of P.term(j) in the order above, light rows starting from
+// P.start(v), others P.start(v) + sum; then P.finish(v, s) (by lane 0 / thread 0
+// for the warp and CTA rows).  The heavy rows come first and in chunks: a CTA
+// per whole row, numbered last, left most SMs idle for half of a pass while the
+// hubs of 70 K edges were walked (SPMV at RMAT-20: 142 us).
 template <class P>
-__device__ void rows_pass(const uint2* __restrict__ rows, const uint32_t* __restrict__ med,
-                          const uint32_t* __restrict__ heavy, uint32_t n_med, uint32_t n_heavy, uint32_t V,
-                          uint32_t nb_light, uint32_t nb_med, P& pol) {
+__device__ void rows_pass(uint32_t b, const uint2* __restrict__ rows, const uint32_t* __restrict__ med,
+                          const HeavyRows& h, uint32_t n_med, uint32_t n_hch, uint32_t V, uint32_t nb_heavy,
+                          uint32_t nb_med, uint32_t nb_light, P& pol) {
   __shared__ float s_part[kT / 32];
-  const uint32_t b = blockIdx.x;
-  if (b < nb_light) {
-    for (uint32_t v = b * kT + threadIdx.x; v < V; v += nb_light * kT) {
-      const uint2 r = rows[v];
-      if (r.y > kWarpThr || !pol.want(v)) continue;
-      const float s = strided_sum4(pol.start(v), r.x, r.x + r.y, 1u, [&](uint32_t j) { return pol.term(j); });
-      pol.finish(v, s);
+  if (b < nb_heavy) {
+    for (uint32_t t = b; t < n_hch; t += nb_heavy) {
+      const uint4 ci = h.chunks[t];
+      if (!pol.want(ci.x)) continue;  // CTA-uniform
+      const float ch = cta_chunk_sum(ci.y, ci.z, [&](uint32_t j) { return pol.term(j); }, s_part);
+      if (threadIdx.x == 0) {
+        const uint32_t n = h.count[ci.w];
+        if (n == 1) {
+          pol.finish(ci.x, __fadd_rn(pol.start(ci.x), ch));
+        } else {
+          h.partials[t] = ch;
+          __threadfence();
+          if (atomicAdd(&h.done[ci.w], 1u) == n - 1) {
+            __threadfence();
+            h.done[ci.w] = 0;
+            const uint32_t f = h.first[ci.w];
+            float tot = 0.0f;
+            for (uint32_t c = 0; c < n; c++) tot = __fadd_rn(tot, __ldcg(&h.partials[f + c]));
+            pol.finish(ci.x, __fadd_rn(pol.start(ci.x), tot));
+          }
+        }
+      }
     }
-  } else if (b < nb_light + nb_med) {
-    const uint32_t w0 = (b - nb_light) * (kT / 32) + (threadIdx.x >> 5);
+  } else if (b < nb_heavy + nb_med) {
+    const uint32_t w0 = (b - nb_heavy) * (kT / 32) + (threadIdx.x >> 5);
     for (uint32_t t = w0; t < n_med; t += nb_med * (kT / 32)) {
       const uint32_t v = med[t];
       if (!pol.want(v)) continue;  // warp-uniform
@@ -234,13 +283,11 @@ __device__ void rows_pass(const uint2* __restrict__ rows, const uint32_t* __rest
       if (lane_id() == 0) pol.finish(v, __fadd_rn(pol.start(v), s));
     }
   } else {
-    const uint32_t cb = b - nb_light - nb_med, ncb = gridDim.x - nb_light - nb_med;
-    for (uint32_t t = cb; t < n_heavy; t += ncb) {
-      const uint32_t v = heavy[t];
-      if (!pol.want(v)) continue;  // CTA-uniform
+    for (uint32_t v = (b - nb_heavy - nb_med) * kT + threadIdx.x; v < V; v += nb_light * kT) {
       const uint2 r = rows[v];
-      const float s = cta_row_sum(r.x, r.y, [&](uint32_t j) { return pol.term(j); }, s_part);
-      if (threadIdx.x == 0) pol.finish(v, __fadd_rn(pol.start(v), s));
+      if (r.y > kWarpThr || !pol.want(v)) continue;
+      const float s = strided_sum4(pol.start(v), r.x, r.x + r.y, 1u, [&](uint32_t j) { return pol.term(j); });
+      pol.finish(v, s);
     }
   }
 }
@@ -347,11 +394,10 @@ struct PullPolicy {
 };
 
 __global__ void __launch_bounds__(kT) dd_pull_kernel(const uint2* __restrict__ rows, const uint32_t* __restrict__ med,
-                                                     const uint32_t* __restrict__ heavy, uint32_t nb_light,
-                                                     uint32_t nb_med, PullPolicy pol, DdCtl* __restrict__ ctl,
-                                                     uint32_t it) {
+                                                     HeavyRows heavy, Grid3 G, PullPolicy pol,
+                                                     DdCtl* __restrict__ ctl, uint32_t it) {
   if (ctl->stop) return;
-  rows_pass(rows, med, heavy, ctl->n_med, ctl->n_heavy, pol.p.V, nb_light, nb_med, pol);
+  rows_pass(blockIdx.x, rows, med, heavy, ctl->n_med, ctl->n_hch, pol.p.V, G.heavy, G.med, G.light, pol);
   if (block_totals(pol.err, pol.act, &ctl->err[it], &ctl->active[it], &ctl->done_a[it])) {
     if (ld_volatile_u32(&ctl->active[it]) == 0) {
       ctl->stop_iter = it;
@@ -378,10 +424,9 @@ struct ResidPolicy {
 };
 
 __global__ void __launch_bounds__(kT) dd_resid_kernel(const uint2* __restrict__ rows, const uint32_t* __restrict__ med,
-                                                      const uint32_t* __restrict__ heavy, uint32_t nb_light,
-                                                      uint32_t nb_med, ResidPolicy pol, const DdCtl* __restrict__ ctl,
-                                                      uint32_t V) {
-  rows_pass(rows, med, heavy, ctl->n_med, ctl->n_heavy, V, nb_light, nb_med, pol);
+                                                      HeavyRows heavy, Grid3 G, ResidPolicy pol,
+                                                      const DdCtl* __restrict__ ctl, uint32_t V) {
+  rows_pass(blockIdx.x, rows, med, heavy, ctl->n_med, ctl->n_hch, V, G.heavy, G.med, G.light, pol);
 }
 
 // One push of delta into resid[u]: the returned old value decides whether u
@@ -520,11 +565,10 @@ struct PullPushPolicy {
 
 __global__ void __launch_bounds__(kT) dd_pullpush_kernel(const uint2* __restrict__ rows,
                                                          const uint32_t* __restrict__ med,
-                                                         const uint32_t* __restrict__ heavy, uint32_t nb_light,
-                                                         uint32_t nb_med, PullPushPolicy pol,
+                                                         HeavyRows heavy, Grid3 G, PullPushPolicy pol,
                                                          DdCtl* __restrict__ ctl, uint32_t it) {
   if (ctl->stop) return;
-  rows_pass(rows, med, heavy, ctl->n_med, ctl->n_heavy, pol.p.V, nb_light, nb_med, pol);
+  rows_pass(blockIdx.x, rows, med, heavy, ctl->n_med, ctl->n_hch, pol.p.V, G.heavy, G.med, G.light, pol);
   block_totals(pol.err, pol.act, &ctl->err[it], &ctl->active[it], &ctl->done_a[it]);
 }
 
@@ -627,10 +671,9 @@ struct SpmvPullPolicy {
 };
 
 __global__ void __launch_bounds__(kT) spmv_pull_kernel(const uint2* __restrict__ rows, const uint32_t* __restrict__ med,
-                                                       const uint32_t* __restrict__ heavy, uint32_t nb_light,
-                                                       uint32_t nb_med, SpmvPullPolicy pol,
+                                                       HeavyRows heavy, Grid3 G, SpmvPullPolicy pol,
                                                        const DdCtl* __restrict__ ctl, uint32_t V) {
-  rows_pass(rows, med, heavy, ctl->n_med, ctl->n_heavy, V, nb_light, nb_med, pol);
+  rows_pass(blockIdx.x, rows, med, heavy, ctl->n_med, ctl->n_hch, V, G.heavy, G.med, G.light, pol);
 }
 
 // Push: rows of at most kWarpThr out-edges by a thread, rows up to kOutBig
@@ -700,7 +743,6 @@ int dd_work_get(DevGraph& g, DdWork** out, cudaStream_t s) {
     OGB_TRY(w->flags1.alloc((size_t)V + 16));
     OGB_TRY(w->resid.alloc((size_t)V * 4 + 16));
     OGB_TRY(w->med.alloc((size_t)V * 4 + 16));
-    OGB_TRY(w->heavy.alloc((size_t)V * 4 + 16));
     OGB_TRY(w->defer.alloc((size_t)V + 16));
     OGB_TRY(w->dvec.alloc((size_t)V * 4 + 16));
     OGB_TRY(w->selfcnt.alloc((size_t)V * 4 + 16));
@@ -726,8 +768,8 @@ int dd_work_get(DevGraph& g, DdWork** out, cudaStream_t s) {
   OGB_CUDA(cudaMemsetAsync(w->defer.p, 0, (size_t)V + 16, s));
   OGB_CUDA(cudaMemsetAsync(w->selfcnt.p, 0, (size_t)V * 4 + 16, s));
   const int grid = sm_count() * 8;
-  dd_count_kernel<<<grid, kT, 0, s>>>(V, g.inv.d_rows(), ctl);
-  dd_fill_kernel<<<grid, kT, 0, s>>>(V, g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.as<uint32_t>(), ctl);
+  OGB_TRY(w->heavy.alloc(g.E));
+  dd_fill_kernel<<<grid, kT, 0, s>>>(0, V, g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), ctl);
   dd_self_kernel<<<grid, kT, 0, s>>>(g.E, g.fwd.d_src(), g.fwd.d_dst(), w->selfcnt.as<uint32_t>());
   OGB_CUDA(cudaGetLastError());
   DevBuf tmp;
@@ -751,20 +793,6 @@ int dd_work_get(DevGraph& g, DdWork** out, cudaStream_t s) {
   w->ready = true;
   *out = w;
   return OK;
-}
-
-struct Grid3 {
-  uint32_t light, med, heavy;
-  uint32_t total() const { return light + med + heavy; }
-};
-
-Grid3 rows_grid(uint32_t V) {
-  const uint32_t sms = sm_count();
-  Grid3 g;
-  g.light = std::max<uint32_t>(1, std::min<uint32_t>(sms * 8, ceil_div(V, kT)));
-  g.med = sms * 8;
-  g.heavy = sms * 2;
-  return g;
 }
 
 }  // namespace
@@ -806,8 +834,7 @@ int pagerank_dd_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsil
     // (1.0f - damp) * damp, then times the row sum (pageRank.c:2614), in float
     const float coef = (1.0f - p.damp) * p.damp;
     ResidPolicy rp{g.inv.d_dst(), g.fwd.d_out_degree(), resid, coef};
-    dd_resid_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.as<uint32_t>(), G.light,
-                                             G.med, rp, ctl, V);
+    dd_resid_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), G, rp, ctl, V);
     launches++;
     if (mode == PR_DD_PULLPUSH) {  // the starting ranks / out-degree (flags cleared on the way)
       dd_contrib_kernel<<<sms * 8, kT, 0, s>>>(V, g.fwd.d_out_degree(), ranks, w->contrib.as<float>(), nxt,
@@ -824,8 +851,7 @@ int pagerank_dd_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsil
       dd_contrib_kernel<<<sms * 8, kT, 0, s>>>(V, g.fwd.d_out_degree(), ranks, w->contrib.as<float>(), nxt, defer,
                                                ctl);
       PullPolicy pol{cur, nxt, w->contrib.as<float>(), g.inv.d_dst(), ranks, g.fwd.d_rows(), g.fwd.d_dst(), defer, p};
-      dd_pull_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.as<uint32_t>(),
-                                               G.light, G.med, pol, ctl, it);
+      dd_pull_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), G, pol, ctl, it);
       dd_defer_kernel<false><<<sms * 8, kT, 0, s>>>(V, g.fwd.d_rows(), g.fwd.d_dst(), defer, dvec, och, resid, nxt,
                                                     epsilon, false, ctl, it);
     } else {
@@ -836,8 +862,7 @@ int pagerank_dd_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsil
       } else {
         PullPushPolicy pol{cur,   nxt,  g.inv.d_dst(), w->contrib.as<float>(), ranks, resid, g.fwd.d_rows(),
                            g.fwd.d_dst(), w->selfcnt.as<uint32_t>(), defer, dvec, p};
-        dd_pullpush_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.as<uint32_t>(),
-                                                     G.light, G.med, pol, ctl, it);
+        dd_pullpush_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), G, pol, ctl, it);
       }
       dd_defer_kernel<true><<<sms * 8, kT, 0, s>>>(V, g.fwd.d_rows(), g.fwd.d_dst(), defer, dvec, och, resid, nxt,
                                                    epsilon, mode == PR_DD_PULLPUSH, ctl, it);
@@ -890,8 +915,7 @@ int spmv_run(DevGraph& g, uint32_t mode, uint32_t iterations, float* x, float* y
     const Grid3 G = rows_grid(V);
     SpmvPullPolicy pol{g.inv.d_dst(), g.weighted ? g.inv.d_w() : nullptr, x, y};
     for (uint32_t it = 0; it < iterations; it++)
-      spmv_pull_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.as<uint32_t>(),
-                                                 G.light, G.med, pol, w->ctl.as<DdCtl>(), V);
+      spmv_pull_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), G, pol, w->ctl.as<DdCtl>(), V);
   } else {
     for (uint32_t it = 0; it < iterations; it++)
       spmv_push_kernel<<<sms * 8, kT, 0, s>>>(V, g.fwd.d_rows(), g.fwd.d_dst(), g.weighted ? g.fwd.d_w() : nullptr, x,
@@ -946,34 +970,11 @@ namespace {
 struct RangeWork {
   uint32_t lo = 0, hi = 0, build = 0;
   bool ready = false;
-  DevBuf ctl, med, heavy;
+  DevBuf ctl, med;
+  HeavyBuf heavy;
 };
 std::mutex g_range_mu;
 std::vector<std::pair<const DevGraph*, RangeWork*>> g_range;
-
-__global__ void range_count_kernel(uint32_t lo, uint32_t hi, const uint2* __restrict__ rows,
-                                   DdCtl* __restrict__ ctl) {
-  uint32_t cm = 0, ch = 0;
-  for (uint32_t v = lo + blockIdx.x * blockDim.x + threadIdx.x; v < hi; v += gridDim.x * blockDim.x) {
-    const uint32_t d = rows[v].y;
-    cm += (d > kWarpThr && d <= kCtaThr);
-    ch += (d > kCtaThr);
-  }
-  warp_atomic_add_total(&ctl->n_med, cm);
-  warp_atomic_add_total(&ctl->n_heavy, ch);
-}
-
-__global__ void range_fill_kernel(uint32_t lo, uint32_t hi, const uint2* __restrict__ rows,
-                                  uint32_t* __restrict__ med, uint32_t* __restrict__ heavy,
-                                  DdCtl* __restrict__ ctl) {
-  for (uint32_t v = lo + blockIdx.x * blockDim.x + threadIdx.x; v < hi; v += gridDim.x * blockDim.x) {
-    const uint32_t d = rows[v].y;
-    if (d > kCtaThr)
-      heavy[atomicAdd(&ctl->cur_heavy, 1u)] = v;
-    else if (d > kWarpThr)
-      med[atomicAdd(&ctl->cur_med, 1u)] = v;
-  }
-}
 
 struct RangePolicy {
   uint32_t lo;
@@ -1007,10 +1008,8 @@ struct RangePolicy {
 // rows_pass over [lo, hi): the light blocks walk [lo, hi), the lists hold
 // the range's medium and heavy rows.
 __global__ void __launch_bounds__(kT) range_step_kernel(const uint2* __restrict__ rows, uint32_t lo, uint32_t hi,
-                                                        const uint32_t* __restrict__ med,
-                                                        const uint32_t* __restrict__ heavy, uint32_t nb_light,
-                                                        uint32_t nb_med, RangePolicy pol,
-                                                        const DdCtl* __restrict__ ctl, double* g_err,
+                                                        const uint32_t* __restrict__ med, HeavyRows heavy, Grid3 G,
+                                                        RangePolicy pol, const DdCtl* __restrict__ ctl, double* g_err,
                                                         uint32_t* g_act) {
   // shift the light rows' vertex numbering to the range: rows_pass walks
   // [0, n) of the shifted arrays
@@ -1023,11 +1022,11 @@ __global__ void __launch_bounds__(kT) range_step_kernel(const uint2* __restrict_
     __device__ void finish(uint32_t v, float s) { q.finish(v + lo, s); }
   };
   Shift sh{pol, lo};
-  if (blockIdx.x < nb_light) {
-    rows_pass(rows + lo, nullptr, nullptr, 0, 0, hi - lo, nb_light, 0, sh);
+  if (blockIdx.x >= G.heavy + G.med) {
+    rows_pass(blockIdx.x - G.heavy - G.med, rows + lo, nullptr, heavy, 0, 0, hi - lo, 0, 0, G.light, sh);
   } else {
-    // medium / heavy lists hold absolute vertex ids: run them unshifted
-    rows_pass(rows, med, heavy, ctl->n_med, ctl->n_heavy, 0, nb_light, nb_med, pol);
+    // the medium list and the heavy chunks hold absolute vertex ids: run them unshifted
+    rows_pass(blockIdx.x, rows, med, heavy, ctl->n_med, ctl->n_hch, 0, G.heavy, G.med, 0, pol);
   }
   // peer stores (other GPUs' memory over NVLink) ordered before anything
   // this thread does after the step, the caller's barrier included
@@ -1108,12 +1107,11 @@ int pagerank_range_step(DevGraph& g, uint32_t lo, uint32_t hi, const float* cont
   if (!w->ready || w->lo != lo || w->hi != hi || w->build != g.build_id) {
     OGB_TRY(w->ctl.alloc(sizeof(DdCtl)));
     OGB_TRY(w->med.alloc((size_t)(hi - lo) * 4 + 16));
-    OGB_TRY(w->heavy.alloc((size_t)(hi - lo) * 4 + 16));
+    OGB_TRY(w->heavy.alloc(g.E));
     ctl = w->ctl.as<DdCtl>();
     OGB_CUDA(cudaMemsetAsync(ctl, 0, sizeof(DdCtl), s));
     const int grid = sm_count() * 8;
-    range_count_kernel<<<grid, kT, 0, s>>>(lo, hi, g.inv.d_rows(), ctl);
-    range_fill_kernel<<<grid, kT, 0, s>>>(lo, hi, g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.as<uint32_t>(), ctl);
+    dd_fill_kernel<<<grid, kT, 0, s>>>(lo, hi, g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), ctl);
     OGB_CUDA(cudaGetLastError());
     w->lo = lo;
     w->hi = hi;
@@ -1128,8 +1126,8 @@ int pagerank_range_step(DevGraph& g, uint32_t lo, uint32_t hi, const float* cont
   p.epsilon = epsilon;
   RangePolicy pol{lo, g.inv.d_dst(), g.fwd.d_out_degree(), contrib, ranks, contrib_next, p, peers, npeers};
   const Grid3 G = rows_grid(hi - lo);
-  range_step_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), lo, hi, w->med.as<uint32_t>(), w->heavy.as<uint32_t>(),
-                                             G.light, G.med, pol, ctl, d_err, d_active);
+  range_step_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), lo, hi, w->med.as<uint32_t>(), w->heavy.view(), G, pol,
+                                             ctl, d_err, d_active);
   OGB_CUDA(cudaGetLastError());
   return OK;
 }
