@@ -323,6 +323,8 @@ int bfs_set_policy(const float* params_host) {
 
 // ------------------------------------------------------------ shared memory
 
+constexpr uint32_t kInvalid = 0xFFFFFFFFu;
+
 struct ScanSmem {
   uint32_t w[kScanT / 32];
   uint32_t tile, prefix;
@@ -343,6 +345,16 @@ struct TdSmemHost : TdSmem {
   uint32_t d[kExpTile + 2];
   BlockAppend<kExpTile> q_all;
 };
+// In-rows of a bottom-up round by what is left of them: a 4-lane group scans
+// kLongCut edges of a row, a warp up to kMoreCut more, and the CTA the rest.  A
+// 4-lane group walking whole rows (8 edges per step) made a round wait for its
+// longest row without a hit: 10 K edges and more on a hub that the search does
+// not reach (a batch of 96 graphs whose roots reach little: 1.25 ms per search,
+// 0.36 ms with the cuts; 0.45 ms with kLongCut at 256).  The rows left are marked
+// in the round's own list: handing them on through lists of their own, with a
+// check inside the groups' loop, made RMAT-22's first bottom-up step 68 -> 75 us.
+constexpr uint32_t kLongCut = 64, kMoreCut = 2048;
+constexpr uint32_t kMoreBit = 1u << 31, kHugeBit = 1u << 30;  // marks on a round's entries, which are below 2^30
 // Bottom-up: a round's appends and its deferred long in-edge rows.  A round
 // appends each of its at most kBuCap candidates to at most one list, so
 // the new frontier list fills one buffer from the front and the unvisited
@@ -352,43 +364,39 @@ struct BuSmem {
   uint32_t buf[kBuCap];
   uint32_t nheavy;
   uint32_t hv[kBuCap];
+  uint32_t nmore, nhuge;  // nonzero: hv holds rows left over by the 4-lane groups (kMoreBit), by the warps (kHugeBit)
+  // what their scan reads and writes (set at the step's start: as arguments these
+  // pushed the search kernel into spills)
+  const uint2* rows_i;
+  const uint32_t *nbr_i, *out_degree, *bm_cur;
+  uint32_t* bm_next;
+  const uint4* rec_a;  // null: dense step
+  int32_t* parents;
+  uint32_t* distances;
+  uint32_t dnext;
+  uint32_t first;                        // CTA-wide scan: position of the first hit in the step
+  uint32_t x_nf, x_edges, x_mx;          // totals of those rows
+  unsigned long long x_fed;
 };
+__device__ __forceinline__ void bu_init(BuSmem& sm, const BfsBufs& b, const uint32_t* bm_cur, uint32_t* bm_next,
+                                        const uint4* rec_a, int32_t* parents, uint32_t* distances, uint32_t dnext) {
+  sm.rows_i = b.rows_i;
+  sm.nbr_i = b.nbr_i;
+  sm.out_degree = b.out_degree;
+  sm.bm_cur = bm_cur;
+  sm.bm_next = bm_next;
+  sm.rec_a = rec_a;
+  sm.parents = parents;
+  sm.distances = distances;
+  sm.dnext = dnext;
+  sm.nlist = sm.nul = sm.nheavy = sm.nmore = sm.nhuge = 0;
+  sm.x_nf = sm.x_edges = sm.x_mx = 0;
+  sm.x_fed = 0;
+}
 __device__ __forceinline__ void bu_push_list(BuSmem& sm, uint32_t v) { sm.buf[warp_atomic_inc(&sm.nlist)] = v; }
 __device__ __forceinline__ void bu_push_ul(BuSmem& sm, uint32_t v) {
   sm.buf[kBuCap - 1u - warp_atomic_inc(&sm.nul)] = v;
 }
-// A round's appends out, then the buffer and the long-row list are empty:
-// discoveries (vertices) into list_out, and the records of the unvisited
-// candidates (staged as indices into in_a / in_b) copied into out_a /
-// out_b; the offsets of both are reserved together.
-__device__ __forceinline__ void bu_flush(BuSmem& sm, uint32_t* list_out, uint32_t* list_count,
-                                             const uint4* in_a, const uint4* in_b, uint4* out_a, uint4* out_b,
-                                             uint32_t* ul_count) {
-  __syncthreads();
-  const uint32_t nl = sm.nlist, nu = sm.nul;
-  if (threadIdx.x == 0) {
-    uint32_t bl = 0, bu = 0;
-    if (nl) bl = atomicAdd(list_count, nl);
-    if (nu) bu = atomicAdd(ul_count, nu);
-    sm.base_list = bl;
-    sm.base_ul = bu;
-  }
-  __syncthreads();
-  for (uint32_t k = threadIdx.x; k < nl; k += blockDim.x) list_out[sm.base_list + k] = sm.buf[k];
-  for (uint32_t k = threadIdx.x; k < nu; k += blockDim.x) {
-    const uint32_t s = sm.buf[kBuCap - 1u - k];
-    out_a[sm.base_ul + k] = in_a[s];
-    out_b[sm.base_ul + k] = in_b[s];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    sm.nlist = 0;
-    sm.nul = 0;
-    sm.nheavy = 0;  // the round's long rows were all read before the first barrier above
-  }
-  __syncthreads();
-}
-
 // A flat top-down step's appends: each of a CTA's threads expands one list
 // entry of at most kFlatMaxDeg out-edges per pass.
 constexpr uint32_t kFlatMaxDeg = 16;
@@ -911,7 +919,6 @@ __device__ void td_flat_phase(const BfsBufs& b, const uint32_t* list, uint32_t* 
 
 // ------------------------------------------------------------ bottom-up ----
 
-constexpr uint32_t kInvalid = 0xFFFFFFFFu;
 constexpr int kBuV = kBuRound / kSearchT;  // candidates per thread per round
 constexpr uint32_t kFirst = 6;             // dense step: in-edges probed per candidate before deferral
 constexpr uint32_t kRecN = 4;              // list step: in-neighbours held in a candidate record
@@ -953,12 +960,13 @@ __device__ __forceinline__ void bu_long_rows(const BfsBufs& b, const uint32_t* b
       end = rr.x + rr.y;
     }
     bool hit_row = false;
-    for (uint32_t j = j0; j < end; j += kLongStep) {
+    const uint32_t lim = min(end, j0 + kLongCut);
+    for (uint32_t j = j0; j < lim; j += kLongStep) {
       uint32_t x[kLongLoads];
 #pragma unroll
       for (uint32_t q = 0; q < kLongLoads; q++) {
         const uint32_t jq = j + q * kLongLanes + gl;
-        x[q] = jq < end ? (__ldg(&b.nbr_i[jq]) & 0x3FFFFFFFu) : kInvalid;
+        x[q] = jq < lim ? (__ldg(&b.nbr_i[jq]) & 0x3FFFFFFFu) : kInvalid;
       }
       bool bit[kLongLoads];
 #pragma unroll
@@ -992,10 +1000,201 @@ __device__ __forceinline__ void bu_long_rows(const BfsBufs& b, const uint32_t* b
       }
     }
     if (!hit_row && gl == 0) {
-      edges += end - j0;
-      bu_push_ul(sm, hv);
+      edges += lim - j0;
+      if (lim < end) {
+        sm.hv[h] = hv | kMoreBit;
+        sm.nmore = 1;
+      } else {
+        bu_push_ul(sm, hv);
+      }
     }
   }
+}
+
+// A row's vertex, out-degree (0 in the dense step: read on a hit), the first
+// in-edge the 4-lane groups left and the end.
+__device__ __forceinline__ void bu_row_of(uint32_t hv, const BuSmem& sm, uint32_t& v, uint32_t& od, uint32_t& j0,
+                                          uint32_t& end) {
+  if (sm.rec_a) {
+    const uint4 r = sm.rec_a[hv];
+    v = r.x;
+    od = r.w;
+    j0 = r.y + kRecN + kLongCut;
+    end = r.y + r.z;
+  } else {
+    const uint2 r = __ldg(&sm.rows_i[hv]);
+    v = hv;
+    od = 0;
+    j0 = r.x + kFirst + kLongCut;
+    end = r.x + r.y;
+  }
+}
+
+// One thread records a discovery of the leftover rows.
+__device__ __forceinline__ void bu_more_found(uint32_t v, uint32_t u, uint32_t od, BuSmem& sm) {
+  if (!sm.rec_a) od = __ldg(&sm.out_degree[v]);
+  sm.parents[v] = (int32_t)u;
+  sm.distances[v] = sm.dnext;
+  atomicOr(&sm.bm_next[v >> 5], 1u << (v & 31));
+  atomicAdd(&sm.x_nf, 1u);
+  atomicAdd(&sm.x_fed, (unsigned long long)od);
+  if (od) {
+    bu_push_list(sm, v);
+    atomicMax(&sm.x_mx, od);
+  }
+}
+
+// The rows the 4-lane groups left: a warp per row, 128 in-edges per step, then
+// what is still left after kMoreCut edges by the whole CTA, 1024 per step.  The
+// first hit in CSR order wins.  Kept out of line: it runs only when a round has
+// such rows, and the search kernel has no registers to spare for it.
+__device__ __noinline__ void bu_more_rows(BuSmem& sm) {
+  constexpr uint32_t K = 4;
+  const uint32_t* nbr_i = sm.nbr_i;
+  const uint32_t* bm_cur = sm.bm_cur;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, nheavy = sm.nheavy;
+  for (uint32_t h0 = warp * 32; h0 < nheavy; h0 += kSearchT) {
+    uint32_t todo = __ballot_sync(0xffffffffu, h0 + lane < nheavy && (sm.hv[h0 + lane] & kMoreBit));
+    while (todo) {
+      const uint32_t h = h0 + (uint32_t)__ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint32_t hv = sm.hv[h] & ~kMoreBit;
+      uint32_t v, od, j0, end;
+      bu_row_of(hv, sm, v, od, j0, end);
+      const uint32_t lim = min(end, j0 + kMoreCut);
+      bool found = false;
+      for (uint32_t j = j0; j < lim; j += 32 * K) {
+        uint32_t x[K];
+#pragma unroll
+        for (uint32_t q = 0; q < K; q++) {
+          const uint32_t jq = j + q * 32 + lane;
+          x[q] = jq < lim ? (__ldg(&nbr_i[jq]) & 0x3FFFFFFFu) : kInvalid;
+        }
+        uint32_t q0 = 0, u = 0, m = 0;
+#pragma unroll
+        for (int q = (int)K - 1; q >= 0; q--) {
+          const uint32_t mq = __ballot_sync(0xffffffffu, x[q] != kInvalid && ((bm_cur[x[q] >> 5] >> (x[q] & 31)) & 1u));
+          if (mq) {
+            q0 = (uint32_t)q;
+            m = mq;
+            u = x[q];
+          }
+        }
+        if (m) {
+          const uint32_t l0 = (uint32_t)__ffs(m) - 1;
+          if (lane == l0) {
+            atomicAdd(&sm.x_edges, j + q0 * 32 + l0 + 1 - j0);
+            bu_more_found(v, u, od, sm);
+          }
+          found = true;
+          break;
+        }
+      }
+      if (!found && lane == 0) {
+        atomicAdd(&sm.x_edges, lim - j0);
+        if (lim < end) {
+          sm.hv[h] = hv | kHugeBit;
+          sm.nhuge = 1;
+        } else {
+          bu_push_ul(sm, hv);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (!sm.nhuge) return;
+  for (uint32_t h0 = 0; h0 < nheavy; h0 += 32) {
+    uint32_t todo = __ballot_sync(0xffffffffu, h0 + lane < nheavy && (sm.hv[h0 + lane] & kHugeBit));  // the same in every warp
+    while (todo) {
+      const uint32_t hv = sm.hv[h0 + (uint32_t)__ffs(todo) - 1] & ~kHugeBit;
+      todo &= todo - 1;
+      uint32_t v, od, j0, end;
+      bu_row_of(hv, sm, v, od, j0, end);
+      j0 += kMoreCut;
+      if (threadIdx.x == 0) sm.first = kInvalid;
+      __syncthreads();
+      bool found = false;
+      for (uint32_t j = j0; j < end; j += kSearchT * K) {
+        uint32_t x[K], mine = kInvalid, u = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < K; q++) {
+          const uint32_t jq = j + q * kSearchT + threadIdx.x;
+          x[q] = jq < end ? (__ldg(&nbr_i[jq]) & 0x3FFFFFFFu) : kInvalid;
+        }
+#pragma unroll
+        for (int q = (int)K - 1; q >= 0; q--)
+          if (x[q] != kInvalid && ((bm_cur[x[q] >> 5] >> (x[q] & 31)) & 1u)) {
+            mine = j + q * kSearchT + threadIdx.x;
+            u = x[q];
+          }
+        if (mine != kInvalid) atomicMin(&sm.first, mine);
+        __syncthreads();
+        const uint32_t first = sm.first;
+        __syncthreads();
+        if (first != kInvalid) {
+          if (mine == first) {
+            atomicAdd(&sm.x_edges, first + 1 - j0);
+            bu_more_found(v, u, od, sm);
+          }
+          found = true;
+          break;
+        }
+      }
+      if (!found && threadIdx.x == 0) {
+        atomicAdd(&sm.x_edges, end - j0);
+        bu_push_ul(sm, hv);
+      }
+      __syncthreads();  // before the next row resets `first`
+    }
+  }
+}
+
+// The rows the 4-lane groups left are finished, then the round's appends go
+// out and the buffer and the long-row list are empty:
+// discoveries (vertices) into list_out, and the records of the unvisited
+// candidates (staged as indices into in_a / in_b) copied into out_a /
+// out_b; the offsets of both are reserved together.
+// keep_ul false (dense step): no unvisited list is written.
+__device__ __forceinline__ void bu_flush(BuSmem& sm, uint32_t* list_out, uint32_t* list_count, const uint4* in_a, const uint4* in_b, uint4* out_a,
+                                         uint4* out_b, uint32_t* ul_count, bool keep_ul, uint32_t& nf,
+                                         uint32_t& edges, uint32_t& mx, unsigned long long& fed) {
+  __syncthreads();
+  if (sm.nmore) {
+    bu_more_rows(sm);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      nf += sm.x_nf;
+      edges += sm.x_edges;
+      mx = max(mx, sm.x_mx);
+      fed += sm.x_fed;
+      sm.x_nf = sm.x_edges = sm.x_mx = 0;
+      sm.x_fed = 0;
+      sm.nmore = 0;
+      sm.nhuge = 0;
+    }
+  }
+  const uint32_t nl = sm.nlist, nu = keep_ul ? sm.nul : 0u;
+  if (threadIdx.x == 0) {
+    uint32_t bl = 0, bu = 0;
+    if (nl) bl = atomicAdd(list_count, nl);
+    if (nu) bu = atomicAdd(ul_count, nu);
+    sm.base_list = bl;
+    sm.base_ul = bu;
+  }
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < nl; k += blockDim.x) list_out[sm.base_list + k] = sm.buf[k];
+  for (uint32_t k = threadIdx.x; k < nu; k += blockDim.x) {
+    const uint32_t s = sm.buf[kBuCap - 1u - k];
+    out_a[sm.base_ul + k] = in_a[s];
+    out_b[sm.base_ul + k] = in_b[s];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sm.nlist = 0;
+    sm.nul = 0;
+    sm.nheavy = 0;  // the round's long rows were all read before the first barrier above
+  }
+  __syncthreads();
 }
 
 // Step totals: nf and the edges examined, packed, the discoveries' out-edges
@@ -1026,9 +1225,7 @@ __device__ void bu_dense_phase(const BfsBufs& b, const uint32_t* bm_cur, uint32_
                                BfsCtl* ctl, BuSmem& sm, unsigned long long* s_red) {
   grid_clear(bm_clear, nullptr, b.words);
   if (threadIdx.x == 0) {
-    sm.nlist = 0;
-    sm.nul = 0;
-    sm.nheavy = 0;
+    bu_init(sm, b, bm_cur, bm_next, nullptr, parents, distances, dnext);
   }
   __syncthreads();
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
@@ -1107,12 +1304,8 @@ __device__ void bu_dense_phase(const BfsBufs& b, const uint32_t* bm_cur, uint32_
     }
     __syncthreads();
     bu_long_rows(b, bm_cur, bm_next, nullptr, parents, distances, dnext, sm, nf, edges, mx, fed);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      sm.nheavy = 0;
-      sm.nul = 0;  // long rows without a hit: no unvisited list in this mode
-    }
-    bu_flush(sm, list_next, &ctl->lnext, nullptr, nullptr, nullptr, nullptr, &ctl->ul_size);
+    bu_flush(sm, list_next, &ctl->lnext, nullptr, nullptr, nullptr,
+             nullptr, &ctl->ul_size, false, nf, edges, mx, fed);
   }
   bu_publish(ctl, nf, edges, fed, mx, s_red);
 }
@@ -1145,9 +1338,7 @@ __device__ void bu_rec_phase(const BfsBufs& b, const uint32_t* bm_cur, uint32_t*
                              unsigned long long* s_red) {
   grid_clear(bm_clear, nullptr, b.words);
   if (threadIdx.x == 0) {
-    sm.nlist = 0;
-    sm.nul = 0;
-    sm.nheavy = 0;
+    bu_init(sm, b, bm_cur, bm_next, in_a, parents, distances, dnext);
   }
   __syncthreads();
   uint32_t nf = 0, edges = 0, mx = 0;
@@ -1215,7 +1406,8 @@ __device__ void bu_rec_phase(const BfsBufs& b, const uint32_t* bm_cur, uint32_t*
     __syncthreads();
     bu_long_rows(b, bm_cur, bm_next, in_a, parents, distances, dnext, sm, nf, edges, mx, fed);
     // the flush's first barrier ends the long rows (it also clears their count)
-    bu_flush(sm, list_next, &ctl->lnext, in_a, in_b, out_a, out_b, &ctl->ul_size);
+    bu_flush(sm, list_next, &ctl->lnext, in_a, in_b, out_a, out_b,
+             &ctl->ul_size, true, nf, edges, mx, fed);
   }
   bu_publish(ctl, nf, edges, fed, mx, s_red);
 }
