@@ -5,19 +5,23 @@
 // once, one bit-lane per root.  Per vertex, three 64-bit words: the lanes
 // that have visited it, the lanes whose frontier holds it, and the lanes that
 // reach it in the level being built.  A level is either
-//  * push (top-down): the frontier's out-edges, edge-balanced (a device scan
-//    of the frontier vertices' out-degrees, then a warp per 32 consecutive
-//    edges, each lane locating its edge's vertex by binary search); each
-//    edge ORs the frontier word of its source, minus the target's visited
-//    lanes, into the target's next word (64-bit atomicOr);
+//  * push (top-down): a warp takes 32 vertices of the frontier list and walks
+//    their out-edges as one sequence (each lane finds its edge's vertex by a
+//    search through shuffles); rows of more than kMsLong edges are cut into
+//    pieces, a warp each in a second kernel.  Each edge ORs the frontier word of
+//    its source, minus the target's visited lanes, into the target's next word
+//    (64-bit atomicOr);
 //  * pull (bottom-up): every vertex with a lane still unvisited ORs the
 //    frontier words of its in-neighbours, stopping once every unvisited lane
 //    is covered; rows of at most kMsLight in-edges by a thread (four edges
 //    per step), longer rows by a warp;
 // then one dense pass turns the next words into the new frontier, sets the
 // visited lanes, writes the depths of the lanes each vertex gained (a warp
-// per vertex row, coalesced) and counts the new frontier and its out-edges
-// for the direction choice.
+// per vertex row, coalesced) and counts the new frontier and its out-edges; the
+// pass's last CTA chooses the next level's direction.  The level loop's state
+// stays on the device: the host launches kMsBatch levels at a time (three
+// kernels each, which return at once when the search has ended) and looks only
+// then, where a look per level cost a wait of 15 us.
 // Depths are u16 per (vertex, lane), row-major by vertex (128 bytes per
 // vertex, 0xFFFF = unreached).  The search is level-synchronous in every
 // lane, so every lane's depths are those of a single-root BFS.
@@ -30,19 +34,41 @@ namespace ogb {
 
 constexpr uint32_t kMsLight = 32;    // pull: rows up to this many in-edges by one thread
 constexpr uint32_t kMsAlpha = 14;    // push while the frontier's out-edges < E / kMsAlpha
+constexpr uint32_t kMsLong = 512;    // push: rows of more out-edges go in pieces of this many
+constexpr int kMsBatch = 4;          // levels launched between two looks of the host
+constexpr uint32_t kMsMaxLevels = 0xFFFE;
 
 struct MsCtl {
-  uint32_t nlist;              // vertices of the new frontier
+  // the frontier the next level starts from
+  uint32_t nlist;
+  uint32_t pull;               // direction of the next level
+  uint32_t done;               // 1: the frontier is empty, 2: too many levels
+  uint32_t levels, push_levels, pull_levels;  // levels finished, by direction
+  unsigned long long mf;       // out-edges of the frontier
+  // counted by the level in progress
+  uint32_t next_n, items, ctas;  // vertices found, row pieces, CTAs finished
   uint32_t pad;
-  unsigned long long mf;       // their out-edges
-  unsigned long long reached;  // (vertex, lane) pairs reached by the level
-  unsigned long long edges;    // edges read by the level
+  unsigned long long next_mf;
+  // of the whole search
+  unsigned long long reached;  // (vertex, lane) pairs reached after the roots
+  unsigned long long edges;    // edges read
 };
+
+// Direction of the level that starts from the frontier in c, or its end.
+__device__ __forceinline__ void ms_next_level(MsCtl& c, uint32_t E) {
+  if (c.nlist == 0) {
+    c.done = 1;
+  } else if (c.levels >= kMsMaxLevels) {
+    c.done = 2;
+  } else {
+    c.pull = c.mf < (unsigned long long)E / kMsAlpha ? 0u : 1u;
+  }
+}
 
 struct MsWork {
   uint32_t V = 0, heavy_build = 0;
   bool heavy_ready = false;
-  DevBuf F, N, vis, list, cnt, off, heavy, ctl, scan_tmp;
+  DevBuf F, N, vis, list, items, heavy, ctl, roots;
   uint32_t n_heavy = 0;
   MsCtl* h_ctl = nullptr;
   cudaEvent_t ev_init = nullptr, ev0 = nullptr, ev1 = nullptr;
@@ -61,7 +87,7 @@ void ms_work_free(MsWork* w) { delete w; }
 __global__ void msk_roots(const uint32_t* __restrict__ verts, const unsigned long long* __restrict__ masks,
                           uint32_t n, unsigned long long* __restrict__ F, unsigned long long* __restrict__ vis,
                           uint16_t* __restrict__ depth, uint32_t* __restrict__ list,
-                          const uint32_t* __restrict__ out_degree, MsCtl* __restrict__ ctl) {
+                          const uint32_t* __restrict__ out_degree, uint32_t E, MsCtl* __restrict__ ctl) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint32_t v = verts[i];
     const unsigned long long m = masks[i];
@@ -76,119 +102,131 @@ __global__ void msk_roots(const uint32_t* __restrict__ verts, const unsigned lon
     }
     atomicAdd(&ctl->mf, (unsigned long long)out_degree[v]);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->nlist = n;
+  __syncthreads();  // one CTA: mf is complete
+  if (threadIdx.x == 0) {
+    __threadfence();
+    ctl->nlist = n;
+    ctl->mf = atomicAdd(&ctl->mf, 0ull);
+    ms_next_level(*ctl, E);
+  }
 }
 
-// push: out-degree of each frontier vertex (scanned into edge offsets)
-__global__ void msk_frontier_degree(const uint32_t* __restrict__ list, uint32_t n, const uint2* __restrict__ rows,
-                                    uint32_t* __restrict__ cnt) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    cnt[i] = rows[list[i]].y;
+// Push of the edges of the frontier word f: four targets at once.
+__device__ __forceinline__ void ms_push4(const unsigned long long* f, const uint32_t* w, const bool* ok,
+                                         const unsigned long long* __restrict__ vis, unsigned long long* N) {
+  unsigned long long m[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) m[k] = ok[k] ? f[k] & ~vis[w[k]] : 0ull;
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (m[k]) atomicOr(&N[w[k]], m[k]);
 }
 
-// push, a frontier list of at most kMsSmallScan entries: its out-degrees
-// scanned by one CTA (entry i's first edge in off[i], the total in off[n]) --
-// one launch instead of a degree pass and a three-kernel device scan.
-constexpr uint32_t kMsSmallScan = 8192;
-__global__ void __launch_bounds__(1024) msk_small_scan(const uint32_t* __restrict__ list, uint32_t n,
-                                                        const uint2* __restrict__ rows, uint32_t* __restrict__ off) {
-  constexpr uint32_t K = kMsSmallScan / 1024;  // entries per thread
-  __shared__ uint32_t s_w[32];
-  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  uint32_t d[K], sum = 0;
-#pragma unroll
-  for (uint32_t k = 0; k < K; k++) {
-    const uint32_t i = threadIdx.x * K + k;
-    d[k] = i < n ? rows[list[i]].y : 0u;
-    sum += d[k];
-  }
-  uint32_t x = sum;
-#pragma unroll
-  for (uint32_t o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) s_w[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t t = s_w[lane];
-#pragma unroll
-    for (uint32_t o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) t += y;
-    }
-    s_w[lane] = t;  // inclusive warp totals
-  }
-  __syncthreads();
-  uint32_t e = (warp ? s_w[warp - 1] : 0u) + x - sum;
-#pragma unroll
-  for (uint32_t k = 0; k < K; k++) {
-    const uint32_t i = threadIdx.x * K + k;
-    if (i < n) off[i] = e;
-    e += d[k];
-  }
-  if (threadIdx.x == blockDim.x - 1) off[n] = e;  // the list's out-edges
-}
-
-// push: the frontier's out-edges, edge-balanced: a warp takes 32 consecutive
-// edges of the frontier's edge range; lane 0 finds the first edge's vertex
-// by binary search over the offsets, each lane then its own edge's vertex
-// from there.
-__global__ void __launch_bounds__(256) msk_push(const uint32_t* __restrict__ list, uint32_t n,
-                                                const uint32_t* __restrict__ off, const uint2* __restrict__ rows,
-                                                const uint32_t* __restrict__ nbr,
-                                                const unsigned long long* __restrict__ F,
-                                                const unsigned long long* __restrict__ vis,
-                                                unsigned long long* __restrict__ N, MsCtl* __restrict__ ctl) {
+// The level's edges, by its direction: push over the frontier list, or pull
+// over the vertices (blocks [0, nb_heavy): the vertices with more than kMsLight
+// in-edges, a warp each, lanes strided, the warp's OR checked every 128 edges;
+// the rest: a thread per vertex, four in-edges per step, until every unvisited
+// lane is covered).
+__global__ void __launch_bounds__(256) msk_expand(uint32_t V, unsigned long long lanes, uint32_t nb_heavy,
+                                                  const uint32_t* __restrict__ heavy, uint32_t n_heavy,
+                                                  const uint2* __restrict__ rows_f, const uint32_t* __restrict__ nbr_f,
+                                                  const uint2* __restrict__ rows_i, const uint32_t* __restrict__ nbr_i,
+                                                  const unsigned long long* __restrict__ F,
+                                                  const unsigned long long* __restrict__ vis, unsigned long long* N,
+                                                  const uint32_t* __restrict__ list, uint4* __restrict__ items,
+                                                  MsCtl* ctl) {
+  if (ctl->done) return;
   const uint32_t lane = lane_id();
-  const uint32_t total = off[n];
   const uint32_t gw = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  const uint32_t nw = gridDim.x * (blockDim.x / 32);
-  for (uint32_t e0 = gw * 32; e0 < total; e0 += nw * 32) {
-    uint32_t i0 = 0;
-    if (lane == 0) {
-      uint32_t lo = 0, hi = n - 1;  // last i with off[i] <= e0
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (off[mid] <= e0)
-          lo = mid;
-        else
-          hi = mid - 1;
+  if (!ctl->pull) {
+    const uint32_t n = ctl->nlist, nw = gridDim.x * (blockDim.x / 32);
+    for (uint64_t i0 = (uint64_t)gw * 32; i0 < n; i0 += (uint64_t)nw * 32) {
+      uint32_t u = 0;
+      uint2 r = make_uint2(0u, 0u);
+      unsigned long long fu = 0;
+      if (i0 + lane < n) {
+        u = list[i0 + lane];
+        r = rows_f[u];
+        fu = F[u];
       }
-      i0 = lo;
-    }
-    i0 = __shfl_sync(0xffffffffu, i0, 0);
-    const uint32_t e = e0 + lane;
-    if (e < total) {
-      uint32_t lo = i0, hi = n - 1;  // entries without out-edges share an offset, so no tighter bound
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (off[mid] <= e)
-          lo = mid;
-        else
-          hi = mid - 1;
+      if (r.y > kMsLong) {
+        const uint32_t np = (r.y + kMsLong - 1) / kMsLong, at = atomicAdd(&ctl->items, np);
+        for (uint32_t c = 0; c < np; c++)
+          items[at + c] = make_uint4(u, r.x + c * kMsLong, r.x + min(r.y, (c + 1) * kMsLong), 0u);
+        r.y = 0;
       }
-      const uint32_t u = list[lo];
-      const uint32_t w = __ldg(&nbr[rows[u].x + (e - off[lo])]) & 0x3FFFFFFFu;
-      const unsigned long long m = F[u] & ~vis[w];
-      if (m) atomicOr(&N[w], m);
+      uint32_t ex = r.y;
+#pragma unroll
+      for (int k = 1; k < 32; k <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, ex, k);
+        if (lane >= (uint32_t)k) ex += y;
+      }
+      const uint32_t total = __shfl_sync(0xffffffffu, ex, 31);
+      ex -= r.y;
+      for (uint32_t e0 = 0; e0 < total; e0 += 128) {
+        unsigned long long f[4];
+        uint32_t w[4];
+        bool ok[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint32_t e = e0 + k * 32 + lane;
+          uint32_t p = 0;  // last vertex whose first edge is at or before e
+#pragma unroll
+          for (int step = 16; step; step >>= 1) {
+            const uint32_t first = __shfl_sync(0xffffffffu, ex, p + step);
+            if (first <= e) p += step;
+          }
+          const uint32_t from = __shfl_sync(0xffffffffu, r.x - ex, p) + e;
+          f[k] = __shfl_sync(0xffffffffu, fu, p);
+          ok[k] = e < total;
+          w[k] = ok[k] ? (__ldg(&nbr_f[from]) & 0x3FFFFFFFu) : 0u;
+        }
+        ms_push4(f, w, ok, vis, N);
+      }
     }
+    return;
   }
-  if (gw == 0 && lane == 0) atomicAdd(&ctl->edges, (unsigned long long)total);
-}
-
-// pull, light rows: a thread per vertex, four in-edges per step, stop once
-// every unvisited lane is covered
-__global__ void __launch_bounds__(256) msk_pull_light(uint32_t V, unsigned long long lanes,
-                                                      const uint2* __restrict__ rows, const uint32_t* __restrict__ nbr,
-                                                      const unsigned long long* __restrict__ F,
-                                                      const unsigned long long* __restrict__ vis,
-                                                      unsigned long long* __restrict__ N, MsCtl* __restrict__ ctl) {
   uint32_t edges = 0;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+  if (blockIdx.x < nb_heavy) {
+    const uint32_t nw = nb_heavy * (blockDim.x / 32);
+    for (uint32_t t = gw; t < n_heavy; t += nw) {
+      const uint32_t v = heavy[t];
+      const unsigned long long pending = lanes & ~vis[v];
+      if (!pending) continue;
+      const uint2 r = rows_i[v];
+      const uint32_t end = r.x + r.y;
+      unsigned long long acc = 0;
+      uint32_t j = r.x;
+      for (; j < end; j += 128) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint32_t jj = j + k * 32 + lane;
+          if (jj < end) acc |= F[__ldg(&nbr_i[jj]) & 0x3FFFFFFFu];
+        }
+        // the warp's OR
+        unsigned int lo = (unsigned int)acc, hi = (unsigned int)(acc >> 32);
+        lo = __reduce_or_sync(0xffffffffu, lo);
+        hi = __reduce_or_sync(0xffffffffu, hi);
+        acc = ((unsigned long long)hi << 32) | lo;
+        if ((acc & pending) == pending) {
+          j += 128;
+          break;
+        }
+      }
+      if (lane == 0) {
+        edges += min(j, end) - r.x;
+        const unsigned long long m = acc & pending;
+        if (m) N[v] = m;
+      }
+    }
+    if (lane == 0 && edges) atomicAdd(&ctl->edges, (unsigned long long)edges);
+    return;
+  }
+  const uint32_t nb = gridDim.x - nb_heavy;
+  for (uint32_t v = (blockIdx.x - nb_heavy) * blockDim.x + threadIdx.x; v < V; v += nb * blockDim.x) {
     const unsigned long long pending = lanes & ~vis[v];
     if (!pending) continue;
-    const uint2 r = rows[v];
+    const uint2 r = rows_i[v];
     if (r.y == 0 || r.y > kMsLight) continue;
     unsigned long long acc = 0;
     uint32_t j = r.x;
@@ -196,7 +234,7 @@ __global__ void __launch_bounds__(256) msk_pull_light(uint32_t V, unsigned long 
     for (; j < end; j += 4) {
       unsigned long long f[4];
 #pragma unroll
-      for (int k = 0; k < 4; k++) f[k] = (j + k < end) ? F[__ldg(&nbr[j + k]) & 0x3FFFFFFFu] : 0ull;
+      for (int k = 0; k < 4; k++) f[k] = (j + k < end) ? F[__ldg(&nbr_i[j + k]) & 0x3FFFFFFFu] : 0ull;
       acc |= f[0] | f[1] | f[2] | f[3];
       if ((acc & pending) == pending) {
         j += 4;
@@ -204,55 +242,36 @@ __global__ void __launch_bounds__(256) msk_pull_light(uint32_t V, unsigned long 
       }
     }
     edges += min(j, end) - r.x;
-    const unsigned long long n = acc & pending;
-    if (n) N[v] = n;
+    const unsigned long long m = acc & pending;
+    if (m) N[v] = m;
   }
   warp_atomic_add_total64(&ctl->edges, edges);
 }
 
-// pull, long rows: a warp per vertex of the heavy list, lanes strided, the
-// warp's OR checked every 128 edges
-__global__ void __launch_bounds__(256) msk_pull_heavy(const uint32_t* __restrict__ heavy, uint32_t n_heavy,
-                                                      unsigned long long lanes, const uint2* __restrict__ rows,
-                                                      const uint32_t* __restrict__ nbr,
-                                                      const unsigned long long* __restrict__ F,
-                                                      const unsigned long long* __restrict__ vis,
-                                                      unsigned long long* __restrict__ N, MsCtl* __restrict__ ctl) {
-  const uint32_t lane = lane_id();
-  const uint32_t gw = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+// push: the pieces of the long rows, a warp each
+__global__ void __launch_bounds__(256) msk_push_long(const uint4* __restrict__ items,
+                                                     const uint32_t* __restrict__ nbr_f,
+                                                     const unsigned long long* __restrict__ F,
+                                                     const unsigned long long* __restrict__ vis, unsigned long long* N,
+                                                     const MsCtl* __restrict__ ctl) {
+  if (ctl->done || ctl->pull) return;
+  const uint32_t n = ctl->items, lane = lane_id();
   const uint32_t nw = gridDim.x * (blockDim.x / 32);
-  uint32_t edges = 0;
-  for (uint32_t t = gw; t < n_heavy; t += nw) {
-    const uint32_t v = heavy[t];
-    const unsigned long long pending = lanes & ~vis[v];
-    if (!pending) continue;
-    const uint2 r = rows[v];
-    const uint32_t end = r.x + r.y;
-    unsigned long long acc = 0;
-    uint32_t j = r.x;
-    for (; j < end; j += 128) {
+  for (uint32_t t = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); t < n; t += nw) {
+    const uint4 it = items[t];
+    const unsigned long long fu = F[it.x];
+    const unsigned long long f[4] = {fu, fu, fu, fu};
+    for (uint32_t j = it.y + lane; j < it.z; j += 128) {
+      uint32_t w[4];
+      bool ok[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const uint32_t jj = j + k * 32 + lane;
-        if (jj < end) acc |= F[__ldg(&nbr[jj]) & 0x3FFFFFFFu];
+        ok[k] = j + k * 32 < it.z;
+        w[k] = ok[k] ? (__ldg(&nbr_f[j + k * 32]) & 0x3FFFFFFFu) : 0u;
       }
-      // the warp's OR
-      unsigned int lo = (unsigned int)acc, hi = (unsigned int)(acc >> 32);
-      lo = __reduce_or_sync(0xffffffffu, lo);
-      hi = __reduce_or_sync(0xffffffffu, hi);
-      acc = ((unsigned long long)hi << 32) | lo;
-      if ((acc & pending) == pending) {
-        j += 128;
-        break;
-      }
-    }
-    if (lane == 0) {
-      edges += min(j, end) - r.x;
-      const unsigned long long n = acc & pending;
-      if (n) N[v] = n;
+      ms_push4(f, w, ok, vis, N);
     }
   }
-  if (lane == 0 && edges) atomicAdd(&ctl->edges, (unsigned long long)edges);
 }
 
 // Next words -> new frontier: visited lanes, the depths of the newly reached
@@ -260,33 +279,38 @@ __global__ void __launch_bounds__(256) msk_pull_heavy(const uint32_t* __restrict
 // covers 32 consecutive vertices; for each of them that gained lanes, the
 // whole warp writes its depths (lane l: depth lanes l and l + 32 of the
 // vertex's 128-byte row, 2-byte stores, no read -- every (vertex, lane) is
-// written once).
-__global__ void __launch_bounds__(256) msk_finish(uint32_t V, uint16_t level, unsigned long long* __restrict__ F,
+// written once).  The last CTA makes the counted frontier the next level's.
+__global__ void __launch_bounds__(256) msk_finish(uint32_t V, uint32_t E, unsigned long long* __restrict__ F,
                                                   unsigned long long* __restrict__ N,
                                                   unsigned long long* __restrict__ vis,
                                                   uint16_t* __restrict__ depth, const uint32_t* __restrict__ out_degree,
-                                                  uint32_t* __restrict__ list, MsCtl* __restrict__ ctl) {
+                                                  uint32_t* __restrict__ list, MsCtl* ctl) {
+  if (ctl->done) return;
   __shared__ BlockAppend<1024> q;
   __shared__ unsigned long long s_red[8];
   ba_init(q);
+  const uint16_t level = (uint16_t)(ctl->levels + 1);
   const uint32_t lane = lane_id();
-  unsigned long long mf = 0, reached = 0;
+  unsigned long long mf = 0;
+  uint32_t reached = 0;
   for (uint32_t base = blockIdx.x * 1024; base < V; base += gridDim.x * 1024) {
+    const uint32_t wb = base + (threadIdx.x & ~31u);
+    unsigned long long nx[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) nx[k] = wb + k * 256 + lane < V ? N[wb + k * 256 + lane] : 0ull;
 #pragma unroll
     for (uint32_t k = 0; k < 4; k++) {
-      const uint32_t w0 = base + k * 256 + (threadIdx.x & ~31u);
-      const uint32_t v = w0 + lane;
+      const uint32_t w0 = wb + k * 256, v = w0 + lane;
       unsigned long long n = 0;
       if (v < V) {
-        const unsigned long long nx = N[v];
-        if (nx) {
+        if (nx[k]) {
           const unsigned long long vi = vis[v];
-          n = nx & ~vi;
+          n = nx[k] & ~vi;
           N[v] = 0;
           if (n) {
             vis[v] = vi | n;
             mf += out_degree[v];
-            reached += (unsigned long long)__popcll(n);
+            reached += __popcll(n);
             ba_push(q, v);
           }
         }
@@ -302,10 +326,38 @@ __global__ void __launch_bounds__(256) msk_finish(uint32_t V, uint16_t level, un
         if ((f >> (lane + 32)) & 1ull) row[lane + 32] = level;
       }
     }
-    ba_flush(q, list, &ctl->nlist);
+    if (ba_size(q)) ba_flush(q, list, &ctl->next_n);
   }
-  block_add_total<unsigned long long>(&ctl->mf, mf, s_red);
-  block_add_total<unsigned long long>(&ctl->reached, reached, s_red);
+  block_add_total<unsigned long long>(&ctl->next_mf, mf, s_red);
+  block_add_total<unsigned long long>(&ctl->reached, (unsigned long long)reached, s_red);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&ctl->ctas, 1u) == gridDim.x - 1) {
+      __threadfence();
+      MsCtl c;
+      c.nlist = atomicAdd(&ctl->next_n, 0u);
+      c.mf = atomicAdd(&ctl->next_mf, 0ull);
+      c.levels = ctl->levels + 1;
+      c.done = 0;
+      c.pull = ctl->pull;
+      if (c.pull) {
+        ctl->pull_levels++;
+      } else {
+        ctl->push_levels++;
+        ctl->edges += ctl->mf;  // a push level reads every out-edge of its frontier
+      }
+      ms_next_level(c, E);
+      ctl->nlist = c.nlist;
+      ctl->mf = c.mf;
+      ctl->levels = c.levels;
+      ctl->pull = c.pull;
+      ctl->next_n = 0;
+      ctl->next_mf = 0;
+      ctl->items = 0;
+      ctl->ctas = 0;
+      ctl->done = c.done;
+    }
+  }
 }
 
 // vertices with more than kMsLight in-edges (built once per graph)
@@ -326,14 +378,14 @@ static int ms_work_get(DevGraph& g, MsWork** out, cudaStream_t s) {
     OGB_TRY(w->N.alloc((size_t)V * 8 + 16));
     OGB_TRY(w->vis.alloc((size_t)V * 8 + 16));
     OGB_TRY(w->list.alloc((size_t)V * 4 + 16));
-    OGB_TRY(w->cnt.alloc((size_t)V * 4 + 16));
-    OGB_TRY(w->off.alloc((size_t)V * 4 + 16));
     OGB_TRY(w->heavy.alloc((size_t)V * 4 + 16));
-    OGB_TRY(w->scan_tmp.alloc(scan_tmp_words(V) * 4));
     OGB_TRY(w->ctl.alloc(sizeof(MsCtl) + 16));
+    OGB_TRY(w->roots.alloc(64 * 12 + 32));
     w->V = V;
     w->heavy_ready = false;
   }
+  // pieces of out-rows longer than kMsLong: at most two per kMsLong edges
+  OGB_TRY(w->items.alloc(((size_t)g.E / kMsLong * 2 + 2) * sizeof(uint4)));
   if (!w->h_ctl) OGB_CUDA(cudaMallocHost(&w->h_ctl, sizeof(MsCtl)));
   if (!w->ev0) {
     OGB_CUDA(cudaEventCreate(&w->ev_init));
@@ -375,10 +427,8 @@ int msbfs_run(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint16_t* dep
     }
   }
   const unsigned long long lanes = nroots == 64 ? ~0ull : ((1ull << nroots) - 1);
-  DevBuf d_roots;
-  OGB_TRY(d_roots.alloc(verts.size() * 12 + 32));
-  uint32_t* d_verts = d_roots.as<uint32_t>();
-  unsigned long long* d_masks = reinterpret_cast<unsigned long long*>(d_roots.as<char>() + ((verts.size() * 4 + 15) & ~15ull));
+  uint32_t* d_verts = w->roots.as<uint32_t>();
+  unsigned long long* d_masks = reinterpret_cast<unsigned long long*>(w->roots.as<char>() + 64 * 4);
   OGB_CUDA(cudaMemcpyAsync(d_verts, verts.data(), verts.size() * 4, cudaMemcpyHostToDevice, s));
   OGB_CUDA(cudaMemcpyAsync(d_masks, masks.data(), masks.size() * 8, cudaMemcpyHostToDevice, s));
 
@@ -399,61 +449,38 @@ int msbfs_run(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint16_t* dep
   OGB_CUDA(cudaMemsetAsync(vis, 0, (size_t)V * 8, s));
   OGB_CUDA(cudaMemsetAsync(ctl, 0, sizeof(MsCtl), s));
   msk_roots<<<1, 64, 0, s>>>(d_verts, d_masks, (uint32_t)verts.size(), F, vis, depth, w->list.as<uint32_t>(),
-                             g.fwd.d_out_degree(), ctl);
+                             g.fwd.d_out_degree(), g.E, ctl);
   OGB_CUDA(cudaGetLastError());
   OGB_CUDA(cudaEventRecord(w->ev0, s));
-  OGB_CUDA(cudaMemcpyAsync(w->h_ctl, ctl, sizeof(MsCtl), cudaMemcpyDeviceToHost, s));
-  OGB_CUDA(cudaStreamSynchronize(s));
-  uint32_t nlist = w->h_ctl->nlist;
-  unsigned long long mf = w->h_ctl->mf;
-  MsResult r;
-  r.reached = verts.size() ? __builtin_popcountll(lanes) : 0;
-  uint32_t level = 0, launches = 6;
-  while (nlist > 0) {
-    if (level >= 0xFFFE) return fail(ERR_UNSUPPORTED, "msbfs: more than 65534 levels");
-    level++;
-    OGB_CUDA(cudaMemsetAsync(ctl, 0, sizeof(MsCtl), s));
-    const bool push = mf < (unsigned long long)g.E / kMsAlpha;
-    if (push) {
-      if (nlist <= kMsSmallScan) {
-        msk_small_scan<<<1, 1024, 0, s>>>(w->list.as<uint32_t>(), nlist, rows_f, w->off.as<uint32_t>());
-        launches += 1;
-      } else {
-        msk_frontier_degree<<<std::min<uint32_t>(sms * 8, ceil_div(nlist, 256)), 256, 0, s>>>(
-            w->list.as<uint32_t>(), nlist, rows_f, w->cnt.as<uint32_t>());
-        OGB_TRY(scan_exclusive_u32(w->cnt.as<uint32_t>(), w->off.as<uint32_t>(), nlist, w->scan_tmp.as<uint32_t>(),
-                                   s));
-        launches += 4;
-      }
-      msk_push<<<sms * 8, 256, 0, s>>>(w->list.as<uint32_t>(), nlist, w->off.as<uint32_t>(), rows_f, g.fwd.d_dst(), F,
-                                      vis, N, ctl);
-      launches += 1;
-      r.push_levels++;
-    } else {
-      msk_pull_light<<<sms * 8, 256, 0, s>>>(V, lanes, rows_i, g.inv.d_dst(), F, vis, N, ctl);
-      if (w->n_heavy)
-        msk_pull_heavy<<<sms * 8, 256, 0, s>>>(w->heavy.as<uint32_t>(), w->n_heavy, lanes, rows_i, g.inv.d_dst(), F,
-                                              vis, N, ctl);
-      launches += 2;
-      r.pull_levels++;
+  const uint32_t nb_heavy = w->n_heavy ? std::min<uint32_t>(sms * 8, ceil_div(w->n_heavy, 8)) : 0;
+  const uint32_t nb_light = std::max<uint32_t>(1, std::min<uint32_t>(sms * 8, ceil_div(V, 256)));
+  const uint32_t nb_finish = std::max<uint32_t>(1, std::min<uint32_t>(sms * 8, ceil_div(V, 1024)));
+  uint32_t launches = 6;
+  do {
+    for (int k = 0; k < kMsBatch; k++) {
+      msk_expand<<<nb_heavy + nb_light, 256, 0, s>>>(V, lanes, nb_heavy, w->heavy.as<uint32_t>(), w->n_heavy, rows_f,
+                                                     g.fwd.d_dst(), rows_i, g.inv.d_dst(), F, vis, N,
+                                                     w->list.as<uint32_t>(), w->items.as<uint4>(), ctl);
+      msk_push_long<<<sms * 4, 256, 0, s>>>(w->items.as<uint4>(), g.fwd.d_dst(), F, vis, N, ctl);
+      msk_finish<<<nb_finish, 256, 0, s>>>(V, g.E, F, N, vis, depth, g.fwd.d_out_degree(), w->list.as<uint32_t>(),
+                                           ctl);
     }
-    msk_finish<<<sms * 8, 256, 0, s>>>(V, (uint16_t)level, F, N, vis, depth, g.fwd.d_out_degree(),
-                                       w->list.as<uint32_t>(), ctl);
+    launches += 3 * kMsBatch;
     OGB_CUDA(cudaGetLastError());
+    OGB_CUDA(cudaEventRecord(w->ev1, s));
     OGB_CUDA(cudaMemcpyAsync(w->h_ctl, ctl, sizeof(MsCtl), cudaMemcpyDeviceToHost, s));
     OGB_CUDA(cudaStreamSynchronize(s));
-    launches += 2;
-    nlist = w->h_ctl->nlist;
-    mf = w->h_ctl->mf;
-    r.reached += w->h_ctl->reached;
-    r.edges_examined += w->h_ctl->edges;
-  }
-  OGB_CUDA(cudaEventRecord(w->ev1, s));
-  OGB_CUDA(cudaEventSynchronize(w->ev1));
+  } while (!w->h_ctl->done);
+  if (w->h_ctl->done == 2) return fail(ERR_UNSUPPORTED, "msbfs: more than 65534 levels");
+  MsResult r;
+  r.reached = (unsigned long long)__builtin_popcountll(lanes) + w->h_ctl->reached;
+  r.edges_examined = w->h_ctl->edges;
+  r.push_levels = w->h_ctl->push_levels;
+  r.pull_levels = w->h_ctl->pull_levels;
   float ms = 0.f, init_ms = 0.f;
   OGB_CUDA(cudaEventElapsedTime(&ms, w->ev0, w->ev1));
   OGB_CUDA(cudaEventElapsedTime(&init_ms, w->ev_init, w->ev0));
-  r.levels = level;
+  r.levels = w->h_ctl->levels;
   r.ms = ms;
   r.init_ms = init_ms;
   r.launches = launches;
