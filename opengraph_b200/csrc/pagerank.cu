@@ -340,10 +340,11 @@ struct StagePipe {
 //  (3) light rows, a warp per 32 R consecutive vertices: their edges are
 //      contiguous, gathered into the stage the same way, and each lane adds
 //      its R rows' values in CSR order.
-// A warp's first unit of either kind is its own index (the light ones counted
-// from the other end, so that a graph with few medium units spreads over all
-// warps); only when there are more units than warps are the rest handed out by
-// an atomic counter.  Claiming every unit from the counter cost 19 K atomics on
+// A warp's first unit of either kind is its own index, and on a small graph the
+// three kinds start at different warps, so that an iteration is as long as the
+// longest kind and not as their sum: chunks at the CTAs' last groups, medium
+// units at their first warps, light units at the warps after those.  Only when
+// there are more units than warps are the rest handed out by an atomic counter.  Claiming every unit from the counter cost 19 K atomics on
 // one address per iteration, more than a small graph's whole work (RMAT-22: 266
 // -> 257 us per iteration without them).
 // rows_rl, pr and out_degree are in original vertex order; contrib and
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
   // (1) chunks of very heavy rows, one group per chunk
   {
     const uint32_t grp = threadIdx.x / kPullGroup, gt = threadIdx.x % kPullGroup;
-    for (uint32_t g = blockIdx.x * kPullGroups + grp; g < n_chunks; g += gridDim.x * kPullGroups) {
+    for (uint32_t g = (kPullGroups - 1 - grp) * gridDim.x + blockIdx.x; g < n_chunks; g += gridDim.x * kPullGroups) {
       const PrChunkItem ci = chunks[g];
       float sum = strided_sum<kPullGroup>(contrib, nbr, ci.j0 + gt, ci.j1);
       sum = warp_fold(sum);
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
 
   // (3) light rows, a warp per 32 R consecutive vertices
   const uint32_t n_light = ceil_div_dev(p.V, 32 * R);
-  t = nwarps - 1 - gw;
+  t = n_units < nwarps ? (gw >= n_units ? gw - n_units : gw + nwarps - n_units) : gw;
   while (t < n_light) {
     const uint32_t t_next = (lane == 0 && n_light > nwarps) ? nwarps + atomicAdd(&ctl->claim_light[it], 1u) : n_light;
     const uint32_t base = t * (32 * R);
