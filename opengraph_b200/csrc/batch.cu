@@ -135,6 +135,8 @@ __global__ void __launch_bounds__(256) msk_expand(uint32_t V, unsigned long long
                                                   const unsigned long long* __restrict__ vis, unsigned long long* N,
                                                   const uint32_t* __restrict__ list, uint4* __restrict__ items,
                                                   MsCtl* ctl) {
+  wait_for_prior_kernel();
+  let_next_kernel_start();
   if (ctl->done) return;
   const uint32_t lane = lane_id();
   const uint32_t gw = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
@@ -254,6 +256,8 @@ __global__ void __launch_bounds__(256) msk_push_long(const uint4* __restrict__ i
                                                      const unsigned long long* __restrict__ F,
                                                      const unsigned long long* __restrict__ vis, unsigned long long* N,
                                                      const MsCtl* __restrict__ ctl) {
+  wait_for_prior_kernel();
+  let_next_kernel_start();
   if (ctl->done || ctl->pull) return;
   const uint32_t n = ctl->items, lane = lane_id();
   const uint32_t nw = gridDim.x * (blockDim.x / 32);
@@ -285,6 +289,8 @@ __global__ void __launch_bounds__(256) msk_finish(uint32_t V, uint32_t E, unsign
                                                   unsigned long long* __restrict__ vis,
                                                   uint16_t* __restrict__ depth, const uint32_t* __restrict__ out_degree,
                                                   uint32_t* __restrict__ list, MsCtl* ctl) {
+  wait_for_prior_kernel();
+  let_next_kernel_start();
   if (ctl->done) return;
   __shared__ BlockAppend<1024> q;
   __shared__ unsigned long long s_red[8];
@@ -458,12 +464,13 @@ int msbfs_run(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint16_t* dep
   uint32_t launches = 6;
   do {
     for (int k = 0; k < kMsBatch; k++) {
-      msk_expand<<<nb_heavy + nb_light, 256, 0, s>>>(V, lanes, nb_heavy, w->heavy.as<uint32_t>(), w->n_heavy, rows_f,
-                                                     g.fwd.d_dst(), rows_i, g.inv.d_dst(), F, vis, N,
-                                                     w->list.as<uint32_t>(), w->items.as<uint4>(), ctl);
-      msk_push_long<<<sms * 4, 256, 0, s>>>(w->items.as<uint4>(), g.fwd.d_dst(), F, vis, N, ctl);
-      msk_finish<<<nb_finish, 256, 0, s>>>(V, g.E, F, N, vis, depth, g.fwd.d_out_degree(), w->list.as<uint32_t>(),
-                                           ctl);
+      OGB_CUDA(launch_dependent(msk_expand, nb_heavy + nb_light, 256, 0, s, V, lanes, nb_heavy,
+                                w->heavy.as<uint32_t>(), w->n_heavy, rows_f, g.fwd.d_dst(), rows_i, g.inv.d_dst(),
+                                F, vis, N, w->list.as<uint32_t>(), w->items.as<uint4>(), ctl));
+      OGB_CUDA(launch_dependent(msk_push_long, sms * 4, 256, 0, s, w->items.as<uint4>(), g.fwd.d_dst(), F, vis, N,
+                                ctl));
+      OGB_CUDA(launch_dependent(msk_finish, nb_finish, 256, 0, s, V, g.E, F, N, vis, depth, g.fwd.d_out_degree(),
+                                w->list.as<uint32_t>(), ctl));
     }
     launches += 3 * kMsBatch;
     OGB_CUDA(cudaGetLastError());
@@ -635,6 +642,8 @@ __global__ void __launch_bounds__(256, 6) pprk_iter(const PprChunk* __restrict__
                                                     float* __restrict__ R, PprParams p, PprCtl* __restrict__ ctl,
                                                     uint32_t it) {
   __shared__ double s_err[8][kPprSeeds];
+  wait_for_prior_kernel();
+  let_next_kernel_start();
   if (ctl->stop) return;
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
   const uint32_t grp = lane >> 3, sub = lane & 7, k = ppr_lane_seed(lane);
@@ -711,6 +720,8 @@ __global__ void __launch_bounds__(256, 6) pprk_iter(const PprChunk* __restrict__
 
 // the run stops after an iteration in which every seed changed by < eps (L1)
 __global__ void pprk_check(PprCtl* __restrict__ ctl, uint32_t it, uint32_t nseeds, double eps) {
+  wait_for_prior_kernel();
+  let_next_kernel_start();
   if (threadIdx.x != 0 || ctl->stop) return;
   bool all = true;
   for (uint32_t k = 0; k < nseeds; k++) all = all && (ctl->err[it][k] < eps);
@@ -815,11 +826,11 @@ int ppr_run(DevGraph& g, const uint32_t* seeds, uint32_t nseeds, uint32_t max_it
   pprk_seed<<<1, 32, 0, s>>>(p.seeds, nseeds, g.fwd.d_out_degree(), R, C);
   OGB_CUDA(cudaGetLastError());
   for (uint32_t it = 0; it < max_iters; it++) {
-    pprk_iter<<<sms * 6, 256, 0, s>>>(w->chunks.as<PprChunk>(), w->n_chunks, w->vfirst.as<uint32_t>(),
-                                      w->vcount.as<uint32_t>(), w->done.as<uint32_t>(), w->partials.as<float>(),
-                                      w->light.as<uint32_t>(), it < 2 ? w->n_light : w->n_fed, g.inv.d_rows(), g.inv.d_dst(),
-                                      g.fwd.d_out_degree(), C, Cn, R, p, ctl, it);
-    pprk_check<<<1, 32, 0, s>>>(ctl, it, nseeds, epsilon);
+    OGB_CUDA(launch_dependent(pprk_iter, sms * 6, 256, 0, s, w->chunks.as<PprChunk>(), w->n_chunks,
+                              w->vfirst.as<uint32_t>(), w->vcount.as<uint32_t>(), w->done.as<uint32_t>(),
+                              w->partials.as<float>(), w->light.as<uint32_t>(), it < 2 ? w->n_light : w->n_fed,
+                              g.inv.d_rows(), g.inv.d_dst(), g.fwd.d_out_degree(), C, Cn, R, p, ctl, it));
+    OGB_CUDA(launch_dependent(pprk_check, 1, 32, 0, s, ctl, it, nseeds, epsilon));
     OGB_CUDA(cudaGetLastError());
     std::swap(C, Cn);
   }

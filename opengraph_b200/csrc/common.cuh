@@ -194,6 +194,34 @@ __device__ __forceinline__ void ba_flush(BlockAppend<CAP>& q, uint32_t* out, uin
   __syncthreads();
 }
 
+// A kernel launched by launch_dependent may start before the kernel ahead of it
+// in the stream has ended: wait_for_prior_kernel, its first statement, then waits
+// for that end and for the earlier kernel's writes, so only the launch itself
+// overlaps.  let_next_kernel_start lets the kernel behind this one do the same.
+__device__ __forceinline__ void wait_for_prior_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_kernel(void (*kernel)(P...), bool dependent, unsigned grid, unsigned threads, size_t smem,
+                                 cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
+                                    cudaStream_t s, A... args) {
+  return launch_kernel(kernel, true, grid, threads, smem, s, args...);
+}
+
 inline unsigned ceil_div(uint64_t a, uint64_t b) { return (unsigned)((a + b - 1) / b); }
 
 }  // namespace ogb

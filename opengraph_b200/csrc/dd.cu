@@ -673,6 +673,8 @@ struct SpmvPullPolicy {
 __global__ void __launch_bounds__(kT) spmv_pull_kernel(const uint2* __restrict__ rows, const uint32_t* __restrict__ med,
                                                        HeavyRows heavy, Grid3 G, SpmvPullPolicy pol,
                                                        const DdCtl* __restrict__ ctl, uint32_t V) {
+  wait_for_prior_kernel();
+  let_next_kernel_start();
   rows_pass(blockIdx.x, rows, med, heavy, ctl->n_med, ctl->n_hch, V, G.heavy, G.med, G.light, pol);
 }
 
@@ -915,7 +917,8 @@ int spmv_run(DevGraph& g, uint32_t mode, uint32_t iterations, float* x, float* y
     const Grid3 G = rows_grid(V);
     SpmvPullPolicy pol{g.inv.d_dst(), g.weighted ? g.inv.d_w() : nullptr, x, y};
     for (uint32_t it = 0; it < iterations; it++)
-      spmv_pull_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), G, pol, w->ctl.as<DdCtl>(), V);
+      OGB_CUDA(launch_dependent(spmv_pull_kernel, G.total(), kT, 0, s, g.inv.d_rows(), w->med.as<uint32_t>(),
+                                w->heavy.view(), G, pol, w->ctl.as<DdCtl>(), V));
   } else {
     for (uint32_t it = 0; it < iterations; it++)
       spmv_push_kernel<<<sms * 8, kT, 0, s>>>(V, g.fwd.d_rows(), g.fwd.d_dst(), g.weighted ? g.fwd.d_w() : nullptr, x,
