@@ -731,6 +731,40 @@ __global__ void pprk_check(PprCtl* __restrict__ ctl, uint32_t it, uint32_t nseed
   }
 }
 
+// The vertices by class: in-edges but no chunks, number of chunks, chunked.
+__global__ void pprk_classes(uint32_t V, const uint2* __restrict__ rows, uint32_t* __restrict__ fed,
+                             uint32_t* __restrict__ nchunk, uint32_t* __restrict__ cut) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    const uint32_t d = rows[v].y;
+    fed[v] = d && d <= kPprChunk ? 1u : 0u;
+    nchunk[v] = d > kPprChunk ? (d + kPprChunk - 1) / kPprChunk : 0u;
+    cut[v] = d > kPprChunk ? 1u : 0u;
+  }
+}
+
+// From the classes' scans: the vertices without chunks, those with in-edges
+// first, each part in vertex order; and the chunk table.  (Built on the host from
+// a copy of the rows, these lists took longer than the iterations.)
+__global__ void pprk_lists(uint32_t V, const uint2* __restrict__ rows, const uint32_t* __restrict__ fed,
+                           const uint32_t* __restrict__ nchunk, const uint32_t* __restrict__ cut, uint32_t n_fed,
+                           uint32_t* __restrict__ light, PprChunk* __restrict__ chunks, uint32_t* __restrict__ vfirst,
+                           uint32_t* __restrict__ vcount, uint32_t* __restrict__ done) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    const uint2 r = rows[v];
+    const uint32_t k = cut[v];
+    if (r.y > kPprChunk) {
+      const uint32_t at = nchunk[v], n = (r.y + kPprChunk - 1) / kPprChunk;
+      vfirst[k] = at;
+      vcount[k] = n;
+      done[k] = 0;
+      for (uint32_t c = 0; c < n; c++)
+        chunks[at + c] = {v, r.x + c * kPprChunk, r.x + min(r.y, (c + 1) * kPprChunk), k};
+    } else {
+      light[r.y ? fed[v] : n_fed + (v - fed[v] - k)] = v;
+    }
+  }
+}
+
 static int ppr_work_get(DevGraph& g, PprWork** out, cudaStream_t s) {
   if (!g.ppr) g.ppr = new PprWork();
   PprWork* w = g.ppr;
@@ -752,45 +786,39 @@ static int ppr_work_get(DevGraph& g, PprWork** out, cudaStream_t s) {
   if (!w->ready || w->build != g.build_id) {
     // rows from the inverse CSR: rows over kPprChunk in-edges become chunks
     const uint2* rows = g.inv.d_rows();
-    std::vector<uint2> h_rows(V);
-    OGB_CUDA(cudaMemcpyAsync(h_rows.data(), rows, (size_t)V * 8, cudaMemcpyDeviceToHost, s));
-    OGB_CUDA(cudaStreamSynchronize(s));
-    std::vector<uint32_t> light;
-    std::vector<PprChunk> chunks;
-    std::vector<uint32_t> first, count;
-    light.reserve(V);
-    for (uint32_t v = 0; v < V; v++) {
-      const uint2 r = h_rows[v];
-      if (r.y > kPprChunk) {
-        const uint32_t k = (uint32_t)first.size();
-        first.push_back((uint32_t)chunks.size());
-        for (uint32_t c = 0; c < r.y; c += kPprChunk) chunks.push_back({v, r.x + c, r.x + std::min(r.y, c + kPprChunk), k});
-        count.push_back((uint32_t)chunks.size() - first.back());
-      } else if (r.y) {
-        light.push_back(v);
-      }
+    const size_t Vp = (size_t)V + 4;
+    DevBuf tmp;
+    OGB_TRY(tmp.alloc((Vp * 6 + scan_tmp_words(V)) * 4));
+    uint32_t* cls[3];  // vertices with in-edges and no chunks, chunks, chunked vertices: counts, then their scans
+    uint32_t* pos[3];
+    for (int i = 0; i < 3; i++) {
+      cls[i] = tmp.as<uint32_t>() + (size_t)i * Vp;
+      pos[i] = tmp.as<uint32_t>() + (size_t)(3 + i) * Vp;
     }
-    w->n_fed = (uint32_t)light.size();
-    for (uint32_t v = 0; v < V; v++)
-      if (!h_rows[v].y) light.push_back(v);
-    w->n_light = (uint32_t)light.size();
-    w->n_chunks = (uint32_t)chunks.size();
-    w->n_cut = (uint32_t)first.size();
+    const int grid = sm_count() * 8;
+    pprk_classes<<<grid, 256, 0, s>>>(V, rows, cls[0], cls[1], cls[2]);
+    OGB_CUDA(cudaGetLastError());
+    uint32_t total[3];
+    for (int i = 0; i < 3; i++) {
+      OGB_TRY(scan_exclusive_u32(cls[i], pos[i], V, tmp.as<uint32_t>() + 6 * Vp, s));
+      OGB_CUDA(cudaMemcpyAsync(&total[i], pos[i] + V, 4, cudaMemcpyDeviceToHost, s));
+    }
+    OGB_CUDA(cudaStreamSynchronize(s));
+    w->n_fed = total[0];
+    w->n_chunks = total[1];
+    w->n_cut = total[2];
+    w->n_light = V - w->n_cut;
     OGB_TRY(w->light.alloc((size_t)w->n_light * 4 + 16));
     OGB_TRY(w->chunks.alloc((size_t)w->n_chunks * sizeof(PprChunk) + 16));
     OGB_TRY(w->partials.alloc((size_t)w->n_chunks * kPprSeeds * 4 + 16));
     OGB_TRY(w->vfirst.alloc((size_t)w->n_cut * 4 + 16));
     OGB_TRY(w->vcount.alloc((size_t)w->n_cut * 4 + 16));
     OGB_TRY(w->done.alloc((size_t)w->n_cut * 4 + 16));
-    if (w->n_light) OGB_CUDA(cudaMemcpyAsync(w->light.p, light.data(), light.size() * 4, cudaMemcpyHostToDevice, s));
-    if (w->n_chunks)
-      OGB_CUDA(cudaMemcpyAsync(w->chunks.p, chunks.data(), chunks.size() * sizeof(PprChunk), cudaMemcpyHostToDevice, s));
-    if (w->n_cut) {
-      OGB_CUDA(cudaMemcpyAsync(w->vfirst.p, first.data(), first.size() * 4, cudaMemcpyHostToDevice, s));
-      OGB_CUDA(cudaMemcpyAsync(w->vcount.p, count.data(), count.size() * 4, cudaMemcpyHostToDevice, s));
-    }
-    OGB_CUDA(cudaMemsetAsync(w->done.p, 0, (size_t)w->n_cut * 4 + 16, s));
-    OGB_CUDA(cudaStreamSynchronize(s));
+    pprk_lists<<<grid, 256, 0, s>>>(V, rows, pos[0], pos[1], pos[2], w->n_fed, w->light.as<uint32_t>(),
+                                    w->chunks.as<PprChunk>(), w->vfirst.as<uint32_t>(), w->vcount.as<uint32_t>(),
+                                    w->done.as<uint32_t>());
+    OGB_CUDA(cudaGetLastError());
+    OGB_CUDA(cudaStreamSynchronize(s));  // before the scratch is released
     w->ready = true;
     w->build = g.build_id;
   }
