@@ -911,8 +911,11 @@ __device__ __forceinline__ float pr_push_vtx(float s, float prev, uint32_t d, fl
 
 // Push update: next -> ranks and next contribs, next cleared.  Four vertices
 // per thread and step with 16-byte loads and stores (the arrays are 16-byte
-// aligned), so each thread keeps several loads in flight; a scalar tail.
-__global__ void __launch_bounds__(kPrThreads) pr_push_update_kernel(uint32_t V, const uint32_t* __restrict__ out_degree,
+// aligned), so each thread keeps several loads in flight; a scalar tail.  Two
+// CTAs of 512 threads per SM: eight CTAs of 256 spent most of the kernel in their
+// 1184 closing atomics on the same counters (18 us at RMAT-20).
+constexpr int kPushUpdThreads = 512;
+__global__ void __launch_bounds__(kPushUpdThreads) pr_push_update_kernel(uint32_t V, const uint32_t* __restrict__ out_degree,
                                                                     float* __restrict__ next,
                                                                     float* __restrict__ contrib_next,
                                                                     float* __restrict__ pr, PrParams p,
@@ -921,14 +924,14 @@ __global__ void __launch_bounds__(kPrThreads) pr_push_update_kernel(uint32_t V, 
   double err = 0.0;
   uint32_t active = 0;
   const double inv_v = 1.0 / (double)p.V;
-  const uint32_t stride = gridDim.x * kPrThreads;
+  const uint32_t stride = gridDim.x * kPushUpdThreads;
   const bool vec = !p.frozen && !p.delta &&
                    ((reinterpret_cast<uintptr_t>(next) | reinterpret_cast<uintptr_t>(contrib_next) |
                      reinterpret_cast<uintptr_t>(pr) | reinterpret_cast<uintptr_t>(out_degree)) & 15) == 0;
   uint32_t v0 = 0;
   if (vec) {
     const uint32_t nq = V / 4;
-    for (uint32_t q = blockIdx.x * kPrThreads + threadIdx.x; q < nq; q += stride) {
+    for (uint32_t q = blockIdx.x * kPushUpdThreads + threadIdx.x; q < nq; q += stride) {
       const float4 sv = reinterpret_cast<const float4*>(next)[q];
       const float4 pv = reinterpret_cast<const float4*>(pr)[q];
       const uint4 dv = reinterpret_cast<const uint4*>(out_degree)[q];
@@ -943,7 +946,7 @@ __global__ void __launch_bounds__(kPrThreads) pr_push_update_kernel(uint32_t V, 
     }
     v0 = nq * 4;
   }
-  for (uint32_t v = v0 + blockIdx.x * kPrThreads + threadIdx.x; v < V; v += stride) {
+  for (uint32_t v = v0 + blockIdx.x * kPushUpdThreads + threadIdx.x; v < V; v += stride) {
     const float sv = next[v];
     next[v] = 0.0f;
     if (vec) {
@@ -954,7 +957,7 @@ __global__ void __launch_bounds__(kPrThreads) pr_push_update_kernel(uint32_t V, 
       pr_update(v, sv, pr, out_degree, contrib_next, p, err, active);
     }
   }
-  pr_block_finish(err, active, ctl, it);
+  pr_block_finish<kPushUpdThreads>(err, active, ctl, it);
 }
 
 __global__ void pr_init_kernel(uint32_t V, const uint32_t* __restrict__ out_degree, const float* __restrict__ init,
@@ -1236,6 +1239,7 @@ int pagerank_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsilon,
   const uint32_t nb_hub = (!pull && w->n_hub_items)
                               ? std::min<uint32_t>(sms * 4, ceil_div(w->n_hub_items, T / 32)) : 0;
   const uint32_t grid = nb_hub + nb_chunk + nb_warp + nb_light;
+  const uint32_t nb_update = std::max<uint32_t>(1, std::min<uint32_t>(sms * 2, ceil_div(V, 4 * kPushUpdThreads)));
   const uint2* rows = w->rows_fp.as<uint2>();
   const uint32_t* nbr = w->nbr_fp.as<uint32_t>();
   const uint32_t* heavy = w->heavy.as<uint32_t>();
@@ -1249,7 +1253,7 @@ int pagerank_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsilon,
       pr_push_scatter_kernel<<<grid, T, 0, s>>>(nb_hub, w->hub_items.as<uint4>(), w->n_hub_items, g.inv.d_dst(),
                                                  nb_chunk, nb_warp, heavy, w->n_warp, chunks, w->n_chunks, V,
                                                  g_warp_thr, rows, nbr, c_cur, nxt, d_ctl);
-      pr_push_update_kernel<<<sms * 8, T, 0, s>>>(V, g.fwd.d_out_degree(), nxt, c_nxt, ranks, p, d_ctl, it);
+      pr_push_update_kernel<<<nb_update, kPushUpdThreads, 0, s>>>(V, g.fwd.d_out_degree(), nxt, c_nxt, ranks, p, d_ctl, it);
     }
     OGB_CUDA(cudaGetLastError());
     std::swap(c_cur, c_nxt);
