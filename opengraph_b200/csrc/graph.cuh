@@ -52,7 +52,7 @@ struct DevGraph {
   DevCSR fwd, inv;
   SortWorkspace sort_ws;
   DevBuf input_src, input_dst, input_w;  // staging of host uploads
-  DevBuf err;                            // u32 error word of the build kernels
+  DevBuf err;                            // u32 error words of the build kernels: CSR map, sorts
   DevBuf range_q;                        // scratch of the partitioned BFS steps (bfs_range.cu)
   uint32_t build_id = 0;  // bumped whenever the edges change (caches key on it)
   BfsWork* bfs = nullptr;

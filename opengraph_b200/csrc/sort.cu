@@ -6,9 +6,11 @@
 // ordered by key, ties kept in input order.
 //
 // Design (one pass = one kernel, no separate upsweep):
-//  * digit histograms of every 8-bit digit are built by one read of the keys;
-//    digits that are constant over all keys are skipped (for V = 2^22 only
-//    three passes run, the last with 6 live bits);
+//  * digit histograms of every digit are built by one read of the keys; digits
+//    that are constant over all keys are skipped.  Which passes run, and between
+//    which buffers, is decided on the device (plan_kernel): every pass is
+//    launched, and the skipped ones return at once, so a sort needs no round
+//    trip to the host;
 //  * each CTA claims a tile of kTile keys in launch order, ranks the keys of
 //    the tile stably with warp ballots (order = warp, item, lane, which is
 //    input order), publishes its per-digit counts and resolves the per-digit
@@ -16,8 +18,6 @@
 //  * keys and payloads are staged in shared memory in digit order and written
 //    out so that consecutive threads store consecutive addresses of a run.
 #include "sort.cuh"
-
-#include <vector>
 
 namespace ogb {
 
@@ -51,11 +51,16 @@ __device__ __forceinline__ void lb_store(uint32_t* p, uint32_t v) {
 __device__ __forceinline__ void lb_store(unsigned long long* p, unsigned long long v) { st_volatile_u64(p, v); }
 
 // counters layout (u32): [0, kMaxPasses) tile counters, [kMaxPasses] error
-// word, [kMaxPasses+1] OR of all primary keys, [kMaxPasses+2] OR of all
-// secondary keys.
+// word; then a PassPlan per pass.
 constexpr int kCtrErr = kMaxPasses;
-constexpr int kCtrOr0 = kMaxPasses + 1;
-constexpr int kCtrWords = kMaxPasses + 4;
+constexpr int kCtrPlan = kMaxPasses + 4;
+
+// One pass: whether it runs, and its buffers (0 the input, 1 the scratch set, 2
+// the output).
+struct PassPlan {
+  uint32_t active, src, dst, pad;
+};
+constexpr int kCtrWords = kCtrPlan + kMaxPasses * (int)(sizeof(PassPlan) / 4);
 
 __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_t* s_warp) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -82,9 +87,8 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_
 }
 
 // Histograms of `ndig` digits of keys[0, n) into hist[ndig][256] (digit d
-// = (key >> 8-aligned or narrower lay.shift[d]) & lay.mask[d]) and the OR of
-// all keys into *or_out.  Each warp counts into its own copy of
-// the histograms in shared memory (conflicts only inside a warp's atomic),
+// = (key >> 8-aligned or narrower lay.shift[d]) & lay.mask[d]).  Each warp
+// counts into its own copy of the histograms in shared memory (conflicts only inside a warp's atomic),
 // and the copies are summed once at the end.
 // The digits of one key: ndig groups of at most 8 bits from bit 0 up.
 struct DigitLayout {
@@ -113,15 +117,11 @@ static DigitLayout digit_layout(uint32_t bits) {
 constexpr int kHistThreads = 256, kHistWarps = kHistThreads / 32;
 __global__ void __launch_bounds__(kHistThreads) digit_hist_kernel(const uint32_t* __restrict__ keys, uint64_t n,
                                                                   int ndig, DigitLayout lay,
-                                                                  uint32_t* __restrict__ hist,
-                                                                  uint32_t* __restrict__ or_out) {
+                                                                  uint32_t* __restrict__ hist) {
   __shared__ uint32_t sh[kHistWarps][4][256];
-  __shared__ uint32_t s_or;
   for (int i = threadIdx.x; i < kHistWarps * 4 * 256; i += blockDim.x) (&sh[0][0][0])[i] = 0;
-  if (threadIdx.x == 0) s_or = 0;
   __syncthreads();
   uint32_t(*h)[256] = sh[threadIdx.x >> 5];
-  uint32_t acc_or = 0;
   const uint64_t nvec = n / 4;
   const uint4* kv = reinterpret_cast<const uint4*>(keys);
   const bool aligned = (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
@@ -133,7 +133,6 @@ __global__ void __launch_bounds__(kHistThreads) digit_hist_kernel(const uint32_t
       const uint32_t a[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        acc_or |= a[j];
 #pragma unroll
         for (int d = 0; d < 4; d++)
           if (d < ndig) atomicAdd(&h[d][(a[j] >> lay.shift[d]) & lay.mask[d]], 1u);
@@ -144,13 +143,10 @@ __global__ void __launch_bounds__(kHistThreads) digit_hist_kernel(const uint32_t
   for (uint64_t i = start_scalar + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t k = keys[i];
-    acc_or |= k;
 #pragma unroll
     for (int d = 0; d < 4; d++)
       if (d < ndig) atomicAdd(&h[d][(k >> lay.shift[d]) & lay.mask[d]], 1u);
   }
-  acc_or = __reduce_or_sync(0xffffffffu, acc_or);
-  if ((threadIdx.x & 31) == 0) atomicOr(&s_or, acc_or);
   __syncthreads();
   for (int i = threadIdx.x; i < ndig * 256; i += blockDim.x) {
     uint32_t c = 0;
@@ -158,16 +154,39 @@ __global__ void __launch_bounds__(kHistThreads) digit_hist_kernel(const uint32_t
     for (int w = 0; w < kHistWarps; w++) c += (&sh[w][0][0])[i];
     if (c) atomicAdd(&hist[i], c);
   }
-  if (threadIdx.x == 0) atomicOr(or_out, s_or);
 }
 
-// Exclusive scan of each 256-bucket histogram (one block per histogram).
-__global__ void __launch_bounds__(256) digit_scan_kernel(const uint32_t* __restrict__ hist,
-                                                         uint32_t* __restrict__ base) {
+// The histogram of each pass.
+struct PlanHists {
+  int h[kMaxPasses];
+};
+
+// One CTA: the exclusive scan of every pass's 256-bucket histogram, and the
+// passes that run -- those whose digit is not the same in all n keys, or, if all
+// are, the last one (a stable copy).  The output buffer is the last active pass's;
+// they alternate before it.
+__global__ void __launch_bounds__(256) plan_kernel(const uint32_t* __restrict__ hist, uint32_t* __restrict__ base,
+                                                   uint32_t n, PlanHists hists, int passes, PassPlan* __restrict__ plan) {
   __shared__ uint32_t s_warp[kWarps];
-  uint32_t v = hist[blockIdx.x * 256 + threadIdx.x];
-  uint32_t e = block_exclusive_scan_256(v, s_warp);
-  base[blockIdx.x * 256 + threadIdx.x] = e;
+  uint32_t live = 0;
+  for (int j = 0; j < passes; j++) {
+    const int h = hists.h[j];
+    const uint32_t v = hist[h * 256 + threadIdx.x];
+    base[h * 256 + threadIdx.x] = block_exclusive_scan_256(v, s_warp);
+    if (!__syncthreads_or(v == n)) live |= 1u << j;
+  }
+  if (threadIdx.x != 0) return;
+  if (!live) live = 1u << (passes - 1);
+  uint32_t left = __popc(live), src = 0;
+  for (int j = 0; j < passes; j++) {
+    PassPlan p = {};
+    if ((live >> j) & 1u) {
+      left--;
+      p = {1u, src, left % 2 == 0 ? 2u : 1u, 0u};
+      src = p.dst;
+    }
+    plan[j] = p;
+  }
 }
 
 __device__ __forceinline__ void cp_async_u32(uint32_t* dst_smem, const uint32_t* src) {
@@ -198,8 +217,9 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d, uint32_t valid) {
   return p;
 }
 
+// The arrays a tile works on, and the pass's digit.
 template <class S>
-struct PassArgs {
+struct TileArgs {
   const uint32_t* kin;
   const uint32_t* p0in;
   const uint32_t* p1in;
@@ -209,8 +229,20 @@ struct PassArgs {
   uint32_t n, shift, mask;
   const uint32_t* digit_base;
   S* status;
+  uint32_t* err;
+};
+
+// A launched pass: the three buffers it may work between (as key and first
+// payload of this pass), its digit and its entry of the plan.
+template <class S>
+struct PassArgs {
+  uint32_t *k[3], *p0[3], *p1[3];
+  uint32_t n, shift, mask;
+  const uint32_t* digit_base;
+  S* status;
   uint32_t* tile_ctr;
   uint32_t* err;
+  const PassPlan* plan;
 };
 
 // One pass over one tile.  Only the keys pass through registers: once the
@@ -229,7 +261,7 @@ struct PassArgs {
 // look-back word at a time and 32-bit histograms.  512 threads (476 us), 20 keys
 // per thread (457 us) and payloads through registers were slower.
 template <bool HAS_P1, int NB, class S, bool FULL>
-__device__ __forceinline__ void onesweep_tile(const PassArgs<S>& a, uint32_t tile, uint32_t* s_dyn,
+__device__ __forceinline__ void onesweep_tile(const TileArgs<S>& a, uint32_t tile, uint32_t* s_dyn,
                                               uint16_t (*s_whist)[256], uint32_t* s_global_start, uint32_t* s_warp) {
   uint32_t* s_k = s_dyn;
   uint32_t* s_p0 = s_dyn + kTile;
@@ -367,16 +399,25 @@ __device__ __forceinline__ void onesweep_tile(const PassArgs<S>& a, uint32_t til
 }
 
 template <bool HAS_P1, int NB, class S>
-__global__ void __launch_bounds__(kSortThreads, HAS_P1 ? 4 : 5) onesweep_kernel(PassArgs<S> a) {
+__global__ void __launch_bounds__(kSortThreads, HAS_P1 ? 4 : 5) onesweep_kernel(const PassArgs<S> pa) {
   __shared__ uint32_t s_tile;
   __shared__ uint16_t s_whist[kWarps][256];
   __shared__ uint32_t s_global_start[256];
   __shared__ uint32_t s_warp[kWarps];
   extern __shared__ uint32_t s_dyn[];  // kTile keys, kTile payload0 [, kTile payload1]
-  if (threadIdx.x == 0) s_tile = atomicAdd(a.tile_ctr, 1u);
+  const PassPlan plan = *pa.plan;
+  if (!plan.active) return;
+  if (threadIdx.x == 0) s_tile = atomicAdd(pa.tile_ctr, 1u);
   for (int i = threadIdx.x; i < kWarps * 128; i += kSortThreads) reinterpret_cast<uint32_t*>(s_whist)[i] = 0;
   __syncthreads();
   const uint32_t tile = s_tile;
+  // src is 0, 1 or 2; dst 1 or 2
+  const auto from = [&](uint32_t* const* b) { return plan.src == 0 ? b[0] : (plan.src == 1 ? b[1] : b[2]); };
+  const auto to = [&](uint32_t* const* b) { return plan.dst == 1 ? b[1] : b[2]; };
+  const TileArgs<S> a = {from(pa.k), from(pa.p0), HAS_P1 ? from(pa.p1) : nullptr,
+                         to(pa.k),   to(pa.p0),   HAS_P1 ? to(pa.p1) : nullptr,
+                         pa.n,       pa.shift,    pa.mask,
+                         pa.digit_base, pa.status, pa.err};
   if (((uint64_t)tile + 1) * kTile <= a.n)
     onesweep_tile<HAS_P1, NB, S, true>(a, tile, s_dyn, s_whist, s_global_start, s_warp);
   else
@@ -399,28 +440,10 @@ static int launch_pass_of(const PassArgs<S>& a, cudaStream_t stream) {
 // seven ballots instead of eight when the digit has at most seven bits.
 template <class S>
 static int launch_pass(const PassArgs<S>& a, cudaStream_t stream) {
-  const bool p1 = a.p1in != nullptr, narrow = a.mask < 128;
+  const bool p1 = a.p1[0] != nullptr, narrow = a.mask < 128;
   if (p1) return narrow ? launch_pass_of<true, 7>(a, stream) : launch_pass_of<true, 8>(a, stream);
   return narrow ? launch_pass_of<false, 7>(a, stream) : launch_pass_of<false, 8>(a, stream);
 }
-
-struct PinnedCounts {
-  uint32_t* h = nullptr;  // 8*256 counts + kCtrWords counters
-  PinnedCounts() {
-    if (cudaMallocHost(&h, (8 * 256 + kCtrWords) * sizeof(uint32_t)) != cudaSuccess) h = nullptr;
-  }
-};
-
-PinnedCounts& pinned_counts() {
-  static thread_local PinnedCounts pc;
-  return pc;
-}
-
-struct PassPlan {
-  int role;  // 0: key = primary (k), payloads (v0, v1); 1: key = secondary (v0), payloads (k, v1)
-  uint32_t shift, mask;
-  int hist_index;  // which 256-bucket histogram holds the digit counts
-};
 
 }  // namespace
 
@@ -457,63 +480,48 @@ static int sort_impl(const KV& in, const KV& out, uint64_t n, bool lex, uint32_t
   const int grid = sm_count() * 4;
   // hist[0..3]: primary key digits; hist[4..7]: secondary key digits (lex).
   const DigitLayout lay = digit_layout(key_bits);
-  digit_hist_kernel<<<grid, 256, 0, stream>>>(in.k, n, lay.ndig, lay, d_hist, d_ctr + kCtrOr0);
-  if (lex)
-    digit_hist_kernel<<<grid, 256, 0, stream>>>(in.v0, n, lay.ndig, lay, d_hist + 4 * 256, d_ctr + kCtrOr0 + 1);
-  OGB_CUDA(cudaGetLastError());
-  digit_scan_kernel<<<lex ? 8 : 4, 256, 0, stream>>>(d_hist, d_base);
+  digit_hist_kernel<<<grid, 256, 0, stream>>>(in.k, n, lay.ndig, lay, d_hist);
+  if (lex) digit_hist_kernel<<<grid, 256, 0, stream>>>(in.v0, n, lay.ndig, lay, d_hist + 4 * 256);
   OGB_CUDA(cudaGetLastError());
 
-  PinnedCounts& pc = pinned_counts();
-  if (!pc.h) return fail(ERR_NOMEM, "cudaMallocHost for sort counts failed");
-  OGB_CUDA(cudaMemcpyAsync(pc.h, d_hist, 8 * 256 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-  OGB_CUDA(cudaStreamSynchronize(stream));
-
-  // LSD order: secondary digits first (lex), then primary digits.
-  std::vector<PassPlan> plan;
-  auto add_passes = [&](int role, int hbase) {
-    for (int d = 0; d < lay.ndig; d++) {
-      const uint32_t* h = pc.h + (hbase + d) * 256;
-      bool trivial = false;
-      for (int b = 0; b < 256; b++)
-        if (h[b] == n) trivial = true;
-      if (!trivial) plan.push_back({role, lay.shift[d], lay.mask[d], hbase + d});
-    }
+  // LSD order: secondary digits first (lex), then primary digits.  role 0: key =
+  // primary (k), payloads (v0, v1); 1: key = secondary (v0), payloads (k, v1)
+  struct Pass {
+    int role, digit, hist;
   };
-  if (lex) add_passes(1, 4);
-  add_passes(0, 0);
+  Pass passes[kMaxPasses];
+  int P = 0;
+  if (lex)
+    for (int d = 0; d < lay.ndig; d++) passes[P++] = {1, d, 4 + d};
+  for (int d = 0; d < lay.ndig; d++) passes[P++] = {0, d, d};
+  PassPlan* d_plan = reinterpret_cast<PassPlan*>(d_ctr + kCtrPlan);
+  PlanHists hists = {};
+  for (int i = 0; i < P; i++) hists.h[i] = passes[i].hist;
+  plan_kernel<<<1, 256, 0, stream>>>(d_hist, d_base, (uint32_t)n, hists, P, d_plan);
+  OGB_CUDA(cudaGetLastError());
 
-  const int P = (int)plan.size();
-  if (P == 0) {
-    OGB_CUDA(cudaMemcpyAsync(out.k, in.k, n * 4, cudaMemcpyDeviceToDevice, stream));
-    OGB_CUDA(cudaMemcpyAsync(out.v0, in.v0, n * 4, cudaMemcpyDeviceToDevice, stream));
-    if (has_p1) OGB_CUDA(cudaMemcpyAsync(out.v1, in.v1, n * 4, cudaMemcpyDeviceToDevice, stream));
-    return OK;
-  }
   const uint64_t tiles = (n + kTile - 1) / kTile;
   const size_t word = status_word_bytes(n);
   OGB_CUDA(cudaMemsetAsync(ws.status.p, 0, (size_t)P * tiles * 256 * word, stream));
 
-  KV tmp{ws.tmp_k.as<uint32_t>(), ws.tmp_v0.as<uint32_t>(), has_p1 ? ws.tmp_v1.as<uint32_t>() : nullptr};
-  KV cur = in;
+  const KV tmp{ws.tmp_k.as<uint32_t>(), ws.tmp_v0.as<uint32_t>(), has_p1 ? ws.tmp_v1.as<uint32_t>() : nullptr};
+  const KV* bufs[3] = {&in, &tmp, &out};
   for (int i = 0; i < P; i++) {
-    const KV dst = ((P - 1 - i) % 2 == 0) ? out : tmp;
-    const PassPlan& pp = plan[i];
     char* st = ws.status.as<char>() + (uint64_t)i * tiles * 256 * word;
     const auto fill = [&](auto& a) {
-      a.kin = pp.role == 0 ? cur.k : cur.v0;
-      a.p0in = pp.role == 0 ? cur.v0 : cur.k;
-      a.p1in = has_p1 ? cur.v1 : nullptr;
-      a.kout = pp.role == 0 ? dst.k : dst.v0;
-      a.p0out = pp.role == 0 ? dst.v0 : dst.k;
-      a.p1out = has_p1 ? dst.v1 : nullptr;
+      for (int b = 0; b < 3; b++) {
+        a.k[b] = passes[i].role == 0 ? bufs[b]->k : bufs[b]->v0;
+        a.p0[b] = passes[i].role == 0 ? bufs[b]->v0 : bufs[b]->k;
+        a.p1[b] = has_p1 ? bufs[b]->v1 : nullptr;
+      }
       a.n = (uint32_t)n;
-      a.shift = pp.shift;
-      a.mask = pp.mask;
-      a.digit_base = d_base + pp.hist_index * 256;
+      a.shift = lay.shift[passes[i].digit];
+      a.mask = lay.mask[passes[i].digit];
+      a.digit_base = d_base + passes[i].hist * 256;
       a.status = reinterpret_cast<decltype(a.status)>(st);
       a.tile_ctr = d_ctr + i;
-      a.err = d_ctr + kCtrErr;
+      a.err = ws.err ? ws.err : d_ctr + kCtrErr;
+      a.plan = d_plan + i;
     };
     if (word == sizeof(uint32_t)) {
       PassArgs<uint32_t> a;
@@ -524,7 +532,6 @@ static int sort_impl(const KV& in, const KV& out, uint64_t n, bool lex, uint32_t
       fill(a);
       OGB_TRY(launch_pass(a, stream));
     }
-    cur = dst;
   }
   return OK;
 }
@@ -538,7 +545,7 @@ int sort_pairs_lex(const KV& in, const KV& out, uint64_t n, SortWorkspace& ws, c
   return sort_impl(in, out, n, true, key_bits, ws, stream);
 }
 
-// Reads the error word of the last sorts on `stream` (synchronizes).
+// Reads the error word of the last sort with this workspace (synchronizes).
 int sort_check(SortWorkspace& ws, cudaStream_t stream) {
   if (!ws.counters.p) return OK;
   uint32_t e = 0;

@@ -15,8 +15,9 @@ struct KV {
 struct SortWorkspace {
   DevBuf hist;       // passes*256 u32 counts, then passes*256 exclusive bases
   DevBuf status;     // look-back words: passes * tiles * 256 of 4 bytes (8 from 2^30 keys on)
-  DevBuf counters;   // per-pass tile counters + error word
+  DevBuf counters;   // per-pass tile counters, error word, the passes' plan
   DevBuf tmp_k, tmp_v0, tmp_v1;  // one ping-pong array set
+  uint32_t* err = nullptr;       // where a pass reports an error (null: the counters' own word)
   int reserve(uint64_t n, bool weighted, int max_passes);
 };
 
@@ -24,8 +25,7 @@ struct SortWorkspace {
 // key must be below 2^key_bits (32: any key); the digits are ceil(key_bits /
 // 8) groups of nearly equal width from bit 0 up, and digit groups in which
 // every key has the same value are skipped.  `in` is not modified unless it
-// aliases `out`.  Runs on `stream`; one small device->host read (the digit
-// histograms) happens inside.
+// aliases `out`.  Runs on `stream` without waiting for it.
 int sort_pairs(const KV& in, const KV& out, uint64_t n, SortWorkspace& ws, cudaStream_t stream,
                uint32_t key_bits = 32);
 
