@@ -1355,9 +1355,24 @@ ResultStage& result_stage() {
 // costs link time of its own (16 equal chunks took 0.10 ms more than one
 // copy of 16.8 MB), and only the last chunk's copy-out is left after the
 // link is done.
+// A graph of at most kSmallResult vertices takes another way: a kernel writes
+// both arrays into the pinned stage, and one thread copies them out.  Its copies,
+// events and host threads cost more than the bytes (RMAT-14, 128 KB: 130 us).
 constexpr size_t kParentChunks = 4;  // <= ResultStage::kEv - 1
+constexpr uint32_t kSmallResult = 1u << 16;
 static int bfs_result_to_host(ogb_graph* dg, uint32_t V, uint32_t levels, int* parents, uint32_t* dist,
                               cudaStream_t s) {
+  if (V <= kSmallResult) {
+    ResultStage& rs = result_stage();
+    std::lock_guard<std::mutex> lk(rs.mu);
+    OGB_TRY(rs.reserve((size_t)V * 8));
+    int32_t* h = reinterpret_cast<int32_t*>(rs.h);
+    OGB_TRY(bfs_export(V, dg->d_parents.as<int32_t>(), dg->d_distances.as<uint32_t>(), h, s));
+    OGB_CUDA(cudaStreamSynchronize(s));
+    memcpy(parents, h, (size_t)V * 4);
+    memcpy(dist, h + V, (size_t)V * 4);
+    return OK;
+  }
   if (levels >= 255) {  // depths do not fit a byte: plain copies
     OGB_TRY(d2h(parents, dg->d_parents.p, (size_t)V * 4, s));
     OGB_TRY(d2h(dist, dg->d_distances.p, (size_t)V * 4, s));

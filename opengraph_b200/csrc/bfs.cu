@@ -2136,6 +2136,23 @@ __global__ void __launch_bounds__(256) bfsk_depth_bytes(uint32_t V, const uint32
   }
 }
 
+// A small search's result, written by the device into pinned host memory
+// (parents, then depths; V 4-byte values each).
+__global__ void __launch_bounds__(256) bfsk_export(uint32_t V, const int32_t* __restrict__ parents,
+                                                   const uint32_t* __restrict__ distances, int32_t* __restrict__ out) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    out[v] = parents[v];
+    out[V + v] = (int32_t)distances[v];
+  }
+}
+
+int bfs_export(uint32_t V, const int32_t* parents, const uint32_t* distances, int32_t* pinned, cudaStream_t s) {
+  bfsk_export<<<std::max<uint32_t>(1, std::min<uint32_t>(sm_count() * 2, ceil_div(V, 256))), 256, 0, s>>>(
+      V, parents, distances, pinned);
+  OGB_CUDA(cudaGetLastError());
+  return OK;
+}
+
 int bfs_depth_bytes(uint32_t V, const uint32_t* distances, uint8_t* out, cudaStream_t s) {
   const uint32_t n4 = (V + 3) / 4;
   const int grid = (int)std::min<uint32_t>(sm_count() * 8, std::max<uint32_t>(1, (n4 + 255) / 256));

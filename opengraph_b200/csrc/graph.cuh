@@ -219,6 +219,9 @@ int ppr_run(DevGraph& g, const uint32_t* seeds, uint32_t nseeds, uint32_t max_it
 // Depths as bytes (out: V bytes, rounded up to a multiple of 4), for the host
 // copy of a search of fewer than 255 levels.  bfs.cu.
 int bfs_depth_bytes(uint32_t V, const uint32_t* distances, uint8_t* out, cudaStream_t s);
+// Parents and depths (V values each, one after the other) into pinned host
+// memory by a kernel.  bfs.cu.
+int bfs_export(uint32_t V, const int32_t* parents, const uint32_t* distances, int32_t* pinned, cudaStream_t s);
 
 }  // namespace ogb
 
