@@ -1958,20 +1958,23 @@ __global__ void __cluster_dims__(kNarC, 1, 1) __launch_bounds__(kNarT, 1) bfsk_n
   uint32_t* qv = s_q;                                             // [2][kNarQ] vertices
   uint32_t* qs = s_q + 2 * kNarQ;                                 // [2][kNarQ] first out-edges
   uint16_t* qd = reinterpret_cast<uint16_t*>(s_q + 4 * kNarQ);    // [2][kNarQ] out-degrees (65535: that or more)
-  __shared__ BfsCtrl S;
+  __shared__ BfsCtrl S;         // what the other threads need of the state; the whole of it is in thread 0's registers
+  __shared__ BfsLevel s_level;  // the step just finished, for the trace
   __shared__ NarCount cnt[2];
   __shared__ uint32_t s_pre[kNarC + 1], s_stay;
-  __shared__ unsigned long long s_t0;
   const cg::cluster_group cl = cg::this_cluster();
   const uint32_t rank = cl.block_rank(), tid = threadIdx.x, lane = lane_id();
+  BfsCtrl c;
   if (tid == 0) {
-    S = st->c;
+    c = st->c;
+    S = c;
     cnt[0] = NarCount{};
     cnt[1] = NarCount{};
   }
   __syncthreads();
   int32_t* parents = st->parents;
   uint32_t* distances = st->distances;
+  unsigned long long t0 = 0;  // start of the step in progress (the thread that writes the trace)
   // the list as the grid-wide kernel left it, dealt out over the CTAs
   {
     const uint32_t* list = b.list[S.par_l];
@@ -1987,6 +1990,7 @@ __global__ void __cluster_dims__(kNarC, 1, 1) __launch_bounds__(kNarT, 1) bfsk_n
   }
   cl.sync();
   bool first = true;
+  uint32_t steps = 0;
   for (uint32_t par = 0;; par ^= 1u) {
     if (tid < 32) {
       // every CTA's totals: the queues' prefix, and the last step's counters
@@ -2011,52 +2015,79 @@ __global__ void __cluster_dims__(kNarC, 1, 1) __launch_bounds__(kNarT, 1) bfsk_n
           k.lnext = n;
           k.maxdeg = mx;
           k.fedges = fed;
-          ctrl_finish_td(S, (uint32_t)S.fedges, k, st, rank == 0, s_t0);
+          const uint32_t total = (uint32_t)c.fedges, frontier = c.frontier;
+          ctrl_finish_td(c, total, k, st, false, 0);
+          s_level = BfsLevel{0u, found, frontier, c.mf, c.mu, total, 0.f};
+          S.qcount = c.qcount;
+          S.qcount_prev = c.qcount_prev;
+          S.fedges = c.fedges;
+          S.edges_visited = c.edges_visited;
+          S.processed = c.processed;
+          S.nlevels = c.nlevels;
+          S.depth = c.depth;
         }
-        s_stay = narrow_fits(S) && td_next(S) && ctrl_decide(S, false) == kActTD;
-        s_t0 = global_ns();
+        s_stay = narrow_fits(c) && td_next(c) && ctrl_decide(c, false) == kActTD;
         cnt[par ^ 1u] = NarCount{};  // its readers are a barrier behind
       }
     }
-    first = false;
     __syncthreads();
+    if (rank == 0 && tid == 32) {
+      // the trace, off the step's path: the finished step, and the inputs of the next
+      const unsigned long long now = global_ns();
+      if (!first && S.nlevels - 1 < (uint32_t)kMaxTrace) {
+        BfsLevel L = s_level;
+        L.ms = (float)((double)(now - t0) * 1e-6);
+        st->steps[S.nlevels - 1].level = L;
+      }
+      t0 = now;
+      if (s_stay && S.nlevels < (uint32_t)kMaxTrace) {
+        float f[kFeat];
+        bfs_features(S, b.E, f);
+        for (int i = 0; i < kFeat; i++) st->steps[S.nlevels].feat[i] = f[i];
+      }
+    }
+    first = false;
     if (!s_stay) {
       // every CTA must have read the others' totals before one leaves
       cl.sync();
-      uint32_t* list = b.list[S.par_l];
+      uint32_t* list = b.list[(S.par_l + steps) & 1u];  // a step swaps the two lists
       const uint32_t n = s_pre[rank + 1] - s_pre[rank];
-      for (uint32_t i = tid; i < n; i += kNarT) list[s_pre[rank] + i] = qv[par * kNarQ + i];
+      for (uint32_t i = tid; i < n; i += kNarT) {
+        const uint32_t v = qv[par * kNarQ + i];
+        list[s_pre[rank] + i] = v;
+        distances[v] = S.depth;
+      }
       if (rank == 0 && tid == 0) {
-        S.more = kMoreWide;
-        S.narrow = 0;
-        S.rebuild = 1;
-        st->c = S;
+        c.more = kMoreWide;
+        c.narrow = 0;
+        c.rebuild = 1;
+        st->c = c;
       }
       return;
     }
-    if (rank == 0 && tid == 32 && S.nlevels < (uint32_t)kMaxTrace) {
-      float f[kFeat];
-      bfs_features(S, b.E, f);
-      for (int i = 0; i < kFeat; i++) st->steps[S.nlevels].feat[i] = f[i];
-    }
+    steps++;
     const uint32_t n = s_pre[kNarC], per = (n + kNarC - 1) / kNarC;
     const uint32_t lo = min(n, rank * per), hi = min(n, lo + per);
     const uint32_t dnext = S.depth + 1;
     const uint32_t to = (par ^ 1u) * kNarQ;
     uint32_t found = 0, mf = 0, fed = 0, mx = 0;
     for (uint32_t i = lo + tid / 4; i < hi; i += kNarT / 4) {
-      uint32_t o = 0;
-      while (i >= s_pre[o + 1]) o++;
+      uint32_t o = 0;  // the CTA whose queue holds entry i
+#pragma unroll
+      for (int k = 1; k < kNarC; k++) o += i >= s_pre[k] ? 1u : 0u;
       const uint32_t at = par * kNarQ + (i - s_pre[o]);
       const uint32_t src = *cl.map_shared_rank(&qv[at], o);
       const uint32_t row = *cl.map_shared_rank(&qs[at], o);
       const uint32_t deg = *cl.map_shared_rank(&qd[at], o);
+      if ((tid & 3) == 0) distances[src] = dnext - 1;  // see below
       for (uint32_t j = tid & 3; j < deg; j += 4) {
         const uint32_t u = __ldg(&b.nbr_f[row + j]) & 0x3FFFFFFFu;
         const int32_t p = __ldcg(&parents[u]);
         const uint2 r = __ldg(&b.rows_f[u]);
         if (p < 0 && atomicCAS(&parents[u], p, (int32_t)src) == p) {
-          distances[u] = dnext;
+          // a listed vertex gets its depth when it is expanded (or the run ends):
+          // a store here would be the last thing the step's barrier waits for
+          if (!r.y) distances[u] = dnext;
           found++;
           mf += (uint32_t)(-p);
           fed += r.y;
