@@ -54,12 +54,20 @@ constexpr int kPrThreads = 256;      // push kernels
 constexpr int kPullThreads = 1024;   // pull: one CTA per SM
 constexpr int kPullGroup = 256;      // threads per chunk group (the oracle's cta_threads)
 constexpr int kPullGroups = kPullThreads / kPullGroup;
-constexpr uint32_t kStage = 256;     // staged edges per warp and window
+// Staged edges per warp and window, by the kernel's variant: a small graph's
+// iteration is as long as its longest chain of windows (RMAT-16: 16 -> 14.5 us an
+// iteration with 512, and eight instead of four gathers in flight per thread of a
+// chunk), a large one needs the shared memory as L1 (RMAT-22 is 1 % slower with
+// either).
+template <int R>
+constexpr uint32_t kStageOf = R == 1 ? 512 : 256;
 constexpr uint32_t kUnitMax = 4096;  // medium-row edges per warp unit: between these, by
 constexpr uint32_t kUnitMin = 256;   // the graph's size (pr_unit_edges)
 constexpr uint32_t kTab = 64;        // medium rows per table batch
-constexpr uint32_t kWarpSmemWords = kStage + 3 * kTab + 1;  // stage + table of one warp
-constexpr size_t kPullDynSmem = (size_t)(kPullThreads / 32) * kWarpSmemWords * 4;
+template <int R>
+constexpr uint32_t kWarpSmemWords = kStageOf<R> + 3 * kTab + 1;  // stage + table of one warp
+template <int R>
+constexpr size_t kPullDynSmem = (size_t)(kPullThreads / 32) * kWarpSmemWords<R> * 4;
 constexpr uint32_t kPrChunk = 8192;  // edges per chunk of a very heavy row
 constexpr uint32_t kPushHubDeg = 256;  // push: destinations with more in-edges are hubs
 constexpr uint32_t kHubChunk = 1024;   // push: in-edges of a hub summed by one warp
@@ -235,20 +243,20 @@ __device__ __forceinline__ void pr_block_finish(double err, uint32_t active, PrC
 }
 
 // s += c[nbr[j]] for j = j0, j0+STRIDE, ... < j1, in that order; each step
-// issues four predicated neighbour loads, then their four gathers.
-template <uint32_t STRIDE>
+// issues K predicated neighbour loads, then their K gathers.
+template <uint32_t STRIDE, int K>
 __device__ __forceinline__ float strided_sum(const float* __restrict__ c, const uint32_t* __restrict__ nbr,
                                              uint32_t j0, uint32_t j1) {
   float s = 0.0f;
-  for (uint32_t j = j0; j < j1; j += 4 * STRIDE) {
-    uint32_t x[4];
+  for (uint32_t j = j0; j < j1; j += K * STRIDE) {
+    uint32_t x[K];
 #pragma unroll
-    for (int k = 0; k < 4; k++) x[k] = (j + k * STRIDE < j1) ? __ldg(&nbr[j + k * STRIDE]) : 0u;
-    float cx[4];
+    for (int k = 0; k < K; k++) x[k] = (j + k * STRIDE < j1) ? __ldg(&nbr[j + k * STRIDE]) : 0u;
+    float cx[K];
 #pragma unroll
-    for (int k = 0; k < 4; k++) cx[k] = (j + k * STRIDE < j1) ? __ldg(&c[x[k]]) : 0.0f;
+    for (int k = 0; k < K; k++) cx[k] = (j + k * STRIDE < j1) ? __ldg(&c[x[k]]) : 0.0f;
 #pragma unroll
-    for (int k = 0; k < 4; k++)
+    for (int k = 0; k < K; k++)
       if (j + k * STRIDE < j1) s = __fadd_rn(s, cx[k]);
   }
   return s;
@@ -301,6 +309,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // contribs of a window are copied straight into the warp's stage by
 // asynchronous 4-byte copies (kStage / 32 per lane in flight, no registers
 // held for them), and the neighbour ids of the next window load meanwhile.
+template <uint32_t kStage>
 struct StagePipe {
   uint32_t u[kStage / 32];
   __device__ __forceinline__ void load(const uint32_t* __restrict__ nbr, uint32_t w0, uint32_t e1, uint32_t lane) {
@@ -358,6 +367,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
     const float* __restrict__ contrib, float* __restrict__ contrib_next, float* __restrict__ pr, PrParams p,
     PrCtl* __restrict__ ctl, uint32_t it) {
   extern __shared__ uint32_t s_dyn[];  // per warp: stage and medium-row table
+  constexpr uint32_t kStage = kStageOf<R>;
   __shared__ float s_part[kPullGroups][kPullGroup / 32];
   __shared__ uint32_t s_last[kPullGroups];
   wait_for_prior_kernel();
@@ -373,7 +383,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
     const uint32_t grp = threadIdx.x / kPullGroup, gt = threadIdx.x % kPullGroup;
     for (uint32_t g = (kPullGroups - 1 - grp) * gridDim.x + blockIdx.x; g < n_chunks; g += gridDim.x * kPullGroups) {
       const PrChunkItem ci = chunks[g];
-      float sum = strided_sum<kPullGroup>(contrib, nbr, ci.j0 + gt, ci.j1);
+      float sum = strided_sum<kPullGroup, R == 1 ? 8 : 4>(contrib, nbr, ci.j0 + gt, ci.j1);
       sum = warp_fold(sum);
       if (lane == 0) s_part[grp][gt >> 5] = sum;
       asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(kPullGroup) : "memory");
@@ -397,7 +407,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
     }
   }
 
-  uint32_t* mine = s_dyn + warp * kWarpSmemWords;
+  uint32_t* mine = s_dyn + warp * kWarpSmemWords<R>;
   float* stage = reinterpret_cast<float*>(mine);
 
   // (2) medium rows, a warp per unit, rows taken in batches of kTab
@@ -419,7 +429,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
       const uint32_t e0 = toff[0], e1 = toff[nr];
       uint32_t r = 0;
       float s = 0.0f;
-      StagePipe pipe;
+      StagePipe<kStage> pipe;
       pipe.load(nbr, e0, e1, lane);
       for (uint32_t w0 = e0; w0 < e1; w0 += kStage) {
         const uint32_t w1 = min(w0 + kStage, e1);
@@ -473,7 +483,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
       }
     }
     const uint32_t seg0 = off_light[base], seg1 = off_light[vend];
-    StagePipe pipe;
+    StagePipe<kStage> pipe;
     pipe.load(nbr, seg0, seg1, lane);
     for (uint32_t w0 = seg0; w0 < seg1; w0 += kStage) {
       const uint32_t w1 = min(w0 + kStage, seg1);
@@ -1037,8 +1047,8 @@ template <int R>
 static int pr_pull_attrs_of(int optin_sm) {
   cudaFuncAttributes fa;
   OGB_CUDA(cudaFuncGetAttributes(&fa, pr_pull_kernel<R>));
-  OGB_CUDA(cudaFuncSetAttribute(pr_pull_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPullDynSmem));
-  const int pct = (int)std::min<size_t>(100, ((kPullDynSmem + fa.sharedSizeBytes + 2048) * 100 + optin_sm - 1) / optin_sm);
+  OGB_CUDA(cudaFuncSetAttribute(pr_pull_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPullDynSmem<R>));
+  const int pct = (int)std::min<size_t>(100, ((kPullDynSmem<R> + fa.sharedSizeBytes + 2048) * 100 + optin_sm - 1) / optin_sm);
   OGB_CUDA(cudaFuncSetAttribute(pr_pull_kernel<R>, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
   return OK;
 }
@@ -1195,9 +1205,10 @@ static int pr_work_get(DevGraph& g, bool pull, PrWork** out, cudaStream_t s) {
 // Not between the kernels of a push iteration, which became 8 us longer.
 static cudaError_t pr_launch_pull(DevGraph& g, PrWork* w, const float* c_cur, float* c_nxt, float* ranks,
                                   const PrParams& p, uint32_t it, bool dependent, cudaStream_t s) {
-  const auto kernel = pr_wide_light(p.V) ? pr_pull_kernel<4> : pr_pull_kernel<1>;
+  const bool wide = pr_wide_light(p.V);
+  const auto kernel = wide ? pr_pull_kernel<4> : pr_pull_kernel<1>;
   return launch_kernel(
-      kernel, dependent, sm_count(), kPullThreads, kPullDynSmem, s,
+      kernel, dependent, sm_count(), kPullThreads, wide ? kPullDynSmem<4> : kPullDynSmem<1>, s,
       w->lay.as<PrLay>(), w->rl_chunks.as<PrChunkItem>(), w->rl_first.as<uint32_t>(), w->rl_count.as<uint32_t>(),
       w->rl_done.as<uint32_t>(), w->rl_partials.as<float>(), w->rows_rl.as<uint2>(), w->off_light.as<uint32_t>(),
       w->unit_first.as<uint32_t>(), w->med_off.as<uint32_t>(), w->med_v.as<uint32_t>(), w->nbr_rl.as<uint32_t>(),
