@@ -10,6 +10,7 @@
 #include "graph.cuh"
 
 #include <stdarg.h>
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
@@ -110,6 +111,15 @@ __global__ void __launch_bounds__(256) csr_boundary_kernel(const uint32_t* __res
   }
 }
 
+// The arrays the boundary kernel fills in part, cleared in one launch.
+__global__ void __launch_bounds__(256) csr_clear_kernel(uint32_t V, uint32_t* __restrict__ edges_idx,
+                                                        uint32_t* __restrict__ run_end) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    edges_idx[v] = 0;
+    run_end[v] = 0;
+  }
+}
+
 // out_degree = run_end - edges_idx (0 - 0 for vertices without edges),
 // mirrored into the other direction's in_degree; rows packed.
 __global__ void __launch_bounds__(256) csr_degree_kernel(uint32_t V, const uint32_t* __restrict__ edges_idx,
@@ -145,9 +155,8 @@ static int reserve_csr(DevCSR& c, uint32_t V, uint32_t E, bool weighted) {
 
 int csr_map(DevCSR& c, DevCSR& other, uint32_t V, uint32_t E, uint32_t* d_err, cudaStream_t s) {
   if (V == 0) return OK;
-  OGB_CUDA(cudaMemsetAsync(c.edges_idx.p, 0, (size_t)V * 4, s));
-  OGB_CUDA(cudaMemsetAsync(c.out_degree.p, 0, (size_t)V * 4, s));
   const int grid = sm_count() * 8;
+  csr_clear_kernel<<<std::min(grid, (int)ceil_div(V, 256)), 256, 0, s>>>(V, c.d_edges_idx(), c.d_out_degree());
   if (E) {
     csr_boundary_kernel<<<grid, 256, 0, s>>>(c.d_src(), E, V, c.d_edges_idx(), c.d_out_degree(), d_err);
     OGB_CUDA(cudaGetLastError());

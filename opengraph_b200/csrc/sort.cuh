@@ -13,9 +13,8 @@ struct KV {
 };
 
 struct SortWorkspace {
-  DevBuf hist;       // passes*256 u32 counts, then passes*256 exclusive bases
+  DevBuf hist;       // 8*256 u32 counts; per-pass tile counters, error word and the passes' plan; 8*256 bases
   DevBuf status;     // look-back words: passes * tiles * 256 of 4 bytes (8 from 2^30 keys on)
-  DevBuf counters;   // per-pass tile counters, error word, the passes' plan
   DevBuf tmp_k, tmp_v0, tmp_v1;  // one ping-pong array set
   uint32_t* err = nullptr;       // where a pass reports an error (null: the counters' own word)
   int reserve(uint64_t n, bool weighted, int max_passes);
