@@ -57,8 +57,8 @@ constexpr int kPullGroups = kPullThreads / kPullGroup;
 // Staged edges per warp and window, by the kernel's variant: a small graph's
 // iteration is as long as its longest chain of windows (RMAT-16: 16 -> 14.5 us an
 // iteration with 512, and eight instead of four gathers in flight per thread of a
-// chunk), a large one needs the shared memory as L1 (RMAT-22 is 1 % slower with
-// either).
+// chunk), a large one needs the shared memory as L1 (RMAT-22: 247 us with 256,
+// 265 with 384, 267 with 512).
 template <int R>
 constexpr uint32_t kStageOf = R == 1 ? 512 : 256;
 constexpr uint32_t kUnitMax = 4096;  // medium-row edges per warp unit: between these, by
@@ -1025,20 +1025,26 @@ static int pr_build_lists(DevGraph& g, PrWork* w, cudaStream_t s) {
   return OK;
 }
 
-// Edges of a medium unit: the graph's edges over two units per warp of the
+// Edges of a medium unit: the graph's edges over four units per warp of the
 // pull kernel, as a power of two between 256 (one window: a smaller unit would
 // be a partial one) and 4096.  A warp walks its unit alone, so with 4096 edges
 // throughout, RMAT-16 (1 M edges) had work for 150 of 4736 warps: 45 us an
-// iteration, 16 us at 256; RMAT-22 (67 M) has two units per warp at 4096.
+// iteration, 16 us at 256.  Two units per warp left a tail where most rows are
+// medium: 1.5 M vertices with 16 in-edges each 138 us, 124 with four; RMAT-21 135
+// and 125; RMAT-22 247 with either.
 static uint32_t pr_unit_edges(uint32_t E) {
-  const uint32_t want = E / (2 * (uint32_t)sm_count() * (kPullThreads / 32));
+  const uint32_t want = E / (4 * (uint32_t)sm_count() * (kPullThreads / 32));
   uint32_t u = kUnitMin;
   while (u < kUnitMax && u < want) u *= 2;
   return u;
 }
 
-// Light rows per lane: four (128 vertices per warp unit) when that still gives
-// every warp a unit, else one.
+// Light rows per lane: two (64 vertices per warp unit) when every warp still has
+// two such units, else one.  Four left a tail on graphs of a few units per warp
+// (RMAT-20 74 us an iteration, 67 with two; 1.65 M vertices with 26 in-edges each
+// 282 and 209; RMAT-22 253 and 247); one in this kernel's small-graph form takes
+// 282 at RMAT-22 and 73 at RMAT-20.  Below the line one is the faster: 400 K
+// vertices with 30 in-edges each 71 us, 80 with two.
 static bool pr_wide_light(uint32_t V) { return V >= 128u * (uint32_t)sm_count() * (kPullThreads / 32); }
 
 // Shared memory of the pull kernels; the rest of the SM's unified L1 / shared
@@ -1057,7 +1063,7 @@ static int pr_pull_attrs() {
   OGB_CUDA(cudaGetDevice(&dev));
   OGB_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
   OGB_TRY(pr_pull_attrs_of<1>(per_sm));
-  return pr_pull_attrs_of<4>(per_sm);
+  return pr_pull_attrs_of<2>(per_sm);
 }
 
 // Re-laid pull graph (once per graph, warp_thr and cta_thr): ids sorted by
@@ -1206,9 +1212,9 @@ static int pr_work_get(DevGraph& g, bool pull, PrWork** out, cudaStream_t s) {
 static cudaError_t pr_launch_pull(DevGraph& g, PrWork* w, const float* c_cur, float* c_nxt, float* ranks,
                                   const PrParams& p, uint32_t it, bool dependent, cudaStream_t s) {
   const bool wide = pr_wide_light(p.V);
-  const auto kernel = wide ? pr_pull_kernel<4> : pr_pull_kernel<1>;
+  const auto kernel = wide ? pr_pull_kernel<2> : pr_pull_kernel<1>;
   return launch_kernel(
-      kernel, dependent, sm_count(), kPullThreads, wide ? kPullDynSmem<4> : kPullDynSmem<1>, s,
+      kernel, dependent, sm_count(), kPullThreads, wide ? kPullDynSmem<2> : kPullDynSmem<1>, s,
       w->lay.as<PrLay>(), w->rl_chunks.as<PrChunkItem>(), w->rl_first.as<uint32_t>(), w->rl_count.as<uint32_t>(),
       w->rl_done.as<uint32_t>(), w->rl_partials.as<float>(), w->rows_rl.as<uint2>(), w->off_light.as<uint32_t>(),
       w->unit_first.as<uint32_t>(), w->med_off.as<uint32_t>(), w->med_v.as<uint32_t>(), w->nbr_rl.as<uint32_t>(),
