@@ -128,15 +128,6 @@ struct DdSlot {
 std::mutex g_dd_mu;
 std::vector<DdSlot> g_dd;
 
-// Self loops per vertex (counted once per graph build).
-__global__ void dd_self_kernel(uint32_t E, const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst,
-                               uint32_t* __restrict__ selfcnt) {
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < E; j += gridDim.x * blockDim.x) {
-    const uint32_t u = src[j] & 0x3FFFFFFFu;
-    if (u == (dst[j] & 0x3FFFFFFFu)) atomicAdd(&selfcnt[u], 1u);
-  }
-}
-
 // Chunk counts of the long out-rows, then the chunks {v, j0, j1} at their
 // scanned offsets.
 __global__ void dd_och_count_kernel(uint32_t V, const uint2* __restrict__ rows_f, uint32_t* __restrict__ nch) {
@@ -152,6 +143,53 @@ __global__ void dd_och_fill_kernel(uint32_t V, const uint2* __restrict__ rows_f,
     if (r.y <= kOutBig) continue;
     uint32_t k = off[v];
     for (uint32_t c = 0; c < r.y; c += kOutChunk, k++) och[k] = make_uint4(v, r.x + c, r.x + min(r.y, c + kOutChunk), 0u);
+  }
+}
+
+// Self loops per vertex (counted once per graph build), from the out-rows: a
+// graph copied from a host GraphCSR has no array of edge sources.  A warp takes 32
+// consecutive rows and reads their edges as one sequence, each lane finding its
+// edge's row by a search through shuffles; the rows longer than kOutBig come in
+// their chunks, a warp each.
+__global__ void __launch_bounds__(kT) dd_self_kernel(uint32_t V, const uint2* __restrict__ rows_f,
+                                                     const uint32_t* __restrict__ nbr_f,
+                                                     const uint4* __restrict__ och, uint32_t n_och,
+                                                     uint32_t* __restrict__ selfcnt) {
+  const uint32_t lane = lane_id();
+  const uint64_t gw = (uint64_t)blockIdx.x * (kT / 32) + (threadIdx.x >> 5), nw = (uint64_t)gridDim.x * (kT / 32);
+  for (uint64_t t = gw; t < n_och; t += nw) {
+    const uint4 c = och[t];
+    uint32_t n = 0;
+    for (uint32_t k = lane; k < c.z - c.y; k += 32) n += (__ldg(&nbr_f[c.y + k]) & 0x3FFFFFFFu) == c.x;
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0 && n) atomicAdd(&selfcnt[c.x], n);
+  }
+  for (uint64_t v0 = gw * 32; v0 < V; v0 += nw * 32) {
+    uint2 r = make_uint2(0u, 0u);
+    if (v0 + lane < V) r = rows_f[v0 + lane];
+    if (r.y > kOutBig) r.y = 0;
+    uint32_t ex = r.y;  // inclusive, then exclusive scan of the 32 lengths
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, ex, k);
+      if (lane >= (uint32_t)k) ex += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, ex, 31);
+    ex -= r.y;
+    for (uint32_t e0 = 0; e0 < total; e0 += 128) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t e = e0 + k * 32 + lane;
+        uint32_t p = 0;  // last row whose first edge is at or before e
+#pragma unroll
+        for (int step = 16; step; step >>= 1) {
+          const uint32_t first = __shfl_sync(0xffffffffu, ex, p + step);
+          if (first <= e) p += step;
+        }
+        const uint32_t from = __shfl_sync(0xffffffffu, r.x - ex, p) + e;
+        if (e < total && (__ldg(&nbr_f[from]) & 0x3FFFFFFFu) == (uint32_t)v0 + p) atomicAdd(&selfcnt[v0 + p], 1u);
+      }
+    }
   }
 }
 
@@ -777,7 +815,6 @@ int dd_work_get(DevGraph& g, DdWork** out, cudaStream_t s) {
   const int grid = sm_count() * 8;
   OGB_TRY(w->heavy.alloc(g.E));
   dd_fill_kernel<<<grid, kT, 0, s>>>(0, V, g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), ctl);
-  dd_self_kernel<<<grid, kT, 0, s>>>(g.E, g.fwd.d_src(), g.fwd.d_dst(), w->selfcnt.as<uint32_t>());
   OGB_CUDA(cudaGetLastError());
   DevBuf tmp;
   OGB_TRY(tmp.alloc(((size_t)V * 2 + 4 + scan_tmp_words(V)) * 4));
@@ -794,6 +831,9 @@ int dd_work_get(DevGraph& g, DdWork** out, cudaStream_t s) {
   dd_och_fill_kernel<<<grid, kT, 0, s>>>(V, g.fwd.d_rows(), off, w->och.as<uint4>());
   OGB_CUDA(cudaGetLastError());
   w->n_och = total;
+  dd_self_kernel<<<grid, kT, 0, s>>>(V, g.fwd.d_rows(), g.fwd.d_dst(), w->och.as<uint4>(), total,
+                                     w->selfcnt.as<uint32_t>());
+  OGB_CUDA(cudaGetLastError());
   OGB_CUDA(cudaMemcpyAsync(&ctl->n_och, &w->n_och, 4, cudaMemcpyHostToDevice, s));
   OGB_CUDA(cudaStreamSynchronize(s));  // the host copy source and tmp outlive the copies
   w->built = g.build_id;
