@@ -121,6 +121,7 @@ struct BfsCtrl {
   uint32_t ul_fresh;                 // 1: the unvisited list comes from the step just before (all unvisited)
   uint32_t lmax;                     // largest out-degree on the expansion list
   uint32_t narrow;                   // narrow lists made in a row by top-down steps
+  uint32_t streak;                   // narrow lists in a row that start the next run of narrow steps
   uint32_t more;                     // why the kernel ended: kMoreNone, kMoreNarrow or kMoreWide
   uint32_t rebuild;                  // 1: the bitmaps must be made from the list (after narrow steps)
   uint32_t phase;                    // counter set of the next phase (an index into ctl)
@@ -1471,12 +1472,19 @@ constexpr uint32_t kMoreNone = 0, kMoreNarrow = 1, kMoreWide = 2;
 
 // Narrow steps (bfsk_narrow).  A list is narrow when its entries have at most
 // kNarDeg out-edges and the discoveries of a CTA's share of it fit the CTA's
-// queue.  The grid-wide kernel hands over after kNarStreak narrow lists of at
-// most kNarEnter entries in a row, so that the two or three small steps at the
-// ends of a low-diameter search, which are followed by a large one or by the
-// end, stay where they are.
+// queue.  The grid-wide kernel hands over after `streak` narrow lists of at most
+// kNarEnter entries in a row, at first kNarStreak, so that the two or three small
+// steps at the ends of a low-diameter search, which are followed by a large one or
+// by the end, stay where they are.
+// A run and the way back (two launches, a wait of the host, the bitmaps remade)
+// cost 33 us, and a narrow step on a path is 3.9 us shorter than a wide one: a run
+// of fewer than kNarShort steps loses.  It doubles `streak`, and a run of
+// kNarLong steps, which has won back several lost ones, resets it.  (A path of
+// 2000 vertices with a hub of 33 leaves at every fifth: 25.4 ms with `streak`
+// left at 4, 12.8 ms with every step wide; at every eighth 16.9 and 12.9; at every
+// twentieth, runs of 16 steps, 9.8 and 12.8.)
 constexpr int kNarT = 1024, kNarC = 8;
-constexpr uint32_t kNarDeg = 32, kNarCap = 8192, kNarEnter = 2048, kNarStreak = 4;
+constexpr uint32_t kNarDeg = 32, kNarCap = 8192, kNarEnter = 2048, kNarStreak = 4, kNarShort = 9, kNarLong = 64;
 constexpr uint32_t kNarQ = 8192;  // queue entries per CTA
 __device__ __forceinline__ bool narrow_fits(const BfsCtrl& c) {
   return c.lmax <= kNarDeg && c.lsize <= kNarCap && (c.lsize + kNarC - 1) / kNarC * c.lmax <= kNarQ;
@@ -1487,7 +1495,7 @@ __device__ __forceinline__ bool td_next(const BfsCtrl& c) {
          (c.mode == BFS_PUSH || (c.mode == BFS_DO && c.mf <= c.mu / kAlpha));
 }
 __device__ __forceinline__ bool narrow_enter(const BfsCtrl& c) {
-  return c.narrow >= kNarStreak && c.lsize <= kNarEnter && narrow_fits(c) && td_next(c);
+  return c.narrow >= c.streak && c.lsize <= kNarEnter && narrow_fits(c) && td_next(c);
 }
 
 // Counters of a finished phase, read past any cached copy.
@@ -1714,6 +1722,7 @@ __global__ void __launch_bounds__(256) bfsk_init(BfsBufs b, BfsDevState* st, uin
     c.fedges = d;
     c.edges_visited = d;
     c.lmax = d;
+    c.streak = kNarStreak;
     // the first bottom-up step walks the cached list of vertices with
     // in-edges (a vertex without any can never be found bottom-up); the
     // dense-probe mode walks every vertex in every step
@@ -2060,6 +2069,10 @@ __global__ void __cluster_dims__(kNarC, 1, 1) __launch_bounds__(kNarT, 1) bfsk_n
       if (rank == 0 && tid == 0) {
         c.more = kMoreWide;
         c.narrow = 0;
+        if (steps < kNarShort)
+          c.streak *= 2;
+        else if (steps >= kNarLong)
+          c.streak = kNarStreak;
         c.rebuild = 1;
         st->c = c;
       }
@@ -2294,7 +2307,7 @@ int bfs_run_roots(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint32_t 
   const BfsDevState* h = w->h_state;
   uint32_t launches = 0;
   // the search kernel; when it ends at a run of narrow steps, that run and the
-  // search kernel again (each round takes at least kNarStreak steps)
+  // search kernel again (each round takes at least `streak` steps)
   for (;;) {
     OGB_CUDA(cudaLaunchCooperativeKernel((void*)bfsk_search, dim3(w->search_grid), dim3(kSearchT), args, 0, s));
     launches++;

@@ -1,0 +1,60 @@
+"""When a search hands its narrow steps to the cluster kernel: paths with hubs
+every few vertices, counted in launches (the search kernel once, and twice more
+per run).  Runs too short to pay must not be tried again and again, long ones must
+go on, and a long one lets short lists start a run again."""
+import numpy as np
+import pytest
+
+from test_bfs_gpu import check_parents
+from test_build_gpu import dev, host
+
+pytestmark = pytest.mark.gpu
+
+
+def hub_path(sections):
+    """A path; a section is (length, period, leaves): every period-th of its
+    vertices, its first among them, has that many leaves (period 0: none)."""
+    hubs, at = [], 0
+    for length, period, leaves in sections:
+        if period:
+            hubs += [(v, leaves) for v in range(at, at + length, period)]
+        at += length
+    ls = np.concatenate([np.full(k, v) for v, k in hubs] + [np.zeros(0, np.int64)]).astype(np.int64)
+    s = np.concatenate([np.arange(at - 1), ls])
+    d = np.concatenate([np.arange(1, at), at + np.arange(len(ls))])
+    V = at + len(ls)
+    perm = np.random.default_rng(3).permutation(V)
+    return perm[s].astype(np.uint32), perm[d].astype(np.uint32), V, int(perm[0])
+
+
+# a run starts after 4, then 8, ... narrow lists; a period of p vertices has p - 1
+CASES = {
+    "every5": ([(1000, 5, 33)], 3),               # a run of 1 step; 8 lists in a row never come
+    "every8": ([(1000, 8, 1000)], 3),             # 4 steps
+    "every12": ([(1200, 12, 33)], 5),             # 8 steps, then 4
+    "every13": ([(1300, 13, 100)], 1 + 2 * 100),  # 9 steps: as good either way, and it stays
+    "every100": ([(1000, 100, 40)], 1 + 2 * 10),
+    "none": ([(600, 0, 0)], 3),
+    "reset": ([(500, 5, 33), (500, 0, 0), (500, 5, 33)], 1 + 2 * 3),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_launches(torch_cuda, lib, oracle, name):
+    torch = torch_cuda
+    sections, launches = CASES[name]
+    s, d, V, root = hub_path(sections)
+    g = oracle.build(s, d, V, 0)
+    dg = lib.device_graph()
+    dg.build(dev(torch, s), dev(torch, d), V, 0)
+    par_t = torch.empty(V, dtype=torch.int32, device="cuda")
+    dist_t = torch.empty(V, dtype=torch.int32, device="cuda")
+    for _ in range(2):  # the second search starts anew
+        info = dg.bfs(root, par_t, dist_t, mode=1)
+        _, edist, est = oracle.bfs(g, root, 1)
+        assert np.array_equal(host(dist_t), edist)
+        for k in ("iteration", "processed_nodes", "td_steps", "reached", "reached_out_edges"):
+            assert info[k] == est[k], k
+        check_parents(g, root, host(par_t, np.int32), host(dist_t))
+        assert info["launches"] == launches
+    dg.close()
