@@ -250,6 +250,7 @@ _DEVICE_API = [
     ("ogb_dropin_bfs_phases", C.c_int, [C.POINTER(C.c_double), u32]),
     ("ogb_graph_create", C.c_int, [C.POINTER(vp)]),
     ("ogb_graph_destroy", None, [vp]),
+    ("ogb_graph_test_option", C.c_int, [vp, u32, u32]),
     ("ogb_graph_build", C.c_int, [vp, vp, vp, vp, u32, u32, u32, vp]),
     ("ogb_graph_view", C.c_int, [vp, C.c_int, C.POINTER(CsrView)]),
     ("ogb_graph_of", vp, [vp]),

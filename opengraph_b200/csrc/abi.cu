@@ -1929,6 +1929,13 @@ extern "C" int ogb_graph_create(ogb_graph** g) {
 }
 
 extern "C" void ogb_graph_destroy(ogb_graph* g) { delete g; }
+extern "C" int ogb_graph_test_option(ogb_graph* g, uint32_t option, uint32_t value) {
+  if (!g) return fail(ERR_ARG, "null");
+  switch (option) {
+    case OGB_TEST_SORT_GIVES_UP: g->g.sort_ws.give_up = value; return OK;
+  }
+  return fail(ERR_ARG, "test option %u", option);
+}
 
 // A null stream argument is the legacy default stream (as in the CUDA
 // libraries), so the call waits for the caller's default-stream work.

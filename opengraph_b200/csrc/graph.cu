@@ -186,7 +186,13 @@ int graph_build(DevGraph& g, const uint32_t* in_src, const uint32_t* in_dst, con
   OGB_TRY(reserve_csr(g.inv, V, E, weighted));
   OGB_TRY(g.err.alloc(16));
   OGB_CUDA(cudaMemsetAsync(g.err.p, 0, 16, s));
-  g.sort_ws.err = g.err.as<uint32_t>() + 1;  // read back with the build's own word
+  // the build's sorts report beside its own word, for one copy back; every other
+  // sort with this workspace in the workspace's word
+  struct Errors {
+    SortWorkspace& ws;
+    ~Errors() { ws.err = nullptr; }
+  } errors{g.sort_ws};
+  g.sort_ws.err = g.err.as<uint32_t>() + 1;
   const bool lex = (sort_type == 1 || sort_type == 3);
 
   // forward: sort by src (or by (src, dst))

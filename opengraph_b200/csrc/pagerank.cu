@@ -540,8 +540,13 @@ __global__ void pr_rl_keys_kernel(uint32_t V, const uint32_t* __restrict__ out_d
 }
 
 // perm[old id] = new id, from the sorted ids (new id -> old id).
-__global__ void pr_rl_perm_kernel(uint32_t V, const uint32_t* __restrict__ order, uint32_t* __restrict__ perm) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x) perm[order[i]] = i;
+// A sort that gave up has left slots of `order` unwritten: the ids then stay as
+// they are, which changes no result.
+__global__ void pr_rl_perm_kernel(uint32_t V, const uint32_t* __restrict__ order, const uint32_t* __restrict__ sort_err,
+                                  uint32_t* __restrict__ perm) {
+  const bool sorted = *sort_err == 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x)
+    perm[sorted ? order[i] : i] = i;
 }
 
 // The classes of all rows (light <= warp_thr < medium <= cta_thr < chunked) and
@@ -1119,7 +1124,7 @@ static int pr_build_relabel(DevGraph& g, PrWork* w, cudaStream_t s) {
   KV in{t0, t0 + Vp, nullptr};
   KV out{t0 + 2 * Vp, t0 + 3 * Vp, nullptr};
   OGB_TRY(sort_pairs(in, out, V, g.sort_ws, s, kRlKeyBits));
-  pr_rl_perm_kernel<<<grid, 256, 0, s>>>(V, out.v0, w->perm.as<uint32_t>());
+  pr_rl_perm_kernel<<<grid, 256, 0, s>>>(V, out.v0, sort_error_word(g.sort_ws), w->perm.as<uint32_t>());
   pr_lay_sums_kernel<<<ntiles, 256, 0, s>>>(V, rows, g_warp_thr, g_cta_thr, sums, ntiles);
   pr_lay_scan_kernel<<<1, 256, 0, s>>>(sums, ntiles, w->unit, lay);
   pr_lay_rows_kernel<<<ntiles, 256, 0, s>>>(V, rows, g_warp_thr, g_cta_thr, sums, ntiles, lay,

@@ -526,7 +526,7 @@ static int sort_impl(const KV& in, const KV& out, uint64_t n, bool lex, uint32_t
       a.digit_base = d_base + passes[i].hist * 256;
       a.status = reinterpret_cast<decltype(a.status)>(st);
       a.tile_ctr = d_ctr + i;
-      a.err = ws.err ? ws.err : d_ctr + kCtrErr;
+      a.err = const_cast<uint32_t*>(sort_error_word(ws));
       a.plan = d_plan + i;
     };
     if (word == sizeof(uint32_t)) {
@@ -539,7 +539,17 @@ static int sort_impl(const KV& in, const KV& out, uint64_t n, bool lex, uint32_t
       OGB_TRY(launch_pass(a, stream));
     }
   }
+  if (ws.give_up) {
+    static const uint32_t gave_up = ERR_SPIN;
+    ws.give_up--;
+    OGB_CUDA(cudaMemsetAsync(out.v0, 0xFF, n * 4, stream));
+    OGB_CUDA(cudaMemcpyAsync(const_cast<uint32_t*>(sort_error_word(ws)), &gave_up, 4, cudaMemcpyHostToDevice, stream));
+  }
   return OK;
+}
+
+const uint32_t* sort_error_word(const SortWorkspace& ws) {
+  return ws.err ? ws.err : ws.hist.as<uint32_t>() + 8 * 256 + kCtrErr;
 }
 
 int sort_pairs(const KV& in, const KV& out, uint64_t n, SortWorkspace& ws, cudaStream_t stream, uint32_t key_bits) {
@@ -555,7 +565,7 @@ int sort_pairs_lex(const KV& in, const KV& out, uint64_t n, SortWorkspace& ws, c
 int sort_check(SortWorkspace& ws, cudaStream_t stream) {
   if (!ws.hist.p) return OK;
   uint32_t e = 0;
-  OGB_CUDA(cudaMemcpyAsync(&e, ws.hist.as<uint32_t>() + 8 * 256 + kCtrErr, 4, cudaMemcpyDeviceToHost, stream));
+  OGB_CUDA(cudaMemcpyAsync(&e, sort_error_word(ws), 4, cudaMemcpyDeviceToHost, stream));
   OGB_CUDA(cudaStreamSynchronize(stream));
   if (e) return fail((int)e, "radix sort: decoupled look-back wait gave up");
   return OK;

@@ -17,6 +17,8 @@ struct SortWorkspace {
   DevBuf status;     // look-back words: passes * tiles * 256 of 4 bytes (8 from 2^30 keys on)
   DevBuf tmp_k, tmp_v0, tmp_v1;  // one ping-pong array set
   uint32_t* err = nullptr;       // where a pass reports an error (null: the counters' own word)
+  // set by tests only
+  uint32_t give_up = 0;               // the next so many sorts report that a look-back gave up, their first payload lost
   int reserve(uint64_t n, bool weighted, int max_passes);
 };
 
@@ -32,5 +34,9 @@ int sort_pairs(const KV& in, const KV& out, uint64_t n, SortWorkspace& ws, cudaS
 // and `in.v0` the secondary key (both below 2^key_bits); payload v1 follows.
 int sort_pairs_lex(const KV& in, const KV& out, uint64_t n, SortWorkspace& ws, cudaStream_t stream,
                    uint32_t key_bits = 32);
+
+// The word in which the last sort with ws reported an error (0: none), on the
+// device; valid until the next one.
+const uint32_t* sort_error_word(const SortWorkspace& ws);
 
 }  // namespace ogb
