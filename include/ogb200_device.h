@@ -103,8 +103,9 @@ int ogb_graph_create(ogb_graph **g);
 void ogb_graph_destroy(ogb_graph *g);
 /* For tests: makes one graph meet what a GPU will not do on request.
  * OGB_TEST_SORT_GIVES_UP: its next `value` sorts report that a bounded wait gave
- * up, their first payload lost. */
-enum { OGB_TEST_SORT_GIVES_UP = 1 };
+ * up, their first payload lost.  OGB_TEST_NO_CLUSTERS, before its first search:
+ * the device cannot launch thread-block clusters. */
+enum { OGB_TEST_SORT_GIVES_UP = 1, OGB_TEST_NO_CLUSTERS = 2 };
 int ogb_graph_test_option(ogb_graph *g, uint32_t option, uint32_t value);
 /* Sort (SORT_TYPE semantics) and build both CSR directions from device edge
  * arrays; all ids < V <= 2^30.  Inputs are read only.  d_w may be NULL. */

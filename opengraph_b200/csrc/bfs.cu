@@ -196,6 +196,7 @@ struct BfsWork {
   BfsDevState* h_state = nullptr;   // pinned copy of the first kStateCopy bytes
   uint32_t epoch = 0;               // last scan epoch used
   int search_grid = 0;          // CTAs of the search launch (co-resident)
+  int narrow = -1;              // 1: the device can hold bfsk_narrow's cluster (-1: not asked yet)
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
   ~BfsWork() {
     if (h_state) cudaFreeHost(h_state);
@@ -1485,6 +1486,7 @@ constexpr uint32_t kMoreNone = 0, kMoreNarrow = 1, kMoreWide = 2;
 // twentieth, runs of 16 steps, 9.8 and 12.8.)
 constexpr int kNarT = 1024, kNarC = 8;
 constexpr uint32_t kNarDeg = 32, kNarCap = 8192, kNarEnter = 2048, kNarStreak = 4, kNarShort = 9, kNarLong = 64;
+constexpr uint32_t kNarNever = 0xFFFFFFFFu;  // a streak that no search reaches (at most 2^30 + 8 steps)
 constexpr uint32_t kNarQ = 8192;  // queue entries per CTA
 __device__ __forceinline__ bool narrow_fits(const BfsCtrl& c) {
   return c.lmax <= kNarDeg && c.lsize <= kNarCap && (c.lsize + kNarC - 1) / kNarC * c.lmax <= kNarQ;
@@ -1690,7 +1692,7 @@ __device__ void ctrl_finish_bu(BfsCtrl& c, const BfsCtl& k, BfsDevState* st, boo
 // out_degree(root), queue = {root}).
 __global__ void __launch_bounds__(256) bfsk_init(BfsBufs b, BfsDevState* st, uint32_t root, int32_t* parents,
                                                  uint32_t* distances, uint32_t mode, uint32_t bu_entry_frontier,
-                                                 uint32_t E, uint32_t epoch, uint32_t n_cand0) {
+                                                 uint32_t E, uint32_t epoch, uint32_t n_cand0, uint32_t streak) {
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < b.V; v += stride) {
     const uint32_t d = b.out_degree[v];
@@ -1722,7 +1724,7 @@ __global__ void __launch_bounds__(256) bfsk_init(BfsBufs b, BfsDevState* st, uin
     c.fedges = d;
     c.edges_visited = d;
     c.lmax = d;
-    c.streak = kNarStreak;
+    c.streak = streak;
     // the first bottom-up step walks the cached list of vertices with
     // in-edges (a vertex without any can never be found bottom-up); the
     // dense-probe mode walks every vertex in every step
@@ -2265,6 +2267,24 @@ static int bfs_cand0(DevGraph& g, BfsWork* w, cudaStream_t s) {
   return OK;
 }
 
+// Whether the device can hold bfsk_narrow's cluster: eight CTAs of 160 KB within one
+// group of SMs, which fewer visible SMs may not have.  Without it every step
+// is a wide one.
+static int narrow_available(const DevGraph& g) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kNarC);
+  cfg.blockDim = dim3(kNarT);
+  cfg.dynamicSmemBytes = kNarSmem;
+  int clusters = 0;
+  if (g.test_no_clusters ||
+      cudaFuncSetAttribute(bfsk_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNarSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, bfsk_narrow, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return clusters > 0 ? 1 : 0;
+}
+
 int bfs_run(DevGraph& g, uint32_t root, uint32_t mode, int32_t* parents, uint32_t* distances, BfsResult* res,
             bool want_trace, bool bu_entry_nf_frontier, cudaStream_t s) {
   return bfs_run_roots(g, &root, 1, mode, parents, distances, res, want_trace, bu_entry_nf_frontier, s);
@@ -2288,6 +2308,7 @@ int bfs_run_roots(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint32_t 
     if (nb < 1) return fail(ERR_CUDA, "bfs: search kernel does not fit on an SM");
     w->search_grid = nb * sm_count();
   }
+  if (w->narrow < 0) w->narrow = narrow_available(g);
   OGB_TRY(bfs_cand0(g, w, s));
   BfsBufs b = make_bufs(g, w);  // after bfs_cand0: it (re)allocates the record buffers
   if (mode != BFS_LEARNED) {  // the network is read only by the learned switch
@@ -2295,7 +2316,7 @@ int bfs_run_roots(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint32_t 
     b.policy_tail = nullptr;
   }
   bfsk_init<<<sm_count() * 8, 256, 0, s>>>(b, st, root, parents, distances, mode, bu_entry_nf_frontier ? 1u : 0u,
-                                            g.E, w->epoch, w->n_cand0);
+                                            g.E, w->epoch, w->n_cand0, w->narrow ? kNarStreak : kNarNever);
   if (nroots > 1) {
     OGB_TRY(w->roots.alloc((size_t)nroots * 4));
     OGB_CUDA(cudaMemcpyAsync(w->roots.p, roots, (size_t)nroots * 4, cudaMemcpyHostToDevice, s));
@@ -2315,7 +2336,6 @@ int bfs_run_roots(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint32_t 
     OGB_CUDA(cudaMemcpyAsync(w->h_state, w->state.p, kStateCopy, cudaMemcpyDeviceToHost, s));
     OGB_CUDA(cudaStreamSynchronize(s));
     if (h->err || h->c.more != kMoreNarrow) break;
-    OGB_CUDA(cudaFuncSetAttribute(bfsk_narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNarSmem));
     bfsk_narrow<<<kNarC, kNarT, kNarSmem, s>>>(b, st);
     OGB_CUDA(cudaGetLastError());
     launches++;

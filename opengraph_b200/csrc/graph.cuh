@@ -54,6 +54,7 @@ struct DevGraph {
   DevBuf input_src, input_dst, input_w;  // staging of host uploads
   DevBuf err;                            // u32 error words of the build kernels: CSR map, sorts
   DevBuf range_q;                        // scratch of the partitioned BFS steps (bfs_range.cu)
+  bool test_no_clusters = false;         // set by tests only: as if no cluster could be launched
   uint32_t build_id = 0;  // bumped whenever the edges change (caches key on it)
   BfsWork* bfs = nullptr;
   PrWork* pr = nullptr;

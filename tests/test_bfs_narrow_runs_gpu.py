@@ -39,13 +39,20 @@ CASES = {
 }
 
 
+NO_CLUSTERS = 2  # test option of a graph: as on a device that cannot launch the cluster
+
+
+@pytest.mark.parametrize("clusters", [True, False])
 @pytest.mark.parametrize("name", list(CASES))
-def test_launches(torch_cuda, lib, oracle, name):
+def test_launches(torch_cuda, lib, oracle, name, clusters):
     torch = torch_cuda
     sections, launches = CASES[name]
     s, d, V, root = hub_path(sections)
     g = oracle.build(s, d, V, 0)
     dg = lib.device_graph()
+    if not clusters:
+        launches = 1
+        lib.check(lib.ogb_graph_test_option(dg.handle, NO_CLUSTERS, 1))
     dg.build(dev(torch, s), dev(torch, d), V, 0)
     par_t = torch.empty(V, dtype=torch.int32, device="cuda")
     dist_t = torch.empty(V, dtype=torch.int32, device="cuda")
