@@ -113,7 +113,7 @@ __global__ void msk_roots(const uint32_t* __restrict__ verts, const unsigned lon
 
 // Push of the edges of the frontier word f: four targets at once.
 __device__ __forceinline__ void ms_push4(const unsigned long long* f, const uint32_t* w, const bool* ok,
-                                         const unsigned long long* __restrict__ vis, unsigned long long* N) {
+                                         const unsigned long long* vis, unsigned long long* N) {
   unsigned long long m[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) m[k] = ok[k] ? f[k] & ~vis[w[k]] : 0ull;
@@ -131,9 +131,8 @@ __global__ void __launch_bounds__(256) msk_expand(uint32_t V, unsigned long long
                                                   const uint32_t* __restrict__ heavy, uint32_t n_heavy,
                                                   const uint2* __restrict__ rows_f, const uint32_t* __restrict__ nbr_f,
                                                   const uint2* __restrict__ rows_i, const uint32_t* __restrict__ nbr_i,
-                                                  const unsigned long long* __restrict__ F,
-                                                  const unsigned long long* __restrict__ vis, unsigned long long* N,
-                                                  const uint32_t* __restrict__ list, uint4* __restrict__ items,
+                                                  const unsigned long long* F, const unsigned long long* vis,
+                                                  unsigned long long* N, const uint32_t* list, uint4* items,
                                                   MsCtl* ctl) {
   wait_for_prior_kernel();
   let_next_kernel_start();
@@ -251,11 +250,9 @@ __global__ void __launch_bounds__(256) msk_expand(uint32_t V, unsigned long long
 }
 
 // push: the pieces of the long rows, a warp each
-__global__ void __launch_bounds__(256) msk_push_long(const uint4* __restrict__ items,
-                                                     const uint32_t* __restrict__ nbr_f,
-                                                     const unsigned long long* __restrict__ F,
-                                                     const unsigned long long* __restrict__ vis, unsigned long long* N,
-                                                     const MsCtl* __restrict__ ctl) {
+__global__ void __launch_bounds__(256) msk_push_long(const uint4* items, const uint32_t* __restrict__ nbr_f,
+                                                     const unsigned long long* F, const unsigned long long* vis,
+                                                     unsigned long long* N, const MsCtl* ctl) {
   wait_for_prior_kernel();
   let_next_kernel_start();
   if (ctl->done || ctl->pull) return;
@@ -284,11 +281,9 @@ __global__ void __launch_bounds__(256) msk_push_long(const uint4* __restrict__ i
 // whole warp writes its depths (lane l: depth lanes l and l + 32 of the
 // vertex's 128-byte row, 2-byte stores, no read -- every (vertex, lane) is
 // written once).  The last CTA makes the counted frontier the next level's.
-__global__ void __launch_bounds__(256) msk_finish(uint32_t V, uint32_t E, unsigned long long* __restrict__ F,
-                                                  unsigned long long* __restrict__ N,
-                                                  unsigned long long* __restrict__ vis,
-                                                  uint16_t* __restrict__ depth, const uint32_t* __restrict__ out_degree,
-                                                  uint32_t* __restrict__ list, MsCtl* ctl) {
+__global__ void __launch_bounds__(256) msk_finish(uint32_t V, uint32_t E, unsigned long long* F, unsigned long long* N,
+                                                  unsigned long long* vis, uint16_t* depth,
+                                                  const uint32_t* __restrict__ out_degree, uint32_t* list, MsCtl* ctl) {
   wait_for_prior_kernel();
   let_next_kernel_start();
   if (ctl->done) return;
@@ -583,7 +578,7 @@ struct PprIds {
 
 // Sum over the in-edges [j0, j1) of their source's 32 contribs, 16 edges at a
 // time (the first 16 ids come loaded); returns this lane's seed's sum.
-__device__ __forceinline__ float ppr_row_sum(const uint32_t* __restrict__ nbr, const float4* __restrict__ C4,
+__device__ __forceinline__ float ppr_row_sum(const uint32_t* __restrict__ nbr, const float4* C4,
                                              uint32_t j0, uint32_t j1, uint32_t grp, uint32_t sub, PprIds ids) {
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (uint32_t j = j0; j < j1; j += 16) {
@@ -591,7 +586,7 @@ __device__ __forceinline__ float ppr_row_sum(const uint32_t* __restrict__ nbr, c
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       c[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (ids.u[q] != 0xFFFFFFFFu) c[q] = __ldg(&C4[(size_t)ids.u[q] * 8 + sub]);
+      if (ids.u[q] != 0xFFFFFFFFu) c[q] = C4[(size_t)ids.u[q] * 8 + sub];
     }
     if (j + 16 < j1) ids.load(nbr, j + 16, j1, grp);
 #pragma unroll
@@ -622,8 +617,8 @@ struct PprParams {
 
 // Update of vertex v from its sums: seed number k, vertex `seed`, on this lane.
 __device__ __forceinline__ void ppr_update(uint32_t v, float s, uint32_t k, uint32_t seed, const PprParams& p,
-                                           const uint32_t* __restrict__ out_degree, float* __restrict__ R,
-                                           float* __restrict__ Cn, double& err, float old, uint32_t d) {
+                                           const uint32_t* __restrict__ out_degree, float* R, float* Cn, double& err,
+                                           float old, uint32_t d) {
   const size_t at = (size_t)v * kPprSeeds + k;
   const float nv = __fadd_rn(seed == v ? p.base : 0.0f, __fmul_rn(p.damp, s));
   R[at] = nv;
@@ -633,13 +628,12 @@ __device__ __forceinline__ void ppr_update(uint32_t v, float s, uint32_t k, uint
 
 __global__ void __launch_bounds__(256, 6) pprk_iter(const PprChunk* __restrict__ chunks, uint32_t n_chunks,
                                                     const uint32_t* __restrict__ vfirst,
-                                                    const uint32_t* __restrict__ vcount, uint32_t* __restrict__ done,
-                                                    float* __restrict__ partials, const uint32_t* __restrict__ light,
+                                                    const uint32_t* __restrict__ vcount, uint32_t* done,
+                                                    float* partials, const uint32_t* __restrict__ light,
                                                     uint32_t n_light, const uint2* __restrict__ rows,
                                                     const uint32_t* __restrict__ nbr,
                                                     const uint32_t* __restrict__ out_degree,
-                                                    const float* __restrict__ C, float* __restrict__ Cn,
-                                                    float* __restrict__ R, PprParams p, PprCtl* __restrict__ ctl,
+                                                    const float* C, float* Cn, float* R, PprParams p, PprCtl* ctl,
                                                     uint32_t it) {
   __shared__ double s_err[8][kPprSeeds];
   wait_for_prior_kernel();
@@ -719,7 +713,7 @@ __global__ void __launch_bounds__(256, 6) pprk_iter(const PprChunk* __restrict__
 }
 
 // the run stops after an iteration in which every seed changed by < eps (L1)
-__global__ void pprk_check(PprCtl* __restrict__ ctl, uint32_t it, uint32_t nseeds, double eps) {
+__global__ void pprk_check(PprCtl* ctl, uint32_t it, uint32_t nseeds, double eps) {
   wait_for_prior_kernel();
   let_next_kernel_start();
   if (threadIdx.x != 0 || ctl->stop) return;

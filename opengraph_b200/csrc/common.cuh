@@ -198,6 +198,10 @@ __device__ __forceinline__ void ba_flush(BlockAppend<CAP>& q, uint32_t* out, uin
 // in the stream has ended: wait_for_prior_kernel, its first statement, then waits
 // for that end and for the earlier kernel's writes, so only the launch itself
 // overlaps.  let_next_kernel_start lets the kernel behind this one do the same.
+// What the kernel ahead writes is not constant for as long as such a kernel is
+// resident: its pointers carry no __restrict__ and are not read through __ldg,
+// either of which lets the compiler take the read-only path or move a load above
+// the wait.  The graph's own arrays, which no such kernel writes, keep both.
 __device__ __forceinline__ void wait_for_prior_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

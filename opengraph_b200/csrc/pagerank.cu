@@ -245,7 +245,7 @@ __device__ __forceinline__ void pr_block_finish(double err, uint32_t active, PrC
 // s += c[nbr[j]] for j = j0, j0+STRIDE, ... < j1, in that order; each step
 // issues K predicated neighbour loads, then their K gathers.
 template <uint32_t STRIDE, int K>
-__device__ __forceinline__ float strided_sum(const float* __restrict__ c, const uint32_t* __restrict__ nbr,
+__device__ __forceinline__ float strided_sum(const float* c, const uint32_t* __restrict__ nbr,
                                              uint32_t j0, uint32_t j1) {
   float s = 0.0f;
   for (uint32_t j = j0; j < j1; j += K * STRIDE) {
@@ -254,7 +254,7 @@ __device__ __forceinline__ float strided_sum(const float* __restrict__ c, const 
     for (int k = 0; k < K; k++) x[k] = (j + k * STRIDE < j1) ? __ldg(&nbr[j + k * STRIDE]) : 0u;
     float cx[K];
 #pragma unroll
-    for (int k = 0; k < K; k++) cx[k] = (j + k * STRIDE < j1) ? __ldg(&c[x[k]]) : 0.0f;
+    for (int k = 0; k < K; k++) cx[k] = (j + k * STRIDE < j1) ? c[x[k]] : 0.0f;
 #pragma unroll
     for (int k = 0; k < K; k++)
       if (j + k * STRIDE < j1) s = __fadd_rn(s, cx[k]);
@@ -328,14 +328,14 @@ struct StagePipe {
   // 1.65 M x 26 210 and 198; RMAT-22 within 1 %); on the medium rows, whose
   // gathers hit more often, it costs instructions (RMAT-22 245 and 261).
   template <bool kTest = false>
-  __device__ __forceinline__ void gather(float* stage, const uint32_t* __restrict__ nbr, const float* __restrict__ c,
+  __device__ __forceinline__ void gather(float* stage, const uint32_t* __restrict__ nbr, const float* c,
                                          uint32_t w0, uint32_t e1, uint32_t lane) {
 #pragma unroll
     for (uint32_t m = 0; m < kStage / 32; m++) {
       const uint32_t j = w0 + m * 32 + lane;
       if (j < e1) {
         if (kTest && u[m] == 0u)
-          stage[m * 32 + lane] = __ldg(c);
+          stage[m * 32 + lane] = *c;
         else
           cp_async4(&stage[m * 32 + lane], c + u[m]);
       }
@@ -373,11 +373,10 @@ struct StagePipe {
 template <int R>
 __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
     const PrLay* __restrict__ lay, const PrChunkItem* __restrict__ chunks, const uint32_t* __restrict__ vfirst,
-    const uint32_t* __restrict__ vcount, uint32_t* __restrict__ done, float* __restrict__ partials,
+    const uint32_t* __restrict__ vcount, uint32_t* done, float* partials,
     const uint2* __restrict__ rows, const uint32_t* __restrict__ off_light, const uint32_t* __restrict__ unit_first,
     const uint32_t* __restrict__ med_off, const uint32_t* __restrict__ med_v, const uint32_t* __restrict__ nbr, const uint32_t* __restrict__ out_degree, const uint32_t* __restrict__ perm,
-    const float* __restrict__ contrib, float* __restrict__ contrib_next, float* __restrict__ pr, PrParams p,
-    PrCtl* __restrict__ ctl, uint32_t it) {
+    const float* contrib, float* contrib_next, float* pr, PrParams p, PrCtl* ctl, uint32_t it) {
   extern __shared__ uint32_t s_dyn[];  // per warp: stage and medium-row table
   constexpr uint32_t kStage = kStageOf<R>;
   __shared__ float s_part[kPullGroups][kPullGroup / 32];
