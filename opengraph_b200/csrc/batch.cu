@@ -262,13 +262,14 @@ __global__ void __launch_bounds__(256) msk_push_long(const uint4* items, const u
     const uint4 it = items[t];
     const unsigned long long fu = F[it.x];
     const unsigned long long f[4] = {fu, fu, fu, fu};
-    for (uint32_t j = it.y + lane; j < it.z; j += 128) {
+    const uint32_t len = it.z - it.y;  // counted from it.y: the piece may end just below 2^32
+    for (uint32_t j = lane; j < len; j += 128) {
       uint32_t w[4];
       bool ok[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        ok[k] = j + k * 32 < it.z;
-        w[k] = ok[k] ? (__ldg(&nbr_f[j + k * 32]) & 0x3FFFFFFFu) : 0u;
+        ok[k] = j + k * 32 < len;
+        w[k] = ok[k] ? (__ldg(&nbr_f[it.y + j + k * 32]) & 0x3FFFFFFFu) : 0u;
       }
       ms_push4(f, w, ok, vis, N);
     }

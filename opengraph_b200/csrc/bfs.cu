@@ -376,7 +376,7 @@ struct BuSmem {
   int32_t* parents;
   uint32_t* distances;
   uint32_t dnext;
-  uint32_t first;                        // CTA-wide scan: position of the first hit in the step
+  uint32_t first;                        // CTA-wide scan: place of the first hit in what it scans of the row
   uint32_t x_nf, x_edges, x_mx;          // totals of those rows
   unsigned long long x_fed;
 };
@@ -962,7 +962,7 @@ __device__ __forceinline__ void bu_long_rows(const BfsBufs& b, const uint32_t* b
       end = rr.x + rr.y;
     }
     bool hit_row = false;
-    const uint32_t lim = min(end, j0 + kLongCut);
+    const uint32_t lim = j0 + min(end - j0, kLongCut);
     for (uint32_t j = j0; j < lim; j += kLongStep) {
       uint32_t x[kLongLoads];
 #pragma unroll
@@ -1063,14 +1063,14 @@ __device__ __noinline__ void bu_more_rows(BuSmem& sm) {
       const uint32_t hv = sm.hv[h] & ~kMoreBit;
       uint32_t v, od, j0, end;
       bu_row_of(hv, sm, v, od, j0, end);
-      const uint32_t lim = min(end, j0 + kMoreCut);
+      const uint32_t n = min(end - j0, kMoreCut);
       bool found = false;
-      for (uint32_t j = j0; j < lim; j += 32 * K) {
+      for (uint32_t k = 0; k < n; k += 32 * K) {  // counted from j0: the row may end just below 2^32
         uint32_t x[K];
 #pragma unroll
         for (uint32_t q = 0; q < K; q++) {
-          const uint32_t jq = j + q * 32 + lane;
-          x[q] = jq < lim ? (__ldg(&nbr_i[jq]) & 0x3FFFFFFFu) : kInvalid;
+          const uint32_t kq = k + q * 32 + lane;
+          x[q] = kq < n ? (__ldg(&nbr_i[j0 + kq]) & 0x3FFFFFFFu) : kInvalid;
         }
         uint32_t q0 = 0, u = 0, m = 0;
 #pragma unroll
@@ -1085,7 +1085,7 @@ __device__ __noinline__ void bu_more_rows(BuSmem& sm) {
         if (m) {
           const uint32_t l0 = (uint32_t)__ffs(m) - 1;
           if (lane == l0) {
-            atomicAdd(&sm.x_edges, j + q0 * 32 + l0 + 1 - j0);
+            atomicAdd(&sm.x_edges, k + q0 * 32 + l0 + 1);
             bu_more_found(v, u, od, sm);
           }
           found = true;
@@ -1093,8 +1093,8 @@ __device__ __noinline__ void bu_more_rows(BuSmem& sm) {
         }
       }
       if (!found && lane == 0) {
-        atomicAdd(&sm.x_edges, lim - j0);
-        if (lim < end) {
+        atomicAdd(&sm.x_edges, n);
+        if (n < end - j0) {
           sm.hv[h] = hv | kHugeBit;
           sm.nhuge = 1;
         } else {
@@ -1116,17 +1116,18 @@ __device__ __noinline__ void bu_more_rows(BuSmem& sm) {
       if (threadIdx.x == 0) sm.first = kInvalid;
       __syncthreads();
       bool found = false;
-      for (uint32_t j = j0; j < end; j += kSearchT * K) {
+      const uint32_t n = end - j0;
+      for (uint64_t k = 0; k < n; k += kSearchT * K) {
         uint32_t x[K], mine = kInvalid, u = 0;
 #pragma unroll
         for (uint32_t q = 0; q < K; q++) {
-          const uint32_t jq = j + q * kSearchT + threadIdx.x;
-          x[q] = jq < end ? (__ldg(&nbr_i[jq]) & 0x3FFFFFFFu) : kInvalid;
+          const uint64_t kq = k + q * kSearchT + threadIdx.x;
+          x[q] = kq < n ? (__ldg(&nbr_i[j0 + (uint32_t)kq]) & 0x3FFFFFFFu) : kInvalid;
         }
 #pragma unroll
         for (int q = (int)K - 1; q >= 0; q--)
           if (x[q] != kInvalid && ((bm_cur[x[q] >> 5] >> (x[q] & 31)) & 1u)) {
-            mine = j + q * kSearchT + threadIdx.x;
+            mine = (uint32_t)k + q * kSearchT + threadIdx.x;
             u = x[q];
           }
         if (mine != kInvalid) atomicMin(&sm.first, mine);
@@ -1135,7 +1136,7 @@ __device__ __noinline__ void bu_more_rows(BuSmem& sm) {
         __syncthreads();
         if (first != kInvalid) {
           if (mine == first) {
-            atomicAdd(&sm.x_edges, first + 1 - j0);
+            atomicAdd(&sm.x_edges, first + 1);
             bu_more_found(v, u, od, sm);
           }
           found = true;
@@ -1143,7 +1144,7 @@ __device__ __noinline__ void bu_more_rows(BuSmem& sm) {
         }
       }
       if (!found && threadIdx.x == 0) {
-        atomicAdd(&sm.x_edges, end - j0);
+        atomicAdd(&sm.x_edges, n);
         bu_push_ul(sm, hv);
       }
       __syncthreads();  // before the next row resets `first`

@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kPullThreads, 1) pr_pull_kernel(
     const uint32_t grp = threadIdx.x / kPullGroup, gt = threadIdx.x % kPullGroup;
     for (uint32_t g = (kPullGroups - 1 - grp) * gridDim.x + blockIdx.x; g < n_chunks; g += gridDim.x * kPullGroups) {
       const PrChunkItem ci = chunks[g];
-      float sum = strided_sum<kPullGroup, R == 1 ? 8 : 4>(contrib, nbr, ci.j0 + gt, ci.j1);
+      float sum = strided_sum<kPullGroup, R == 1 ? 8 : 4>(contrib, nbr + ci.j0, gt, ci.j1 - ci.j0);
       sum = warp_fold(sum);
       if (lane == 0) s_part[grp][gt >> 5] = sum;
       asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(kPullGroup) : "memory");
