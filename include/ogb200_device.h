@@ -104,8 +104,9 @@ void ogb_graph_destroy(ogb_graph *g);
 /* For tests: makes one graph meet what a GPU will not do on request.
  * OGB_TEST_SORT_GIVES_UP: its next `value` sorts report that a bounded wait gave
  * up, their first payload lost.  OGB_TEST_NO_CLUSTERS, before its first search:
- * the device cannot launch thread-block clusters. */
-enum { OGB_TEST_SORT_GIVES_UP = 1, OGB_TEST_NO_CLUSTERS = 2 };
+ * the device cannot launch thread-block clusters.  OGB_TEST_WIDE_LOOKBACK: its
+ * sorts use the look-back words of 2^30 edges and more. */
+enum { OGB_TEST_SORT_GIVES_UP = 1, OGB_TEST_NO_CLUSTERS = 2, OGB_TEST_WIDE_LOOKBACK = 3 };
 int ogb_graph_test_option(ogb_graph *g, uint32_t option, uint32_t value);
 /* Sort (SORT_TYPE semantics) and build both CSR directions from device edge
  * arrays; all ids < V <= 2^30.  Inputs are read only.  d_w may be NULL. */

@@ -1933,6 +1933,7 @@ extern "C" int ogb_graph_test_option(ogb_graph* g, uint32_t option, uint32_t val
   if (!g) return fail(ERR_ARG, "null");
   switch (option) {
     case OGB_TEST_SORT_GIVES_UP: g->g.sort_ws.give_up = value; return OK;
+    case OGB_TEST_WIDE_LOOKBACK: g->g.sort_ws.wide = value != 0; return OK;
     case OGB_TEST_NO_CLUSTERS: g->g.test_no_clusters = value != 0; return OK;
   }
   return fail(ERR_ARG, "test option %u", option);

@@ -455,14 +455,14 @@ static int launch_pass(const PassArgs<S>& a, cudaStream_t stream) {
 
 }  // namespace
 
-static size_t status_word_bytes(uint64_t n) {
-  return n < kNarrowLimit ? sizeof(uint32_t) : sizeof(unsigned long long);
+static size_t status_word_bytes(const SortWorkspace& ws, uint64_t n) {
+  return n < kNarrowLimit && !ws.wide ? sizeof(uint32_t) : sizeof(unsigned long long);
 }
 
 int SortWorkspace::reserve(uint64_t n, bool weighted, int max_passes) {
   const uint64_t tiles = (n + kTile - 1) / kTile;
   OGB_TRY(hist.alloc((2 * 8 * 256 + kCtrWords) * sizeof(uint32_t)));
-  OGB_TRY(status.alloc((size_t)max_passes * tiles * 256 * status_word_bytes(n) + 256));
+  OGB_TRY(status.alloc((size_t)max_passes * tiles * 256 * status_word_bytes(*this, n) + 256));
   OGB_TRY(tmp_k.alloc(n * 4));
   OGB_TRY(tmp_v0.alloc(n * 4));
   if (weighted) OGB_TRY(tmp_v1.alloc(n * 4));
@@ -488,7 +488,7 @@ static int sort_impl(const KV& in, const KV& out, uint64_t n, bool lex, uint32_t
   const DigitLayout lay = digit_layout(key_bits);
   const int P = (lex ? 2 : 1) * lay.ndig;
   const uint64_t tiles = (n + kTile - 1) / kTile;
-  const size_t word = status_word_bytes(n);
+  const size_t word = status_word_bytes(ws, n);
   digit_hist_kernel<<<grid, 256, 0, stream>>>(in.k, n, lay.ndig, lay, d_hist, ws.status.as<uint4>(),
                                               (uint64_t)P * tiles * 256 * word / 16);
   if (lex) digit_hist_kernel<<<grid, 256, 0, stream>>>(in.v0, n, lay.ndig, lay, d_hist + 4 * 256, nullptr, 0);

@@ -18,7 +18,8 @@ struct SortWorkspace {
   DevBuf tmp_k, tmp_v0, tmp_v1;  // one ping-pong array set
   uint32_t* err = nullptr;       // where a pass reports an error (null: the counters' own word)
   // set by tests only
-  uint32_t give_up = 0;               // the next so many sorts report that a look-back gave up, their first payload lost
+  uint32_t give_up = 0;  // the next so many sorts report that a look-back gave up, their first payload lost
+  bool wide = false;     // 8-byte look-back words at any size
   int reserve(uint64_t n, bool weighted, int max_passes);
 };
 
