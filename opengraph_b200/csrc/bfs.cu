@@ -51,8 +51,8 @@
 //    compacted list of still-unvisited vertices; each CTA takes one equal,
 //    contiguous range of candidates; a candidate's first kFirst in-neighbours
 //    and their frontier bits are loaded at once, longer rows go to a per-round
-//    list scanned by groups of 8 lanes (the first hit in CSR order still
-//    wins); the dense-probe mode walks every vertex (a warp's ballot is one
+//    list scanned by groups of 4 lanes, what is left of them by a warp and then
+//    by the CTA (the first hit in CSR order still wins); the dense-probe mode walks every vertex (a warp's ballot is one
 //    whole word of the next bitmap);
 //  * a top-down step sets the bitmap bit of every vertex it discovers and a
 //    bottom-up step lists the vertices it discovers, so a change of
@@ -122,7 +122,7 @@ struct BfsCtrl {
   uint32_t lmax;                     // largest out-degree on the expansion list
   uint32_t narrow;                   // narrow lists made in a row by top-down steps
   uint32_t streak;                   // narrow lists in a row that start the next run of narrow steps
-  uint32_t more;                     // why the kernel ended: kMoreNone, kMoreNarrow or kMoreWide
+  uint32_t to_narrow;                // 1: the grid-wide kernel ended at a run of narrow steps
   uint32_t rebuild;                  // 1: the bitmaps must be made from the list (after narrow steps)
   uint32_t phase;                    // counter set of the next phase (an index into ctl)
   unsigned long long edges_examined;
@@ -1470,7 +1470,6 @@ __device__ void bu_host_phase(const BfsBufs& b, const uint32_t* bm_cur, uint32_t
 // ------------------------------------------------------------ control ------
 
 constexpr uint32_t kActDone = 0, kActTD = 1, kActBU = 2, kActNarrow = 3;
-constexpr uint32_t kMoreNone = 0, kMoreNarrow = 1, kMoreWide = 2;
 
 // Narrow steps (bfsk_narrow).  A list is narrow when its entries have at most
 // kNarDeg out-edges and the discoveries of a CTA's share of it fit the CTA's
@@ -1826,7 +1825,7 @@ __global__ void __launch_bounds__(kSearchT, 4) bfsk_search(BfsBufs b, BfsDevStat
   }
   if (threadIdx.x == 0) {
     S.rebuild = 0;
-    S.more = kMoreNone;
+    S.to_narrow = 0;
   }
   for (;;) {
     const bool learned = S.mode == BFS_LEARNED;
@@ -1877,7 +1876,7 @@ __global__ void __launch_bounds__(kSearchT, 4) bfsk_search(BfsBufs b, BfsDevStat
     }
     const uint32_t act = s_act;
     if (act == kActNarrow && leader) {
-      S.more = kMoreNarrow;
+      S.to_narrow = 1;
       S.phase = p % 3;
     }
     if (act == kActDone || act == kActNarrow) break;
@@ -2070,7 +2069,6 @@ __global__ void __cluster_dims__(kNarC, 1, 1) __launch_bounds__(kNarT, 1) bfsk_n
         distances[v] = S.depth;
       }
       if (rank == 0 && tid == 0) {
-        c.more = kMoreWide;
         c.narrow = 0;
         if (steps < kNarShort)
           c.streak *= 2;
@@ -2336,7 +2334,7 @@ int bfs_run_roots(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint32_t 
     OGB_CUDA(cudaEventRecord(w->ev_stop, s));
     OGB_CUDA(cudaMemcpyAsync(w->h_state, w->state.p, kStateCopy, cudaMemcpyDeviceToHost, s));
     OGB_CUDA(cudaStreamSynchronize(s));
-    if (h->err || h->c.more != kMoreNarrow) break;
+    if (h->err || !h->c.to_narrow) break;
     bfsk_narrow<<<kNarC, kNarT, kNarSmem, s>>>(b, st);
     OGB_CUDA(cudaGetLastError());
     launches++;

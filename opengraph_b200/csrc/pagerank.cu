@@ -27,21 +27,23 @@
 //     the CTA that finishes a vertex's last chunk adds the chunk sums in chunk
 //     order and updates the vertex.  A hub therefore never serializes an
 //     iteration, and every sum has one fixed order (deterministic).
-// Every strided loop issues four independent gathers before it adds them, in
-// the same order as the plain loop, so the order is unchanged.
+// Every strided loop issues four independent gathers (eight on a small graph)
+// before it adds them, in the same order as the plain loop, so the order is
+// unchanged.
 // Pull gathers one contrib value per edge, at random, so it is bound by
 // memory latency more than by HBM bandwidth.  Pull therefore runs on a
 // re-laid copy of the inverse neighbour array (built once per graph): source
 // ids renumbered by descending out-degree, so the contribs of the sources of
-// most edges share few cache lines (contrib is kept in that numbering), and the rows of in-degree <= warp_thr stored first and
-// contiguous, so a warp loads the edges of 128 light rows with coalesced
-// loads and gathers them 256 at a time (light rows were the latency tail of
-// the iteration: a lane walked its row one dependent gather per step).  The
+// most edges share few cache lines (contrib is kept in that numbering), and the
+// rows of in-degree <= warp_thr stored first and contiguous, so a warp loads the
+// edges of 64 light rows (32 on a small graph) with coalesced loads and gathers
+// them 256 (512) at a time (light rows were the latency tail of the iteration: a lane walked its row one dependent gather per step).  The
 // rows, their order and every summation order are unchanged, so the results
 // are bit-identical.  Pull runs one 1024-thread CTA per SM; it takes chunks
-// first (four 256-thread groups per CTA), then warp rows, then light rows.  Iterations are launched back to back
-// without host round trips: each iteration's last CTA records error/active
-// and, when active == 0, sets a stop flag that later launches read first.
+// first (four 256-thread groups per CTA), then warp rows, then light rows.
+// Iterations are launched back to back without host round trips: each iteration's
+// last CTA records error/active and, when active == 0, sets a stop flag that later
+// launches read first.
 #include "graph.cuh"
 
 #include <algorithm>
