@@ -1474,7 +1474,7 @@ constexpr uint32_t kActDone = 0, kActTD = 1, kActBU = 2, kActNarrow = 3;
 // Narrow steps (bfsk_narrow).  A list is narrow when its entries have at most
 // kNarDeg out-edges and the discoveries of a CTA's share of it fit the CTA's
 // queue.  The grid-wide kernel hands over after `streak` narrow lists of at most
-// kNarEnter entries in a row, at first kNarStreak, so that the two or three small
+// kNarEnter entries in a row (narrow_counts), at first kNarStreak, so that the two or three small
 // steps at the ends of a low-diameter search, which are followed by a large one or
 // by the end, stay where they are.
 // A run and the way back (two launches, a wait of the host, the bitmaps remade)
@@ -1490,6 +1490,15 @@ constexpr uint32_t kNarNever = 0xFFFFFFFFu;  // a streak that no search reaches 
 constexpr uint32_t kNarQ = 8192;  // queue entries per CTA
 __device__ __forceinline__ bool narrow_fits(const BfsCtrl& c) {
   return c.lmax <= kNarDeg && c.lsize <= kNarCap && (c.lsize + kNarC - 1) / kNarC * c.lmax <= kNarQ;
+}
+// After a top-down step: the list counts towards a run.  A frontier that grows or
+// shrinks fast does not: either the lists are soon wide or the search soon ends, and
+// the run would not pay (uniform graphs of 1 M vertices, one push-only search in us
+// without and with this condition: 4 out-edges each 327 and 311, 6 out-edges 393 and 370;
+// 1.6 out-edges, whose lists grow slowly, 412 and 427; the grid's the same).
+__device__ __forceinline__ bool narrow_counts(const BfsCtrl& c) {
+  return c.lsize <= kNarEnter && c.lmax <= kNarDeg && c.qcount >= c.frontier / 2 &&
+         c.qcount <= c.frontier + c.frontier / 2 + 2;
 }
 // The next step is top-down by ctrl_decide's rule.
 __device__ __forceinline__ bool td_next(const BfsCtrl& c) {
@@ -1647,7 +1656,7 @@ __device__ void ctrl_finish_td(BfsCtrl& c, uint32_t total_edges, const BfsCtl& k
   c.bm_w = r;
   c.td_steps++;
   c.ul_fresh = 0;  // the unvisited list may now hold vertices this step visited
-  c.narrow = (c.lsize <= kNarEnter && c.lmax <= kNarDeg) ? c.narrow + 1 : 0u;
+  c.narrow = narrow_counts(c) ? c.narrow + 1 : 0u;
   ctrl_level(c, st, leader, 0, c.qcount, total_edges, t0);
 }
 

@@ -1,11 +1,13 @@
 """When a search hands its narrow steps to the cluster kernel: paths with hubs
 every few vertices, counted in launches (the search kernel once, and twice more
 per run).  Runs too short to pay must not be tried again and again, long ones must
-go on, and a long one lets short lists start a run again."""
+go on, a long one lets short lists start a run again, and a frontier that grows or
+shrinks fast starts none."""
 import numpy as np
 import pytest
 
 from test_bfs_gpu import check_parents
+from test_bfs_narrow_gpu import layered
 from test_build_gpu import dev, host
 
 pytestmark = pytest.mark.gpu
@@ -27,15 +29,21 @@ def hub_path(sections):
     return perm[s].astype(np.uint32), perm[d].astype(np.uint32), V, int(perm[0])
 
 
-# a run starts after 4, then 8, ... narrow lists; a period of p vertices has p - 1
+# a run starts after 4, then 8, ... narrow lists of about equal length; the two after a hub's are not
 CASES = {
-    "every5": ([(1000, 5, 33)], 3),               # a run of 1 step; 8 lists in a row never come
-    "every8": ([(1000, 8, 1000)], 3),             # 4 steps
-    "every12": ([(1200, 12, 33)], 5),             # 8 steps, then 4
-    "every13": ([(1300, 13, 100)], 1 + 2 * 100),  # 9 steps: as good either way, and it stays
+    "every5": ([(1000, 5, 33)], 1),               # 4 such lists in a row never come
+    "every8": ([(1000, 8, 1000)], 3),             # a run of 2 steps; 8 lists never come
+    "every12": ([(1200, 12, 33)], 5),             # 6 steps, then 2
+    "every15": ([(1500, 15, 100)], 1 + 2 * 100),  # 9 steps: as good either way, and it stays
     "every100": ([(1000, 100, 40)], 1 + 2 * 10),
     "none": ([(600, 0, 0)], 3),
-    "reset": ([(500, 5, 33), (500, 0, 0), (500, 5, 33)], 1 + 2 * 3),
+    "reset": ([(500, 8, 33), (500, 0, 0), (500, 8, 33)], 1 + 2 * 3),
+}
+# layers of these widths
+LAYERS = {
+    "even": ([1, 4, 16, 64] + [700] * 30, 4, 3),
+    "doubling": ([1 << k for k in range(15)], 2, 1),
+    "shrinking": ([1, 32, 1000, 20_000, 1500, 400, 100, 25, 6], 32, 1),
 }
 
 
@@ -43,11 +51,15 @@ NO_CLUSTERS = 2  # test option of a graph: as on a device that cannot launch the
 
 
 @pytest.mark.parametrize("clusters", [True, False])
-@pytest.mark.parametrize("name", list(CASES))
+@pytest.mark.parametrize("name", list(CASES) + list(LAYERS))
 def test_launches(torch_cuda, lib, oracle, name, clusters):
     torch = torch_cuda
-    sections, launches = CASES[name]
-    s, d, V, root = hub_path(sections)
+    if name in CASES:
+        sections, launches = CASES[name]
+        s, d, V, root = hub_path(sections)
+    else:
+        widths, degree, launches = LAYERS[name]
+        s, d, V, root = layered(widths, degree, 3)
     g = oracle.build(s, d, V, 0)
     dg = lib.device_graph()
     if not clusters:
