@@ -64,6 +64,12 @@ constexpr uint32_t kMarkThr = 32;       // out-rows longer than this are deferre
 constexpr uint32_t kOutBig = 1024;      // deferred out-rows longer than this go by chunks
 constexpr uint32_t kOutChunk = 1024;    // edges per chunk of a long out-row
 constexpr uint32_t kDdMaxIters = 1024;
+// Data-driven pull on fewer vertices starts with the light rows: the vertices they put
+// on the next worklist are marked when the other rows' marks come, which then write
+// nothing to the few lines that hold all flags.  us of 20 iterations, light rows first
+// and heavy rows first: RMAT-11 (16 edges per vertex) 770 and 1200, RMAT-13 1130 and
+// 1290, RMAT-14 1400 and 1270, RMAT-18 2830 and 2580.
+constexpr uint32_t kLightFirst = 1u << 14;
 
 struct DdCtl {
   double err[kDdMaxIters];
@@ -212,21 +218,32 @@ __global__ void dd_fill_kernel(uint32_t lo, uint32_t hi, const uint2* __restrict
   }
 }
 
-// Blocks of a pass by row class: no more than the class has work for.  (With eight
-// blocks per SM for the medium rows, numbered before the light ones' whether there
-// are any or not, 700 K vertices of 9 in-edges each took 5 % longer in the
-// data-driven pull and 3 % in SPMV than with the light rows first.)
+// Blocks of a pass by row class.
 struct Grid3 {
   uint32_t light, med, heavy;
   uint32_t total() const { return light + med + heavy; }
+  // The rows_pass number of block x when the light rows come first, then the medium.
+  __device__ uint32_t light_first(uint32_t x) const {
+    return x < light ? heavy + med + x : (x < light + med ? heavy + x - light : x - light - med);
+  }
 };
 
-Grid3 rows_grid(uint32_t V, uint32_t n_med, uint32_t n_hch) {
+Grid3 rows_grid(uint32_t V) {
   const uint32_t sms = sm_count();
   Grid3 g;
   g.light = std::max<uint32_t>(1, std::min<uint32_t>(sms * 8, ceil_div(V, kT)));
-  g.med = std::min<uint32_t>(sms * 8, ceil_div(n_med, kT / 32));
-  g.heavy = std::min<uint32_t>(sms * 2, n_hch);
+  g.med = sms * 8;
+  g.heavy = sms * 2;
+  return g;
+}
+
+// No more blocks than the classes' lists have work for: with empty blocks before the
+// light rows', 700 K vertices of 9 in-edges each took 5 % longer in the data-driven
+// pull and 3 % in SPMV.
+Grid3 rows_grid(uint32_t V, uint32_t n_med, uint32_t n_hch) {
+  Grid3 g = rows_grid(V);
+  g.med = std::min<uint32_t>(g.med, ceil_div(n_med, kT / 32));
+  g.heavy = std::min<uint32_t>(g.heavy, n_hch);
   return g;
 }
 
@@ -435,10 +452,11 @@ struct PullPolicy {
 };
 
 __global__ void __launch_bounds__(kT) dd_pull_kernel(const uint2* __restrict__ rows, const uint32_t* __restrict__ med,
-                                                     HeavyRows heavy, Grid3 G, PullPolicy pol,
+                                                     HeavyRows heavy, Grid3 G, bool light_first, PullPolicy pol,
                                                      DdCtl* __restrict__ ctl, uint32_t it) {
   if (ctl->stop) return;
-  rows_pass(blockIdx.x, rows, med, heavy, ctl->n_med, ctl->n_hch, pol.p.V, G.heavy, G.med, G.light, pol);
+  const uint32_t b = light_first ? G.light_first(blockIdx.x) : blockIdx.x;
+  rows_pass(b, rows, med, heavy, ctl->n_med, ctl->n_hch, pol.p.V, G.heavy, G.med, G.light, pol);
   if (block_totals(pol.err, pol.act, &ctl->err[it], &ctl->active[it], &ctl->done_a[it])) {
     if (ld_volatile_u32(&ctl->active[it]) == 0) {
       ctl->stop_iter = it;
@@ -612,9 +630,7 @@ __global__ void __launch_bounds__(kT) dd_pullpush_kernel(const uint2* __restrict
   // the light rows first, the heavy last: rows read ranks that this pass has
   // already updated, and the hubs gain most from that (RMAT-22 to 1e-4: 77
   // iterations; 96 with the heavy rows first)
-  const uint32_t x = blockIdx.x;
-  const uint32_t b = x < G.light ? G.heavy + G.med + x : (x < G.light + G.med ? G.heavy + (x - G.light) : x - G.light - G.med);
-  rows_pass(b, rows, med, heavy, ctl->n_med, ctl->n_hch, pol.p.V, G.heavy, G.med, G.light, pol);
+  rows_pass(G.light_first(blockIdx.x), rows, med, heavy, ctl->n_med, ctl->n_hch, pol.p.V, G.heavy, G.med, G.light, pol);
   block_totals(pol.err, pol.act, &ctl->err[it], &ctl->active[it], &ctl->done_a[it]);
 }
 
@@ -875,7 +891,9 @@ int pagerank_dd_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsil
   p.base_pr = 1.0f - p.damp;  // float, as newPageRankStatsGraphCSR (pageRank.c:47-75)
   p.epsilon = epsilon;
   const int sms = sm_count();
-  const Grid3 G = rows_grid(V, w->n_med, w->n_hch);
+  const Grid3 G = rows_grid(V);
+  const bool light_first = V < kLightFirst;
+  const Grid3 Gp = light_first ? G : rows_grid(V, w->n_med, w->n_hch);  // of the pull
   uint8_t* cur = w->flags0.as<uint8_t>();
   uint8_t* nxt = w->flags1.as<uint8_t>();
   float* resid = w->resid.as<float>();
@@ -903,7 +921,8 @@ int pagerank_dd_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsil
       dd_contrib_kernel<<<sms * 8, kT, 0, s>>>(V, g.fwd.d_out_degree(), ranks, w->contrib.as<float>(), nxt, defer,
                                                ctl);
       PullPolicy pol{cur, nxt, w->contrib.as<float>(), g.inv.d_dst(), ranks, g.fwd.d_rows(), g.fwd.d_dst(), defer, p};
-      dd_pull_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), G, pol, ctl, it);
+      dd_pull_kernel<<<Gp.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), Gp, light_first, pol,
+                                               ctl, it);
       dd_defer_kernel<false><<<sms * 8, kT, 0, s>>>(V, g.fwd.d_rows(), g.fwd.d_dst(), defer, dvec, och, resid, nxt,
                                                     epsilon, false, ctl, it);
     } else {
@@ -1180,8 +1199,7 @@ int pagerank_range_step(DevGraph& g, uint32_t lo, uint32_t hi, const float* cont
   p.base_pr = 1.0f - p.damp;
   p.epsilon = epsilon;
   RangePolicy pol{lo, g.inv.d_dst(), g.fwd.d_out_degree(), contrib, ranks, contrib_next, p, peers, npeers};
-  // the lists' lengths stay on the device: no step waits for them
-  const Grid3 G = rows_grid(hi - lo, 0xFFFFFFFFu, 0xFFFFFFFFu);
+  const Grid3 G = rows_grid(hi - lo);  // the lists' lengths stay on the device: no step waits for them
   range_step_kernel<<<G.total(), kT, 0, s>>>(g.inv.d_rows(), lo, hi, w->med.as<uint32_t>(), w->heavy.view(), G, pol,
                                              ctl, d_err, d_active);
   OGB_CUDA(cudaGetLastError());
