@@ -391,7 +391,7 @@ def stages(lib, og, g, ts, td, tw, V, E, dev, hbm_peak):
     out["csr_build"] = {"ms": round(build_ms, 3), "medges_per_s": round(E / build_ms / 1e3, 1),
                         "algorithmic_gb": round(alg / 1e9, 3), "gbs": round(alg / build_ms / 1e6, 1),
                         "frac": round(alg / build_ms / 1e6 / hbm_peak, 4),
-                        "note": "device sort+CSR both directions incl. one 8 KB host read per sort"}
+                        "note": "device sort+CSR both directions; one 8-byte host read at the end"}
     # ---- PageRank pull / push to 1e-6 -----------------------------------
     ranks = torch.empty(V, dtype=torch.float32, device=dev)
     for mode, name, per_edge in ((0, "pr_pull", 8), (1, "pr_push", 12)):

@@ -35,7 +35,11 @@ namespace ogb {
 constexpr uint32_t kMsLight = 32;    // pull: rows up to this many in-edges by one thread
 constexpr uint32_t kMsAlpha = 14;    // push while the frontier's out-edges < E / kMsAlpha
 constexpr uint32_t kMsLong = 512;    // push: rows of more out-edges go in pieces of this many
-constexpr int kMsBatch = 4;          // levels launched between two looks of the host
+// Levels launched between two looks of the host; the levels of the last batch after
+// the search's end are launched for nothing.  us of a 64-root search with 1, 2, 4 and 8:
+// RMAT-20 1090, 1020, 970 and 950; RMAT-16 390, 298, 271 and 240; 300 x 300 grid (600
+// levels) 18400, 13800, 10600 and 9100.
+constexpr int kMsBatch = 4;
 constexpr uint32_t kMsMaxLevels = 0xFFFE;
 
 struct MsCtl {
@@ -519,6 +523,9 @@ int msbfs_run(DevGraph& g, const uint32_t* roots, uint32_t nroots, uint16_t* dep
 // the first two iterations, which write it into both contrib buffers, only the
 // vertices with in-edges are visited.  Dangling vertices' rank is not
 // redistributed, as in the reference.
+// Six CTAs of 256 threads per SM leave a thread 40 registers and 84 bytes of spill
+// stores.  10 iterations with six, five and four CTAs per SM, us: RMAT-20 3770, 3670
+// and 3930; RMAT-16 1060, 960 and 925.
 // ===========================================================================
 
 constexpr uint32_t kPprSeeds = 32;

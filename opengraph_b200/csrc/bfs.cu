@@ -52,8 +52,8 @@
 //    contiguous range of candidates; a candidate's first kFirst in-neighbours
 //    and their frontier bits are loaded at once, longer rows go to a per-round
 //    list scanned by groups of 4 lanes, what is left of them by a warp and then
-//    by the CTA (the first hit in CSR order still wins); the dense-probe mode walks every vertex (a warp's ballot is one
-//    whole word of the next bitmap);
+//    by the CTA (the first hit in CSR order still wins); the dense-probe mode
+//    walks every vertex (a warp's ballot is one whole word of the next bitmap);
 //  * a top-down step sets the bitmap bit of every vertex it discovers and a
 //    bottom-up step lists the vertices it discovers, so a change of
 //    direction needs no conversion pass (arrayQueueToBitmap /
@@ -1474,16 +1474,16 @@ constexpr uint32_t kActDone = 0, kActTD = 1, kActBU = 2, kActNarrow = 3;
 // Narrow steps (bfsk_narrow).  A list is narrow when its entries have at most
 // kNarDeg out-edges and the discoveries of a CTA's share of it fit the CTA's
 // queue.  The grid-wide kernel hands over after `streak` narrow lists of at most
-// kNarEnter entries in a row (narrow_counts), at first kNarStreak, so that the two or three small
-// steps at the ends of a low-diameter search, which are followed by a large one or
-// by the end, stay where they are.
+// kNarEnter entries in a row (narrow_counts), at first kNarStreak, so that the two
+// or three small steps at the ends of a low-diameter search, which are followed by a
+// large one or by the end, stay where they are.
 // A run and the way back (two launches, a wait of the host, the bitmaps remade)
 // cost 33 us, and a narrow step on a path is 3.9 us shorter than a wide one: a run
 // of fewer than kNarShort steps loses.  It doubles `streak`, and a run of
 // kNarLong steps, which has won back several lost ones, resets it.  (A path of
-// 2000 vertices with a hub of 33 leaves at every fifth: 25.4 ms with `streak`
-// left at 4, 12.8 ms with every step wide; at every eighth 16.9 and 12.9; at every
-// twentieth, runs of 16 steps, 9.8 and 12.8.)
+// 2000 vertices with a hub of 33 leaves at every fifth: 25.4 ms with `streak` left at
+// 4 and every narrow list counted, 12.7 now, as with every step wide; at every eighth
+// 16.9 and 12.8; at every twentieth, runs of 14 steps, 10.6.)
 constexpr int kNarT = 1024, kNarC = 8;
 constexpr uint32_t kNarDeg = 32, kNarCap = 8192, kNarEnter = 2048, kNarStreak = 4, kNarShort = 9, kNarLong = 64;
 constexpr uint32_t kNarNever = 0xFFFFFFFFu;  // a streak that no search reaches (at most 2^30 + 8 steps)

@@ -37,9 +37,9 @@
 // most edges share few cache lines (contrib is kept in that numbering), and the
 // rows of in-degree <= warp_thr stored first and contiguous, so a warp loads the
 // edges of 64 light rows (32 on a small graph) with coalesced loads and gathers
-// them 256 (512) at a time (light rows were the latency tail of the iteration: a lane walked its row one dependent gather per step).  The
-// rows, their order and every summation order are unchanged, so the results
-// are bit-identical.  Pull runs one 1024-thread CTA per SM; it takes chunks
+// them 256 (512) at a time (light rows were the latency tail of the iteration: a
+// lane walked its row one dependent gather per step).  The rows, their order and
+// every summation order are unchanged, so the results are bit-identical.  Pull runs one 1024-thread CTA per SM; it takes chunks
 // first (four 256-thread groups per CTA), then warp rows, then light rows.
 // Iterations are launched back to back without host round trips: each iteration's
 // last CTA records error/active and, when active == 0, sets a stop flag that later

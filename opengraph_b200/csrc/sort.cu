@@ -261,8 +261,8 @@ struct PassArgs {
 // A pass is bound by instructions and latency, not by DRAM (31 % of its peak):
 // so a full tile has no bounds checks, a rank is kept with its digit in one
 // word, the leader of a digit is the lane with none before it, and the warp
-// histograms hold 16-bit counts, which with 64 (weighted) and 48 registers
-// gives four and five CTAs per SM.  One pass of 67 M keys by a 7-bit digit:
+// histograms hold 16-bit counts, which with 64 (weighted) and 48 registers (44
+// bytes of spill stores) gives four and five CTAs per SM.  One pass of 67 M keys by a 7-bit digit:
 // 655 -> 435 us weighted (24 bytes per key: 3.7 TB/s), 627 -> 317 us unweighted
 // (3.4 TB/s), against the version with match masks, 64-bit status words, one
 // look-back word at a time and 32-bit histograms.  512 threads (476 us), 20 keys
