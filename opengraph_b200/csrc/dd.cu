@@ -165,8 +165,15 @@ __global__ void __launch_bounds__(kT) dd_self_kernel(uint32_t V, const uint2* __
   const uint64_t gw = (uint64_t)blockIdx.x * (kT / 32) + (threadIdx.x >> 5), nw = (uint64_t)gridDim.x * (kT / 32);
   for (uint64_t t = gw; t < n_och; t += nw) {
     const uint4 c = och[t];
+    const uint32_t len = c.z - c.y;
     uint32_t n = 0;
-    for (uint32_t k = lane; k < c.z - c.y; k += 32) n += (__ldg(&nbr_f[c.y + k]) & 0x3FFFFFFFu) == c.x;
+    for (uint32_t k = lane; k < len; k += 32 * 8) {
+      uint32_t u[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) u[q] = k + q * 32 < len ? (__ldg(&nbr_f[c.y + k + q * 32]) & 0x3FFFFFFFu) : ~c.x;
+#pragma unroll
+      for (int q = 0; q < 8; q++) n += u[q] == c.x;
+    }
     n = __reduce_add_sync(0xffffffffu, n);
     if (lane == 0 && n) atomicAdd(&selfcnt[c.x], n);
   }
@@ -183,18 +190,23 @@ __global__ void __launch_bounds__(kT) dd_self_kernel(uint32_t V, const uint2* __
     const uint32_t total = __shfl_sync(0xffffffffu, ex, 31);
     ex -= r.y;
     for (uint32_t e0 = 0; e0 < total; e0 += 128) {
+      uint32_t p[4], u[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         const uint32_t e = e0 + k * 32 + lane;
-        uint32_t p = 0;  // last row whose first edge is at or before e
+        p[k] = 0;  // last row whose first edge is at or before e
 #pragma unroll
         for (int step = 16; step; step >>= 1) {
-          const uint32_t first = __shfl_sync(0xffffffffu, ex, p + step);
-          if (first <= e) p += step;
+          const uint32_t first = __shfl_sync(0xffffffffu, ex, p[k] + step);
+          if (first <= e) p[k] += step;
         }
-        const uint32_t from = __shfl_sync(0xffffffffu, r.x - ex, p) + e;
-        if (e < total && (__ldg(&nbr_f[from]) & 0x3FFFFFFFu) == (uint32_t)v0 + p) atomicAdd(&selfcnt[v0 + p], 1u);
+        const uint32_t from = __shfl_sync(0xffffffffu, r.x - ex, p[k]) + e;
+        p[k] += (uint32_t)v0;
+        u[k] = e < total ? (__ldg(&nbr_f[from]) & 0x3FFFFFFFu) : ~p[k];
       }
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (u[k] == p[k]) atomicAdd(&selfcnt[p[k]], 1u);
     }
   }
 }
