@@ -64,12 +64,6 @@ constexpr uint32_t kMarkThr = 32;       // out-rows longer than this are deferre
 constexpr uint32_t kOutBig = 1024;      // deferred out-rows longer than this go by chunks
 constexpr uint32_t kOutChunk = 1024;    // edges per chunk of a long out-row
 constexpr uint32_t kDdMaxIters = 1024;
-// Data-driven pull on fewer vertices starts with the light rows: the vertices they put
-// on the next worklist are marked when the other rows' marks come, which then write
-// nothing to the few lines that hold all flags.  us of 20 iterations, light rows first
-// and heavy rows first: RMAT-11 (16 edges per vertex) 770 and 1200, RMAT-13 1130 and
-// 1290, RMAT-14 1400 and 1270, RMAT-18 2830 and 2580.
-constexpr uint32_t kLightFirst = 1u << 14;
 
 struct DdCtl {
   double err[kDdMaxIters];
@@ -251,7 +245,10 @@ Grid3 rows_grid(uint32_t V) {
 
 // No more blocks than the classes' lists have work for: with empty blocks before the
 // light rows', 700 K vertices of 9 in-edges each took 5 % longer in the data-driven
-// pull and 3 % in SPMV.
+// pull and 3 % in SPMV.  (On small graphs the data-driven kernels' times depend on
+// where their buffers lie, by a factor of up to 2.5; means of 15 iterations over 80
+// placements with light rows first and so: RMAT-11 707 and 705 us, RMAT-14 1102 and
+// 1071, 8192 vertices of 8 uniform in-edges 1264 and 819, 65536 of them 1357 and 1405.)
 Grid3 rows_grid(uint32_t V, uint32_t n_med, uint32_t n_hch) {
   Grid3 g = rows_grid(V);
   g.med = std::min<uint32_t>(g.med, ceil_div(n_med, kT / 32));
@@ -464,11 +461,10 @@ struct PullPolicy {
 };
 
 __global__ void __launch_bounds__(kT) dd_pull_kernel(const uint2* __restrict__ rows, const uint32_t* __restrict__ med,
-                                                     HeavyRows heavy, Grid3 G, bool light_first, PullPolicy pol,
+                                                     HeavyRows heavy, Grid3 G, PullPolicy pol,
                                                      DdCtl* __restrict__ ctl, uint32_t it) {
   if (ctl->stop) return;
-  const uint32_t b = light_first ? G.light_first(blockIdx.x) : blockIdx.x;
-  rows_pass(b, rows, med, heavy, ctl->n_med, ctl->n_hch, pol.p.V, G.heavy, G.med, G.light, pol);
+  rows_pass(blockIdx.x, rows, med, heavy, ctl->n_med, ctl->n_hch, pol.p.V, G.heavy, G.med, G.light, pol);
   if (block_totals(pol.err, pol.act, &ctl->err[it], &ctl->active[it], &ctl->done_a[it])) {
     if (ld_volatile_u32(&ctl->active[it]) == 0) {
       ctl->stop_iter = it;
@@ -904,8 +900,7 @@ int pagerank_dd_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsil
   p.epsilon = epsilon;
   const int sms = sm_count();
   const Grid3 G = rows_grid(V);
-  const bool light_first = V < kLightFirst;
-  const Grid3 Gp = light_first ? G : rows_grid(V, w->n_med, w->n_hch);  // of the pull
+  const Grid3 Gp = rows_grid(V, w->n_med, w->n_hch);  // of the pull
   uint8_t* cur = w->flags0.as<uint8_t>();
   uint8_t* nxt = w->flags1.as<uint8_t>();
   float* resid = w->resid.as<float>();
@@ -933,7 +928,7 @@ int pagerank_dd_run(DevGraph& g, uint32_t mode, uint32_t max_iters, double epsil
       dd_contrib_kernel<<<sms * 8, kT, 0, s>>>(V, g.fwd.d_out_degree(), ranks, w->contrib.as<float>(), nxt, defer,
                                                ctl);
       PullPolicy pol{cur, nxt, w->contrib.as<float>(), g.inv.d_dst(), ranks, g.fwd.d_rows(), g.fwd.d_dst(), defer, p};
-      dd_pull_kernel<<<Gp.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), Gp, light_first, pol,
+      dd_pull_kernel<<<Gp.total(), kT, 0, s>>>(g.inv.d_rows(), w->med.as<uint32_t>(), w->heavy.view(), Gp, pol,
                                                ctl, it);
       dd_defer_kernel<false><<<sms * 8, kT, 0, s>>>(V, g.fwd.d_rows(), g.fwd.d_dst(), defer, dvec, och, resid, nxt,
                                                     epsilon, false, ctl, it);
