@@ -1494,11 +1494,12 @@ __device__ __forceinline__ bool narrow_fits(const BfsCtrl& c) {
 // After a top-down step: the list counts towards a run.  A frontier that grows or
 // shrinks fast does not: either the lists are soon wide or the search soon ends, and
 // the run would not pay (uniform graphs of 1 M vertices, one push-only search in us
-// without and with this condition: 4 out-edges each 327 and 311, 6 out-edges 393 and 370;
-// 1.6 out-edges, whose lists grow slowly, 412 and 427; the grid's the same).
+// without this condition and with it: 1.6 out-edges each 420 and 419, 2 out-edges 440 and
+// 434, 3 out-edges 383 and 352, 6 out-edges 390 and 366.  With one and a half times in
+// place of twice, 1.6 out-edges took 439 and a 553 x 553 grid's search 1 % longer).
 __device__ __forceinline__ bool narrow_counts(const BfsCtrl& c) {
   return c.lsize <= kNarEnter && c.lmax <= kNarDeg && c.qcount >= c.frontier / 2 &&
-         c.qcount <= c.frontier + c.frontier / 2 + 2;
+         c.qcount <= 2 * c.frontier + 2;
 }
 // The next step is top-down by ctrl_decide's rule.
 __device__ __forceinline__ bool td_next(const BfsCtrl& c) {

@@ -42,7 +42,8 @@ CASES = {
 # layers of these widths
 LAYERS = {
     "even": ([1, 4, 16, 64] + [700] * 30, 4, 3),
-    "doubling": ([1 << k for k in range(15)], 2, 1),
+    "doubling": ([1 << k for k in range(15)], 2, 3),
+    "tripling": ([3 ** k for k in range(10)], 3, 1),
     "shrinking": ([1, 32, 1000, 20_000, 1500, 400, 100, 25, 6], 32, 1),
 }
 
